@@ -16,6 +16,7 @@ struct pz_ctx {
   cudaStream_t stream = nullptr;
   // device tables
   pz::u64 *d_tw = nullptr;        // fw | fws | iw | iws  (4N words)
+  void *d_fft = nullptr;          // FFT twiddle tables (N = 2048 one-digit sets)
   unsigned short *d_dlog = nullptr;
   pz::u64 *d_tv = nullptr;        // 6 x br_q/2
   // constants
@@ -29,7 +30,7 @@ struct pz_ctx {
   pz::KsParams ks{};
   pz::u32 *d_err = nullptr;  // device error word: DEVERR_* bits set by kernels whose bounded waits ran out
   int grid_limit = 0;
-  int pbs_variant = 0;  // blind-rotation launch shape (see pz::PBS_VARIANTS)
+  int pbs_variant = 0;  // blind-rotation launch shape (see pz::PBS_SPLIT)
   int split_below = -1;  // batches of at most this many gates use the two-CTA kernel (-1: half the SMs)
   int ks_ct = 64;        // key-switch tile: 8, 16, 32 ciphertexts per CTA, 64 = tensor cores (default)
   // autotuned launch shapes per batch-size bucket floor(log2(gates)); a
@@ -52,6 +53,7 @@ struct pz_key {
   pz::u64 *d_rgsw = nullptr, *d_autos = nullptr;
   pz::u32 *d_ksk = nullptr;
   unsigned char *d_ksk8 = nullptr;  // the KSK as byte planes (tensor-core key switch), or null
+  void *d_fft_rgsw = nullptr, *d_fft_autos = nullptr;  // FFT form of d_rgsw and d_autos (both or neither)
   size_t bytes = 0;
 };
 
@@ -67,7 +69,12 @@ namespace pz {
 // the rows come in whole 32-row blocks; otherwise, or when the device is out
 // of memory, the key keeps the IMAD key-switch kernels only).
 void build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s);
+// Build the FFT form of k's RGSW and automorphism keys (N = 2048 one-digit
+// sets; without the memory for it the key keeps the integer kernels only).
+void build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s);
 void free_key_arrays(pz_key *k);
+// BrParams of context c bound to key k (both key forms; k null: no key)
+void br_bind_key(const pz_ctx *c, const pz_key *k, BrParams &br);
 // KsParams of context c bound to key k (both KSK forms)
 void ks_bind_key(const pz_ctx *c, const pz_key *k, KsParams &ks);
 // floor(log2(n)), clamped to the 48 buckets of pz_ctx::tuned

@@ -19,6 +19,7 @@
 
 #include <cooperative_groups.h>
 
+#include "pz_blind.cuh"
 #include "pz_kernels.cuh"
 
 namespace pz {
@@ -32,16 +33,6 @@ constexpr int OP_REGIONS = 2;
 // The two-CTA blind rotation: region 0 exchanges / scatter, region 1 schedule
 // scratch / permutation of b, regions 2-3 the two digit slots read by the peer.
 constexpr int SPLIT_REGIONS = 4;
-
-// Operation codes of the blind-rotation schedule: an external product with
-// RGSW key `i` is `i`; an automorphism with key slot v (0 = -g) is
-// OP_AUTO | v, plus OP_TRIVIAL while the accumulator is still trivial.
-// OP_KEEPB marks an operation whose successor is a non-trivial automorphism:
-// it leaves b in the evaluation domain (scaled by N^{-1}, values < 2q), where
-// the automorphism permutes it and adds it before its own inverse transform,
-// so b skips one inverse and one forward-domain round trip.
-constexpr u32 OP_AUTO = 0x8000u, OP_TRIVIAL = 0x4000u, OP_KEEPB = 0x2000u, OP_SLOT = 0x00ffu,
-              OP_INDEX = 0x1fffu;
 
 // ---------------------------------------------------------------------------
 // Key conversion and NTT microbench
@@ -864,12 +855,6 @@ __global__ void ksk_planes_kernel(const u32 *ksk, u32 rows, u32 stride, u32 n, u
 // ---------------------------------------------------------------------------
 // The bootstrap: one CTA per ciphertext (grid-stride over the batch)
 // ---------------------------------------------------------------------------
-// pbs.rs:416-420
-__device__ __forceinline__ u32 mod_switch_odd(u32 v, double from_q, double to_q) {
-  u64 odd = (u64)floor(__ddiv_rn(__dmul_rn((double)v, to_q), from_q));
-  return (u32)(odd + ((odd & 1ull) ^ 1ull));
-}
-
 // Shared memory of pbs_kernel: OP_REGIONS x N words, then u16 arrays:
 // bucket starts (R + 1), bucket members (n), the schedule (n + R + 1), and
 // the schedule length.
@@ -886,172 +871,6 @@ static size_t split_smem_bytes(u32 br_q, u32 n) {
   size_t extra = ((R + 1) + n + (n + R + 1)) * 2 + 4;
   extra = (extra + 15) & ~(size_t)15;
   return SPLIT_REGIONS * 8 * N + extra;
-}
-
-// Shared-memory arrays of the blind-rotation schedule, after `regions` x N words.
-struct SchedSmem {
-  unsigned short *start, *list, *ops;
-  u32 *nops;
-};
-template <int LOGN>
-__device__ __forceinline__ SchedSmem sched_smem(u64 *smem, int regions, u32 R, u32 n) {
-  constexpr int N = 1 << LOGN;
-  SchedSmem m;
-  m.start = (unsigned short *)(smem + regions * N);  // R + 1
-  m.list = m.start + (R + 1);                         // n
-  m.ops = m.list + n;                                 // n + R + 1
-  m.nops = (u32 *)(((size_t)(m.ops + n + R + 1) + 3) & ~(size_t)3);
-  return m;
-}
-
-// Odd mod-switch, dlog buckets (pbs.rs:147-161, stable in LWE index) and the
-// blind-rotation schedule (pbs.rs:240-414) of one key-switched LWE, built in
-// shared memory by the whole CTA (regions 0 and 1 of smem are scratch).
-template <int LOGN>
-__device__ __forceinline__ void build_schedule(const BrParams &P, const u32 *kso, u64 *smem, const SchedSmem &S) {
-  constexpr int N = 1 << LOGN, T = NttShape<LOGN>::T;
-  const u32 R = P.br_q >> 1, q4 = P.br_q >> 2, n = P.n;
-  const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
-  u64 *sm = smem;
-  unsigned short *s_start = S.start, *s_list = S.list, *s_ops = S.ops;
-  u32 *s_nops = S.nops;
-  {
-    // ---- odd mod-switch + dlog buckets (pbs.rs:147-161), stable in LWE index
-    u32 *cnt = (u32 *)sm;                                 // R counters (region 0)
-    unsigned short *keys = (unsigned short *)(cnt + R);   // n keys (region 0)
-    u32 *fill = (u32 *)(sm + N);                          // R fill counters (region 1)
-    u32 *scan = fill + R;                                 // T partial sums (region 1)
-    __syncthreads();
-    for (u32 b = j; b < R; b += T) { cnt[b] = 0; fill[b] = 0; }
-    __syncthreads();
-    for (u32 i = j; i < n; i += T) {
-      const u32 odd = mod_switch_odd(kso[1 + i] & P.ks_mask, P.q_ks_f, P.br_q_f);
-      const u32 k = P.dlog[odd];
-      keys[i] = (unsigned short)k;
-      atomicAdd(&cnt[k], 1u);
-    }
-    __syncthreads();
-    {  // exclusive scan of cnt[0..R) into s_start, s_start[R] = n
-      const u32 per = (R + T - 1) / T;
-      const u32 b0 = j * per;
-      u32 local = 0;
-      for (u32 b = b0; b < b0 + per && b < R; b++) local += cnt[b];
-      u32 incl = local;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        u32 y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (lane == 31) scan[warp] = incl;
-      __syncthreads();
-      u32 woff = 0;
-      for (int w2 = 0; w2 < warp; w2++) woff += scan[w2];
-      u32 run = woff + incl - local;
-      for (u32 b = b0; b < b0 + per && b < R; b++) {
-        s_start[b] = (unsigned short)run;
-        run += cnt[b];
-      }
-      if (j == 0) s_start[R] = (unsigned short)n;
-    }
-    __syncthreads();
-    if (warp == 0) {  // stable placement: within a bucket, increasing LWE index
-      for (u32 i0 = 0; i0 < n; i0 += 32) {
-        const u32 i = i0 + lane;
-        const bool valid = i < n;
-        const u32 k = valid ? keys[i] : 0xFFFFu;
-        const u32 peers = __match_any_sync(0xffffffffu, k);
-        const u32 rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid) s_list[s_start[k] + fill[k] + rank] = (unsigned short)i;
-        __syncwarp();
-        if (valid && rank == 0) fill[k] += __popc(peers);
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    // ---- the blind-rotation schedule (pbs.rs:240-414): buckets of -g^k for
-    // k = q/4-1..1, -g^0, +g^k, +g^0, each followed by an automorphism when
-    // the next bucket is non-empty, the window w is reached or k == 1; the
-    // automorphisms before the first external product act on a trivial RLWE.
-    if (j == 0) {
-      u32 no = 0;
-      bool trivial = true;
-      auto bucket = [&](u32 b) {
-        const u32 e = s_start[b + 1];
-        for (u32 t = s_start[b]; t < e; t++) s_ops[no++] = s_list[t];
-        if (e != s_start[b]) trivial = false;
-      };
-      auto autom = [&](u32 v) {
-        if (!trivial) s_ops[no - 1] |= (unsigned short)OP_KEEPB;  // b stays in the evaluation domain
-        s_ops[no++] = (unsigned short)(OP_AUTO | (trivial ? OP_TRIVIAL : 0u) | v);
-      };
-      u32 v = 0;
-      for (u32 i = q4 - 1; i >= 1; i--) {  // -(g^k)
-        bucket(q4 + i);
-        v++;
-        if (s_start[q4 + i] != s_start[q4 + i - 1] || v == P.w || i == 1) {
-          autom(v);
-          v = 0;
-        }
-      }
-      bucket(q4);  // -(g^0)
-      autom(0);
-      v = 0;
-      for (u32 i = q4 - 1; i >= 1; i--) {  // +(g^k)
-        bucket(i);
-        v++;
-        if (s_start[i] != s_start[i - 1] || v == P.w || i == 1) {
-          autom(v);
-          v = 0;
-        }
-      }
-      bucket(0);  // +(g^0)
-      *s_nops = no;
-    }
-  }
-}
-
-// Trivial test RLWE's b: X^{g * odd(b)} * tv, embedded (pbs.rs:163-211), in
-// the coefficient layout of this thread.
-template <int LOGN>
-__device__ __forceinline__ void test_rlwe_b(const BrParams &P, const u32 *kso, u32 gcode, u64 (&b)[8]) {
-  const u32 R = P.br_q >> 1;
-  const u64 q = P.rc.q;
-  const int j = threadIdx.x;
-  const u32 odd_b = mod_switch_odd(kso[0] & P.ks_mask, P.q_ks_f, P.br_q_f);
-  const u32 gb = (u32)(((u64)P.g * odd_b) % P.br_q);
-  u32 mexp = gb;
-  bool msign = true;
-  if (mexp > R) { mexp -= R; msign = false; }
-  u32 gi = gcode & 7u;
-  if (gi > 5) gi = 5;  // codes are validated on the host; never index past the 6 test vectors
-  const u64 *tv = P.tv + (size_t)gi * R;
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    const u32 p = (u32)pos_coef<LOGN>(j, r);
-    u64 v = 0;
-    if (p % P.emb == 0) {
-      const u32 o = p / P.emb;
-      u32 s;
-      bool sg;
-      if (o >= mexp) { s = o - mexp; sg = msign; } else { s = o + R - mexp; sg = !msign; }
-      const u64 t = tv[s];
-      v = sg ? t : q - t;
-    }
-    b[r] = v;
-  }
-}
-
-// L2 prefetch of a blind-rotation operation's key rows (none for a trivial
-// automorphism).
-template <int LOGN>
-__device__ __forceinline__ void prefetch_next_key(const BrParams &P, u32 op) {
-  constexpr size_t N = (size_t)1 << LOGN;
-  if (op & OP_AUTO) {
-    if (!(op & OP_TRIVIAL))
-      prefetch_l2(P.autos + (size_t)(op & OP_SLOT) * P.auto_rows * N, P.auto_rows * (u32)N * 8);
-  } else {
-    prefetch_l2(P.rgsw + (size_t)(op & OP_INDEX) * P.rgsw_rows * N, P.rgsw_rows * (u32)N * 8);
-  }
 }
 
 // MINB: CTAs per SM the register allocation must allow (launch-shape
@@ -1135,258 +954,6 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, MINB)
     __syncthreads();
     pbs_item<LOGN, D1>(sp, ct, ks + (size_t)ct * ks_stride, gates[ct], out, nullptr, smem);
   }
-}
-
-// ---------------------------------------------------------------------------
-// Blind rotation with the keys streamed into shared memory (launch shape
-// PBS_BULK, N = 2048, one-digit decompositions).  Each CTA keeps a 64 KB key
-// stage.  Right after an operation's multiply-accumulate has read the stage,
-// one thread issues the bulk copy (cp.async.bulk + mbarrier, from this GPU's
-// memory, no multicast) of the next operation's key rows -- the 4 RGSW rows
-// (64 KB) or the 2 automorphism-key rows (32 KB), contiguous in the device
-// layout -- which lands while the CTA runs this operation's inverse
-// transform and the next one's decomposition and forward transform.  The
-// multiply-accumulate then reads its key from shared memory, not from L2.
-// Two CTAs per SM (the stage); the register cap is 128.  Every wait is
-// bounded: one that runs out sets DEVERR_MBAR_TIMEOUT and the CTA returns.
-// ---------------------------------------------------------------------------
-constexpr int BULK_REGIONS = 6;  // 2N words exchange / permutations, 4N words key stage
-
-static size_t bulk_sched_bytes(u32 br_q, u32 n) {
-  const size_t R = br_q / 2;
-  size_t extra = ((R + 1) + n + (n + R + 1)) * 2 + 4;
-  return (extra + 15) & ~(size_t)15;
-}
-static size_t bulk_smem_bytes(u32 br_q, u32 n) {
-  return (size_t)BULK_REGIONS * 8 * 2048 + bulk_sched_bytes(br_q, n) + 16;  // + the mbarrier
-}
-__device__ __forceinline__ u64 *bulk_bar(u64 *smem, u32 br_q, u32 n) {
-  const u32 R = br_q / 2;
-  u32 extra = ((R + 1) + n + (n + R + 1)) * 2 + 4;
-  extra = (extra + 15) & ~15u;
-  return (u64 *)((char *)smem + (size_t)BULK_REGIONS * 8 * 2048 + extra);
-}
-
-// Key rows of a keyed operation (not a trivial automorphism): source and bytes.
-__device__ __forceinline__ void op_key_rows(const BrParams &P, u32 op, const u64 *&src, u32 &bytes) {
-  constexpr size_t N = 2048;
-  if (op & OP_AUTO) {
-    src = P.autos + (size_t)(op & OP_SLOT) * P.auto_rows * N;
-    bytes = P.auto_rows * (u32)N * 8;
-  } else {
-    src = P.rgsw + (size_t)(op & OP_INDEX) * P.rgsw_rows * N;
-    bytes = P.rgsw_rows * (u32)N * 8;
-  }
-}
-__device__ __forceinline__ bool op_keyed(u32 op) { return !((op & OP_AUTO) && (op & OP_TRIVIAL)); }
-
-// mac_pair / mac_auto with the key rows in shared memory (device layout,
-// row r at ks + r N).
-__device__ __forceinline__ void mac_pair_staged(u64 (&x)[8], u64 (&y)[8], const u64 *ks, const RingConsts &rc) {
-  constexpr int LOGN = 11, N = 2048;
-  const int j = threadIdx.x;
-  const u64 q = rc.q, qi = rc.qinv_neg;
-#pragma unroll
-  for (int rr = 0; rr < 4; rr++) {
-    const int di = dev_index<LOGN>(j, 2 * rr);
-    u64 a[2], b[2], c[2], d[2];
-    lds2(ks + di, a[0], a[1]);
-    lds2(ks + N + di, b[0], b[1]);
-    lds2(ks + 2 * N + di, c[0], c[1]);
-    lds2(ks + 3 * N + di, d[0], d[1]);
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int r = 2 * rr + e;
-      const u64 xv = x[r], yv = y[r];
-      u64 hi, lo, hi2, lo2;
-      sum2_128(xv, a[e], yv, c[e], hi, lo);
-      sum2_128(xv, b[e], yv, d[e], hi2, lo2);
-      x[r] = mac_reduce<LOGN>(hi, lo, q, qi);
-      y[r] = mac_reduce<LOGN>(hi2, lo2, q, qi);
-    }
-  }
-}
-__device__ __forceinline__ void mac_auto_staged(u64 (&x)[8], u64 (&y)[8], const u64 *ks, const RingConsts &rc) {
-  constexpr int LOGN = 11, N = 2048;
-  const int j = threadIdx.x;
-  const u64 q = rc.q, qi = rc.qinv_neg, q2 = rc.q << 1;
-#pragma unroll
-  for (int rr = 0; rr < 4; rr++) {
-    const int di = dev_index<LOGN>(j, 2 * rr);
-    u64 a[2], b[2];
-    lds2(ks + di, a[0], a[1]);
-    lds2(ks + N + di, b[0], b[1]);
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int r = 2 * rr + e;
-      u64 hi, lo, hi2, lo2;
-      mac_mul<LOGN>(x[r], a[e], hi, lo);
-      mac_mul<LOGN>(x[r], b[e], hi2, lo2);
-      x[r] = mac_reduce<LOGN>(hi, lo, q, qi);
-      y[r] = mac_add_b<LOGN>(mac_reduce<LOGN>(hi2, lo2, q, qi) + y[r], q2);
-    }
-  }
-}
-
-// One keyed operation of the staged blind rotation: bootstrap_op's one-digit
-// path with the key from the stage (its copy completes phase `parity` of
-// *bar); after the multiply-accumulate the copy of the next operation's key
-// (next_src, next_bytes; none when next_src is null) is issued into the same
-// stage.  False (uniformly over the CTA) when the wait ran out.
-__device__ __forceinline__ bool bootstrap_op_staged(u64 (&acc)[2][8], u32 op, const BrParams &P, u64 *sm,
-                                                    u64 *stage, u64 *bar, u32 parity, const u64 *next_src,
-                                                    u32 next_bytes) {
-  constexpr int LOGN = 11, N = 2048;
-  const u64 q = P.rc.q;
-  const int j = threadIdx.x;
-  u64(&x)[8] = acc[0];
-  u64(&y)[8] = acc[1];
-  const bool is_auto = (op & OP_AUTO) != 0;
-  const bool keep_b = (op & OP_KEEPB) != 0;
-  u64 *s_a = sm, *s_b = sm + N;
-  if (is_auto) {  // non-trivial: a(X^k) with sign, b permuted in the evaluation domain
-    const u32 k = P.auto_k[op & OP_SLOT];
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      u32 t = ((u32)pos_coef<LOGN>(j, r) * k) & (2 * N - 1);
-      const bool neg = t >= (u32)N;
-      if (neg) t -= N;
-      s_a[swz(t)] = neg ? q - x[r] : x[r];
-      s_b[swz(pos_eval<LOGN>(j, r))] = y[r];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 8; r++) y[r] = s_b[swz(auto_eval_src<LOGN>(pos_eval<LOGN>(j, r), k))];
-#pragma unroll
-    for (int r = 0; r < 8; r++) x[r] = decompose1<AUTO_LOGB, AUTO_IGN>(s_a[swz(pos_coef<LOGN>(j, r))], q);
-    ntt_fwd<LOGN, false>(x, x, sm, P.rc);
-  } else {
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      x[r] = decompose1<RLRG_LOGB, RLRG_IGN>(x[r], q);
-      y[r] = decompose1<RLRG_LOGB, RLRG_IGN>(y[r], q);
-    }
-    ntt_fwd<LOGN, true>(x, y, sm, P.rc);
-  }
-  if (!__syncthreads_and(mbar_wait(bar, parity))) {
-    if (j == 0) {
-      atomicOr(P.err, DEVERR_MBAR_TIMEOUT);
-      mbar_wait(bar, parity);  // bounded: the copy this CTA still has in flight
-    }
-    return false;
-  }
-  if (is_auto) mac_auto_staged(x, y, stage, P.rc);
-  else mac_pair_staged(x, y, stage, P.rc);
-  __syncthreads();  // every thread has read the stage (also the exchange barrier of the inverse)
-  if (j == 0 && next_src) {
-    fence_proxy_async_smem();
-    bulk_load(stage, next_src, next_bytes, bar);
-  }
-  if (keep_b) {
-    ntt_inv<LOGN, false, false>(x, x, sm, P.rc);
-#pragma unroll
-    for (int r = 0; r < 8; r++) x[r] = reduce2(x[r], q);
-  } else {
-    ntt_inv<LOGN, true, false>(x, y, sm, P.rc);
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      x[r] = reduce2(x[r], q);
-      y[r] = reduce2(y[r], q);
-    }
-  }
-  return true;
-}
-
-// One gate bootstrap with staged keys; `phase` counts this CTA's completed
-// waits (the mbarrier's phase parity).  False when a wait ran out.
-__device__ __forceinline__ bool pbs_item_staged(const BrParams &P, int ct, const u32 *kso, u32 gcode, u64 *out,
-                                                u64 *smem, u64 *bar, u32 &phase) {
-  constexpr int LOGN = 11, N = 2048;
-  u64 *sm = smem, *stage = smem + 2 * N;
-  const SchedSmem S = sched_smem<LOGN>(smem, BULK_REGIONS, P.br_q >> 1, P.n);
-  const int j = threadIdx.x;
-  const u64 q = P.rc.q;
-  build_schedule<LOGN>(P, kso, smem, S);
-  u64 acc[2][8];
-#pragma unroll
-  for (int r = 0; r < 8; r++) acc[0][r] = 0;
-  test_rlwe_b<LOGN>(P, kso, gcode, acc[1]);
-  __syncthreads();
-  const u32 nops = *S.nops;
-  u32 t = 0;
-  // trivial automorphisms (only before the first external product) need no key
-#pragma unroll 1
-  for (; t < nops && !op_keyed(S.ops[t]); t++) bootstrap_op<LOGN, true>(acc, S.ops[t], P, sm);
-  if (j == 0 && t < nops) {
-    const u64 *src;
-    u32 bytes;
-    op_key_rows(P, S.ops[t], src, bytes);
-    fence_proxy_async_smem();
-    bulk_load(stage, src, bytes, bar);
-  }
-#pragma unroll 1
-  for (; t < nops; t++) {
-    const u64 *nsrc = nullptr;
-    u32 nbytes = 0;
-    if (t + 1 < nops) op_key_rows(P, S.ops[t + 1], nsrc, nbytes);
-    if (!bootstrap_op_staged(acc, S.ops[t], P, sm, stage, bar, phase & 1u, nsrc, nbytes)) return false;
-    phase++;
-  }
-  // ---- sample extract at index 0 (pbs.rs:423-449)
-  u64 *o = out + (size_t)(P.out_idx ? P.out_idx[ct] : (u32)ct) * (N + 1);
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    const u32 p = (u32)pos_coef<LOGN>(j, r);
-    if (p == 0) {
-      o[0] = acc[1][r];
-      o[1] = acc[0][r];
-    } else {
-      o[1 + N - p] = q - acc[0][r];
-    }
-  }
-  return true;
-}
-
-// The staged-key blind rotation over a ragged batch: item ct uses descriptor
-// item_desc[ct] (parameter set and key of its session) and scatters to
-// out_idx[ct]; the schedule arrays are laid out for the launch's maximum
-// (br_q, n), the mbarrier after them.
-__global__ void __launch_bounds__(256, 2)
-    pbs_bulk_ragged_kernel(const BrParams *descs, const u32 *item_desc, const u32 *ks, u32 ks_stride,
-                           const unsigned char *gates, u64 *out, const u32 *out_idx, int count, u32 max_br_q,
-                           u32 max_n) {
-  extern __shared__ __align__(128) u64 smem[];
-  __shared__ BrParams sp;
-  u64 *bar = bulk_bar(smem, max_br_q, max_n);
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_init_fence();
-  }
-  u32 phase = 0;
-  for (int ct = blockIdx.x; ct < count; ct += gridDim.x) {
-    __syncthreads();  // the previous item is done with sp (and the mbarrier is initialised)
-    if (threadIdx.x == 0) {
-      sp = descs[item_desc[ct]];
-      sp.out_idx = out_idx;
-    }
-    __syncthreads();
-    if (!pbs_item_staged(sp, ct, ks + (size_t)ct * ks_stride, gates[ct], out, smem, bar, phase)) return;
-  }
-}
-
-__global__ void __launch_bounds__(256, 2)
-    pbs_bulk_kernel(BrParams P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out, int count) {
-  extern __shared__ __align__(128) u64 smem[];
-  u64 *bar = bulk_bar(smem, P.br_q, P.n);
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  u32 phase = 0;
-  for (int ct = blockIdx.x; ct < count; ct += gridDim.x)
-    if (!pbs_item_staged(P, ct, ks + (size_t)ct * ks_stride, gates[ct], out, smem, bar, phase)) return;
 }
 
 // ---------------------------------------------------------------------------
@@ -1748,8 +1315,24 @@ cudaError_t launch_key_convert(int logn, const u64 *in, u64 *out, size_t npolys,
   return cudaGetLastError();
 }
 
+cudaError_t opt_in_smem(const void *kernel, size_t bytes) {
+  // the attribute is per kernel and per device: remember the largest size set
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, size_t> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t &have = done[{kernel, dev}];
+  if (bytes <= have) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) have = bytes;
+  return e;
+}
 template <typename K>
-static cudaError_t set_smem(K kernel, size_t bytes);
+static cudaError_t set_smem(K kernel, size_t bytes) {
+  return opt_in_smem((const void *)kernel, bytes);
+}
 
 // Persistent grid of the batched NTT: two CTAs per SM, no more CTAs than pairs.
 static int ntt_batch_grid(size_t count) {
@@ -1787,23 +1370,6 @@ cudaError_t launch_ntt_inv(int logn, u64 *polys, size_t count, const RingConsts 
   return cudaGetLastError();
 }
 
-// Opt the kernel into its dynamic shared memory once (largest size asked so
-// far), outside of any launch sequence that may be captured into a graph.
-template <typename K>
-static cudaError_t set_smem(K kernel, size_t bytes) {
-  // the attribute is per kernel and per device: remember the largest size set
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, size_t> done;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lock(mu);
-  size_t &have = done[{(const void *)kernel, dev}];
-  if (bytes <= have) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) have = bytes;
-  return e;
-}
 cudaError_t launch_ext_product(int logn, bool d1, const BrParams &P, u64 *rlwe, const u32 *idx,
                                size_t count, int trivial, cudaStream_t s, int variant) {
   if (count == 0) return cudaSuccess;
@@ -1931,27 +1497,17 @@ cudaError_t launch_pbs(int logn, bool d1, const BrParams &P, const u32 *ks, u32 
   int grid = (int)count;
   if (grid_limit > 0 && grid > grid_limit) grid = grid_limit;
   cudaError_t e;
-#define PZ_LAUNCH(LN, DD, MB, TH)                                                                    \
-  if ((e = set_smem(pbs_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;                        \
-  pbs_kernel<LN, DD, MB><<<grid, TH, smem, s>>>(P, ks, ks_stride, gates, out, (int)count, rlwe_dbg);
   if (logn == 11 && d1 && variant == PBS_SPLIT && rlwe_dbg == nullptr) {
     const size_t ssmem = split_smem_bytes(P.br_q, P.n);
     if ((e = set_smem(pbs_split_kernel<11>, ssmem)) != cudaSuccess) return e;
     pbs_split_kernel<11><<<2 * grid, 256, ssmem, s>>>(P, ks, ks_stride, gates, out, (int)count);
     return cudaGetLastError();
   }
-  if (logn == 11 && d1 && variant == PBS_BULK && rlwe_dbg == nullptr) {
-    const size_t bsmem = bulk_smem_bytes(P.br_q, P.n);
-    if ((e = set_smem(pbs_bulk_kernel, bsmem)) != cudaSuccess) return e;
-    pbs_bulk_kernel<<<grid, 256, bsmem, s>>>(P, ks, ks_stride, gates, out, (int)count);
-    return cudaGetLastError();
-  }
-  if (variant > 2) variant = 0;  // shapes without a debug-output form
-  if (logn == 11 && d1) {
-    if (variant == 0) { PZ_LAUNCH(11, true, 2, 256) }
-    else if (variant == 1) { PZ_LAUNCH(11, true, 3, 256) }
-    else { PZ_LAUNCH(11, true, 4, 256) }
-  }
+  if (logn == 11 && d1 && P.fft_rgsw) return launch_pbs_fft(P, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
+#define PZ_LAUNCH(LN, DD, MB, TH)                                                                    \
+  if ((e = set_smem(pbs_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;                        \
+  pbs_kernel<LN, DD, MB><<<grid, TH, smem, s>>>(P, ks, ks_stride, gates, out, (int)count, rlwe_dbg);
+  if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }  // a key without its FFT form
   else if (logn == 11) { PZ_LAUNCH(11, false, 1, 256) }
   else if (logn == 9 && d1) { PZ_LAUNCH(9, true, 1, 64) }
   else if (logn == 9) { PZ_LAUNCH(9, false, 1, 64) }
@@ -1977,12 +1533,8 @@ cudaError_t pbs_slots(int logn, bool d1, u32 br_q, u32 n, int variant, size_t *s
   if (logn == 11 && d1 && variant == PBS_SPLIT) {
     PZ_OCC(pbs_split_kernel<11>, 256, split_smem_bytes(br_q, n))
     div = 2;
-  } else if (logn == 11 && d1 && variant == PBS_BULK) {
-    PZ_OCC(pbs_bulk_kernel, 256, bulk_smem_bytes(br_q, n))
   } else if (logn == 11 && d1) {
-    if (variant == 0) { PZ_OCC((pbs_kernel<11, true, 2>), 256, smem) }
-    else if (variant == 1) { PZ_OCC((pbs_kernel<11, true, 3>), 256, smem) }
-    else { PZ_OCC((pbs_kernel<11, true, 4>), 256, smem) }
+    e = pbs_fft_per_sm(br_q, n, &per_sm);
   } else if (logn == 11) { PZ_OCC((pbs_kernel<11, false, 1>), 256, smem) }
   else if (logn == 9 && d1) { PZ_OCC((pbs_kernel<9, true, 1>), 64, smem) }
   else if (logn == 9) { PZ_OCC((pbs_kernel<9, false, 1>), 64, smem) }
@@ -2023,7 +1575,8 @@ cudaError_t launch_ks_mma_ragged(const KsParams *d_descs, const KsTile *d_tiles,
 
 cudaError_t launch_pbs_ragged(int logn, bool d1, const BrParams *d_descs, const u32 *item_desc, u32 max_br_q,
                               u32 max_n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
-                              const u32 *out_idx, size_t count, int grid_limit, cudaStream_t s, int variant) {
+                              const u32 *out_idx, size_t count, int grid_limit, cudaStream_t s, int variant,
+                              bool fft) {
   if (count == 0) return cudaSuccess;
   const size_t smem = pbs_smem_bytes(logn, max_br_q, max_n);
   int grid = (int)count;
@@ -2036,23 +1589,14 @@ cudaError_t launch_pbs_ragged(int logn, bool d1, const BrParams *d_descs, const 
                                                              (int)count);
     return cudaGetLastError();
   }
-  if (logn == 11 && d1 && variant == PBS_BULK) {
-    const size_t bsmem = bulk_smem_bytes(max_br_q, max_n);
-    if ((e = set_smem(pbs_bulk_ragged_kernel, bsmem)) != cudaSuccess) return e;
-    pbs_bulk_ragged_kernel<<<grid, 256, bsmem, s>>>(d_descs, item_desc, ks, ks_stride, gates, out, out_idx,
-                                                    (int)count, max_br_q, max_n);
-    return cudaGetLastError();
-  }
-  if (variant > 2) variant = 0;
+  if (logn == 11 && d1 && fft)
+    return launch_pbs_fft_ragged(d_descs, item_desc, max_br_q, max_n, ks, ks_stride, gates, out, out_idx, count, grid,
+                                 s);
 #define PZ_LAUNCH(LN, DD, MB, TH)                                                                    \
   if ((e = set_smem(pbs_ragged_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;                 \
   pbs_ragged_kernel<LN, DD, MB><<<grid, TH, smem, s>>>(d_descs, item_desc, ks, ks_stride, gates, out, out_idx, \
                                                        (int)count);
-  if (logn == 11 && d1) {
-    if (variant == 0) { PZ_LAUNCH(11, true, 2, 256) }
-    else if (variant == 1) { PZ_LAUNCH(11, true, 3, 256) }
-    else { PZ_LAUNCH(11, true, 4, 256) }
-  }
+  if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }  // a session's key without its FFT form
   else if (logn == 11) { PZ_LAUNCH(11, false, 1, 256) }
   else if (logn == 9 && d1) { PZ_LAUNCH(9, true, 1, 64) }
   else if (logn == 9) { PZ_LAUNCH(9, false, 1, 64) }

@@ -7,7 +7,7 @@ namespace pz {
 constexpr int MAX_KS_D = 16;   // key-switch decomposition count bound
 // Revision of the blind-rotation kernels: bumped with every change to their
 // code, so that a profile taken on one revision is not reported for another.
-constexpr const char *BR_KERNEL_REVISION = "br-v15";
+constexpr const char *BR_KERNEL_REVISION = "br-v16";
 constexpr int MAX_AUTO_SLOTS = 16;
 
 // Everything the blind rotation needs for one parameter set + server key.
@@ -26,6 +26,8 @@ struct BrParams {
   const u64 *autos;                // [w+1][auto_rows][N]
   const u32 *out_idx;              // optional scatter: output of gate ct -> LWE out_idx[ct]
   u32 *err;                        // the context's device error word (DEVERR_* bits)
+  // FFT form of the same keys (N = 2048 one-digit sets; null: not built) and its twiddle tables
+  const void *fft_rgsw, *fft_autos, *fft_tw;
 };
 
 // Gate prelude + mod-down + LWE key switch.
@@ -97,16 +99,11 @@ cudaError_t launch_ks(const KsParams &P, const unsigned char *gates, const u64 *
 cudaError_t launch_pbs(int logn, bool d1, const BrParams &P, const u32 *ks, u32 ks_stride,
                        const unsigned char *gates, u64 *out, size_t count, u64 *rlwe_dbg,
                        int grid_limit, cudaStream_t s, int variant);
-// launch-shape variants of the production blind rotation (registers per
-// thread capped for 2, 3 or 4 CTAs of 256 threads per SM)
-constexpr int PBS_VARIANTS = 3;
-// launch shape for small batches (N = 2048, one-digit sets): one ciphertext
-// per cluster of two CTAs, a on one SM and b on the other (lower latency)
-constexpr int PBS_SPLIT = 3;
-// launch shape with every operation's key rows streamed into a shared-memory
-// stage by bulk copies (N = 2048, one-digit sets; two CTAs per SM)
-constexpr int PBS_BULK = 4;
-constexpr int PBS_MAX_VARIANT = PBS_BULK;
+// Launch shapes of the N = 2048 one-digit sets.  0, 1, 2 and 4: one CTA per
+// ciphertext (these were register caps and key staging of an integer kernel;
+// they stay as names of the one shape that is left).  3: one ciphertext per
+// cluster of two CTAs (lower latency, for small batches).
+constexpr int PBS_SPLIT = 3, PBS_MAX_VARIANT = 4;
 // Ragged batches (several sessions / parameter sets in one launch): per-item
 // descriptors in device memory; max_* bound the sizes over the descriptors.
 cudaError_t launch_ks_ragged(const KsParams *d_descs, const KsTile *d_tiles, size_t ntiles, size_t count,
@@ -119,7 +116,23 @@ cudaError_t launch_ks_mma_ragged(const KsParams *d_descs, const KsTile *d_tiles,
                                  const u32 *in0, const u32 *in1, u32 *out, u32 out_stride, cudaStream_t s);
 cudaError_t launch_pbs_ragged(int logn, bool d1, const BrParams *d_descs, const u32 *item_desc, u32 max_br_q,
                               u32 max_n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
-                              const u32 *out_idx, size_t count, int grid_limit, cudaStream_t s, int variant);
+                              const u32 *out_idx, size_t count, int grid_limit, cudaStream_t s, int variant,
+                              bool fft);  // fft: every descriptor in use has its key's FFT form
+// dynamic shared memory of a kernel, opted into once per device and size
+cudaError_t opt_in_smem(const void *kernel, size_t bytes);
+// FFT form (pz_fft.cu): the twiddle tables of a device, the bytes and the
+// conversion of `keys` keys of rows_per_key device rows, and the one-digit
+// N = 2048 blind rotation over it.
+cudaError_t fft_tables(void **out);
+size_t fft_key_bytes(size_t keys);
+cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const RingConsts &rc, const void *tables,
+                           void *out, cudaStream_t s);
+cudaError_t launch_pbs_fft(const BrParams &P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
+                           size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s);
+cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas);  // resident CTAs per SM
+cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc, u32 max_br_q, u32 max_n, const u32 *ks,
+                                  u32 ks_stride, const unsigned char *gates, u64 *out, const u32 *out_idx,
+                                  size_t count, int grid, cudaStream_t s);
 cudaError_t launch_not(const u64 *in, u64 *out, size_t words, u64 q, cudaStream_t s);
 cudaError_t launch_imad_probe(int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);
 cudaError_t launch_pipe_probe(int kind, int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);

@@ -220,7 +220,34 @@ void build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s) {
   k->bytes += bytes;
 }
 
+void build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s) {
+  const pz_params &P = c->P;
+  if (!c->d_fft) return;
+  const size_t rg = fft_key_bytes(P.lwe_n), au = fft_key_bytes(P.n_auto_keys);
+  if (cudaMalloc(&k->d_fft_rgsw, rg) == cudaSuccess && cudaMalloc(&k->d_fft_autos, au) == cudaSuccess &&
+      launch_fft_key(k->d_rgsw, P.rgsw_rows, P.lwe_n, c->rc, c->d_fft, k->d_fft_rgsw, s) == cudaSuccess &&
+      launch_fft_key(k->d_autos, P.auto_rows, P.n_auto_keys, c->rc, c->d_fft, k->d_fft_autos, s) == cudaSuccess &&
+      cudaStreamSynchronize(s) == cudaSuccess) {
+    k->bytes += rg + au;
+    return;
+  }
+  cudaGetLastError();
+  cudaFree(k->d_fft_rgsw);
+  cudaFree(k->d_fft_autos);
+  k->d_fft_rgsw = k->d_fft_autos = nullptr;
+}
+
+void br_bind_key(const pz_ctx *c, const pz_key *k, BrParams &br) {
+  br.rgsw = k ? k->d_rgsw : nullptr;
+  br.autos = k ? k->d_autos : nullptr;
+  br.fft_rgsw = k ? k->d_fft_rgsw : nullptr;
+  br.fft_autos = k ? k->d_fft_autos : nullptr;
+  br.fft_tw = c->d_fft;
+}
+
 void free_key_arrays(pz_key *k) {
+  cudaFree(k->d_fft_rgsw);
+  cudaFree(k->d_fft_autos);
   cudaFree(k->d_rgsw);
   cudaFree(k->d_autos);
   cudaFree(k->d_ksk);
@@ -256,8 +283,7 @@ pz_status run_gates(pz_ctx *c, const pz_key *k, const unsigned char *d_gates, co
                     u64 *d_out, size_t count, u32 *d_ks_out, u64 *d_rlwe, cudaStream_t s, u32 *d_ks_scratch,
                     bool raw, const u32 *in0, const u32 *in1, const u32 *out_idx) {
   pz::BrParams br = c->br;
-  br.rgsw = k->d_rgsw;
-  br.autos = k->d_autos;
+  pz::br_bind_key(c, k, br);
   br.out_idx = out_idx;
   pz::KsParams ks = c->ks;
   pz::ks_bind_key(c, k, ks);
@@ -360,6 +386,7 @@ pz_status pz_ctx_create_ex(int id, int device, uint64_t root, pz_ctx **out) {
   CK_CREATE(cudaMemcpy(c->d_tw, tw.data(), 4 * N * 8, cudaMemcpyHostToDevice));
   CK_CREATE(cudaMalloc(&c->d_dlog, dlog.size() * 2));
   CK_CREATE(cudaMemcpy(c->d_dlog, dlog.data(), dlog.size() * 2, cudaMemcpyHostToDevice));
+  if (c->logn == 11 && P.rlrg_d_a == 1 && P.rlrg_d_b == 1 && P.auto_d == 1) CK_CREATE(pz::fft_tables(&c->d_fft));
   CK_CREATE(cudaMalloc(&c->d_err, sizeof(u32)));
   CK_CREATE(cudaMemset(c->d_err, 0, sizeof(u32)));
   CK_CREATE(cudaMalloc(&c->d_tv, tv.size() * 8));
@@ -429,7 +456,7 @@ void pz_ctx_destroy(pz_ctx *c) {
   if (!c) return;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  cudaFree(c->d_tw); cudaFree(c->d_dlog); cudaFree(c->d_tv); cudaFree(c->d_err);
+  cudaFree(c->d_tw); cudaFree(c->d_fft); cudaFree(c->d_dlog); cudaFree(c->d_tv); cudaFree(c->d_err);
   cudaFree(c->d_c0); cudaFree(c->d_c1); cudaFree(c->d_out); cudaFree(c->d_gates); cudaFree(c->d_ks);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -529,6 +556,7 @@ pz_status pz_key_upload(pz_ctx *c, const pz_server_key_view *v, pz_key **out) {
   if ((e = cudaMemcpy(k->d_ksk, ksk32.data(), ksk32.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
     return cleanup(PZ_ERR_CUDA, std::string("ksk copy: ") + cudaGetErrorString(e));
   pz::build_ksk8(c, k, c->stream);
+  pz::build_fft_key(c, k, c->stream);
   *out = k;
   return PZ_OK;
 }
@@ -599,6 +627,7 @@ pz_status pz_key_upload_seeded(pz_ctx *c, const pz_seeded_server_key_view *v, pz
   cudaFree(d_stage);
   d_stage = nullptr;
   pz::build_ksk8(c, k, c->stream);
+  pz::build_fft_key(c, k, c->stream);
   *out = k;
   return PZ_OK;
 }
@@ -678,8 +707,7 @@ pz_status pz_blind_rotate_batch_device(pz_ctx *c, const pz_key *k, const uint32_
   if (s != PZ_OK) return s;
   PZ_CK(c, cudaSetDevice(c->device));
   pz::BrParams br = c->br;
-  br.rgsw = k->d_rgsw;
-  br.autos = k->d_autos;
+  pz::br_bind_key(c, k, br);
   br.out_idx = nullptr;
   const bool d1 = c->P.rlrg_d_a == 1 && c->P.rlrg_d_b == 1 && c->P.auto_d == 1;
   PZ_CK(c, pz::launch_pbs((int)c->logn, d1, br, d_ks, c->P.lwe_n + 1, d_test_vec, d_out, count, nullptr,
@@ -694,7 +722,8 @@ pz_status pz_ctx_autotune(pz_ctx *c, const pz_key *k, size_t batch, int *variant
   std::lock_guard<std::mutex> lock(c->mu);
   PZ_CK(c, cudaSetDevice(c->device));
   const bool d1 = c->P.rlrg_d_a == 1 && c->P.rlrg_d_b == 1 && c->P.auto_d == 1;
-  const int nv = (c->logn == 11 && d1) ? pz::PBS_MAX_VARIANT + 1 : 1;
+  // the distinct launch shapes
+  const std::vector<int> shapes = (c->logn == 11 && d1) ? std::vector<int>{0, pz::PBS_SPLIT} : std::vector<int>{0};
   // synthetic key-switched LWEs, uniform mod q_ks, and gate codes
   const u32 cols = c->P.lwe_n + 1;
   std::vector<u32> ks(batch * cols);
@@ -714,12 +743,12 @@ pz_status pz_ctx_autotune(pz_ctx *c, const pz_key *k, size_t batch, int *variant
   if (e == cudaSuccess) e = cudaEventCreate(&a);
   if (e == cudaSuccess) e = cudaEventCreate(&b);
   pz::BrParams br = c->br;
-  br.rgsw = k->d_rgsw;
-  br.autos = k->d_autos;
+  pz::br_bind_key(c, k, br);
   br.out_idx = nullptr;
   double best = 1e30;
   int bv = c->pbs_variant;
-  for (int v = 0; v < nv && e == cudaSuccess; v++) {
+  for (int v : shapes) {
+    if (e != cudaSuccess) break;
     // a batch of at least one wave is timed in whole waves of this shape (a
     // partial last wave would charge the shape for the batch's remainder):
     // the largest multiple of the shape's resident items not above the batch
@@ -911,8 +940,7 @@ pz_status pz_rlwe_by_rgsw_device(pz_ctx *c, const pz_key *k, uint64_t *d_rlwe, c
   if (s != PZ_OK) return s;
   PZ_CK(c, cudaSetDevice(c->device));
   pz::BrParams br = c->br;
-  br.rgsw = k->d_rgsw;
-  br.autos = k->d_autos;
+  pz::br_bind_key(c, k, br);
   const bool d1 = c->P.rlrg_d_a == 1 && c->P.rlrg_d_b == 1 && c->P.auto_d == 1;
   PZ_CK(c, pz::launch_ext_product((int)c->logn, d1, br, d_rlwe, d_idx, count, trivial, pick(c, stream),
                                   c->pbs_variant));
@@ -926,8 +954,7 @@ pz_status pz_rlwe_auto_device(pz_ctx *c, const pz_key *k, uint64_t *d_rlwe, cons
   if (s != PZ_OK) return s;
   PZ_CK(c, cudaSetDevice(c->device));
   pz::BrParams br = c->br;
-  br.rgsw = k->d_rgsw;
-  br.autos = k->d_autos;
+  pz::br_bind_key(c, k, br);
   const bool d1 = c->P.rlrg_d_a == 1 && c->P.rlrg_d_b == 1 && c->P.auto_d == 1;
   PZ_CK(c, pz::launch_auto((int)c->logn, d1, br, d_rlwe, d_slot, count, trivial, pick(c, stream), c->pbs_variant));
   return PZ_OK;

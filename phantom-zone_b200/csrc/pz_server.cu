@@ -71,6 +71,7 @@ struct pz_server {
   size_t key_budget = SIZE_MAX, managed_bytes = 0;
   u64 use_clock = 0, key_imports = 0, key_evictions = 0;
   bool descs_dirty = false;
+  bool fft = false;     // every session with a resident key has its FFT form
   bool ks_mma = false;  // every session with a resident key has its KSK byte planes: tensor-core key switch
   int logn = -1;
   bool d1 = true;
@@ -228,17 +229,19 @@ pz_status upload_descs(pz_server *s) {
   for (size_t i = 0; i < s->sessions.size(); i++) {
     const auto &se = s->sessions[i];
     br[i] = se.ctx->br;  // a session without a resident key gets no items: null key pointers
-    br[i].rgsw = se.key ? se.key->d_rgsw : nullptr;
-    br[i].autos = se.key ? se.key->d_autos : nullptr;
+    pz::br_bind_key(se.ctx, se.key, br[i]);
     br[i].out_idx = nullptr;
     ks[i] = se.ctx->ks;
     ks[i].ksk = nullptr;
     if (se.key) pz::ks_bind_key(se.ctx, se.key, ks[i]);
   }
-  bool mma = s->max_d <= 16;
-  for (size_t i = 0; i < s->sessions.size(); i++)
+  bool mma = s->max_d <= 16, fft = true;
+  for (size_t i = 0; i < s->sessions.size(); i++) {
     if (s->sessions[i].key && !s->sessions[i].key->d_ksk8) mma = false;
+    if (s->sessions[i].key && !s->sessions[i].key->d_fft_rgsw) fft = false;
+  }
   s->ks_mma = mma;
+  s->fft = fft;
   s->descs_dirty = false;
   cudaFree(s->d_br);
   cudaFree(s->d_ksp);
@@ -463,7 +466,7 @@ pz_status run_items(pz_server *s, const std::vector<Item> &items) {
     const int variant = (s->logn == 11 && s->d1 && n <= (size_t)s->sm_count / 2) ? pz::PBS_SPLIT : s->pbs_variant;
     e = pz::launch_pbs_ragged(s->logn, s->d1, s->d_br, (const u32 *)(d + lay.desc), s->max_br_q, s->max_n,
                               s->d_ksout, s->ks_stride, d + lay.gate, s->d_arena, (const u32 *)(d + lay.out), n,
-                              s->grid_limit, s->stream, variant);
+                              s->grid_limit, s->stream, variant, s->fft);
     if (e != cudaSuccess) return s->cuda("launch_pbs_ragged", e);
     s->launches += 2;
   }
@@ -503,7 +506,7 @@ void select_jobs(pz_server *s, std::vector<pz_server::Job *> &run) {
     }
   }
   const size_t sms = (size_t)std::max(1, s->sm_count);
-  const size_t cps = (s->pbs_variant == 0 || s->pbs_variant == pz::PBS_BULK) ? 2 : s->pbs_variant == 2 ? 4 : 3;
+  const size_t cps = (s->pbs_variant == 0 || s->pbs_variant == 4) ? 2 : s->pbs_variant == 2 ? 4 : 3;
   const size_t wave = sms * cps;
   const size_t cap = g <= wave ? std::max<size_t>(1, (g + sms - 1) / sms) * sms : (g + wave - 1) / wave * wave;
   std::stable_sort(opt.begin(), opt.end(), [](const pz_server::Job *a, const pz_server::Job *b) {
@@ -832,7 +835,7 @@ pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid
   int bv = s->pbs_variant, bg = s->grid_limit;
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-  const int grids[2] = {0, 2 * sms};
+  const int grids[2] = {0, 4 * sms};
   auto CK = [&](cudaError_t e, const char *w) {
     if (e != cudaSuccess && st == PZ_OK) st = s->cuda(w, e);
     return e == cudaSuccess;
@@ -844,15 +847,12 @@ pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid
       CK(cudaMemcpy(d_out, outi.data(), batch * 4, cudaMemcpyHostToDevice), "cudaMemcpy") &&
       CK(cudaMemcpy(d_g, g.data(), batch, cudaMemcpyHostToDevice), "cudaMemcpy") &&
       CK(cudaEventCreate(&a), "cudaEventCreate") && CK(cudaEventCreate(&b), "cudaEventCreate")) {
-    // one-CTA shapes (register caps 2/3/4 CTAs per SM) and the staged-key shape
-    const int shapes[4] = {0, 1, 2, pz::PBS_BULK};
-    const int nv = (s->logn == 11 && s->d1) ? 4 : 1;
-    for (int vi = 0; vi < nv && st == PZ_OK; vi++) {
-      const int v = shapes[vi];
+    {
+      // one launch shape (0) with a CTA per gate, or as many CTAs as are resident
       for (int gi = 0; gi < 2 && st == PZ_OK; gi++) {
         auto launch = [&]() {
           return pz::launch_pbs_ragged(s->logn, s->d1, s->d_br, d_desc, s->max_br_q, s->max_n, d_ks, s->ks_stride,
-                                       d_g, s->d_arena, d_out, batch, grids[gi], s->stream, v);
+                                       d_g, s->d_arena, d_out, batch, grids[gi], s->stream, 0, s->fft);
         };
         if (!CK(launch(), "launch_pbs_ragged")) break;  // warm-up
         if (!CK(cudaEventRecord(a, s->stream), "cudaEventRecord")) break;
@@ -864,7 +864,7 @@ pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid
         cudaEventElapsedTime(&ms, a, b);
         if (ms / 2 < best) {
           best = ms / 2;
-          bv = v;
+          bv = 0;
           bg = grids[gi];
         }
       }

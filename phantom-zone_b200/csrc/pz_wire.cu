@@ -110,6 +110,7 @@ pz_status pz_key_import(pz_ctx *c, const void *buf, size_t size, pz_key **out) {
     return pz::cuda_fail(c, "pz_key_import", e);
   }
   pz::build_ksk8(c, k, c->stream);  // derived on the device; the blob carries only the u32 rows
+  pz::build_fft_key(c, k, c->stream);
   *out = k;
   return PZ_OK;
 }
