@@ -4,6 +4,8 @@
 #include <cmath>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "pz_blind.cuh"
 #include "pz_fft.cuh"
 #include "pz_internal.h"
@@ -104,86 +106,204 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
-// The operations of a blind rotation, on a CTA of T threads.
-// Shared memory: two exchange buffers (M complex words each) | a's digits (N
-// ints) | twiddles | the schedule.  Between an operation and the next, b's
-// digits (N ints) or the permuted b of an automorphism (N words) sit in the
-// exchange buffer that the last transform did not use.
+// The operations of a blind rotation.  A group of T threads transforms one
+// polynomial at a time.
+//   QUAD   a CTA of one group, four CTAs per SM: both forward transforms, then
+//          for a and for b the three limbs of the key one after the other.
+//   TRIO   a CTA of three groups, one for each limb, one CTA per SM: groups 0
+//          and 1 transform the two digit polynomials, every group multiplies
+//          both with its limb and transforms back (a, then b), and the groups'
+//          parts are added up.  For batches that leave QUAD's places empty.
+//   SPLIT  TRIO on a cluster of two CTAs, rank 0 for a and rank 1 for b: both
+//          transform both digit polynomials, and the new digits go to both.
+//          For batches that leave SMs idle.
+// Shared memory: exchange buffers (M complex words; two per group, one in SPLIT) | what passes from an operation to the next: b or its digits
+// (N words), a's digits (N ints) | TRIO and SPLIT: the groups' next blocks of
+// the key | twiddles | the schedule.  In TRIO and SPLIT the second part is
+// there twice: an operation reads one and writes the other, while other threads
+// may still be reading.  QUAD has no room for it: b (or its digits) sits in the
+// exchange buffer that the last transform did not use, and is read before the
+// operation's first barrier.
+// The key: QUAD loads it into registers, four CTAs covering for each other;
+// TRIO early into more of them (each block while the digits or the output before
+// are transformed); SPLIT has each block copied (cp.async.bulk) into shared
+// memory as soon as the one before has been used, an operation ahead.
 // ---------------------------------------------------------------------------
-constexpr size_t X_WORDS = 4 * M, DA_WORDS = N / 2, TWS_WORDS = 2 * TW_WORDS;
-constexpr size_t FFT_WORDS = X_WORDS + DA_WORDS + TWS_WORDS;
-struct Smem {
-  u64 *x;  // the buffers
-  int *da;
-  cplx *tw;
-  unsigned short *ops;
-  u32 *nops;
-  __device__ __forceinline__ explicit Smem(u64 *s)
-      : x(s), da((int *)(s + X_WORDS)), tw((cplx *)(s + X_WORDS + DA_WORDS)),
-        ops((unsigned short *)(s + FFT_WORDS) + 2), nops((u32 *)(s + FFT_WORDS)) {}
-  __device__ __forceinline__ u64 *buffer(u32 q) const { return x + q * (2 * M); }
+enum Form { QUAD, TRIO, SPLIT };
+template <Form F>
+struct Shape {
+  static constexpr int GROUPS = F == QUAD ? 1 : LIMBS, THREADS = GROUPS * T, CTAS = F == QUAD ? 4 : 1;
+  static constexpr size_t X_WORDS = (F == SPLIT ? 1 : 2) * GROUPS * 2 * M;
+  static constexpr size_t PASS_WORDS = F == QUAD ? N / 2 : 2 * (N + N / 2);
+  static constexpr size_t KEY_WORDS = F == SPLIT ? GROUPS * 4 * M : 0;
+  static constexpr size_t WORDS = X_WORDS + PASS_WORDS + KEY_WORDS + 2 * TW_WORDS;
+  // tensor memory: the transformed digit polynomials (64 columns), the turns
+  // (32 per group), then QUAD: the permuted b of an automorphism until it is
+  // added, TRIO and SPLIT: each group's part of each output (32 columns each)
+  static constexpr u32 SPEC = 0, TURN = 64, PART = TURN + 32 * GROUPS, COLS = F == QUAD ? 128 : 512;
+  static size_t smem_bytes(u32 br_q, u32 n) {
+    return WORDS * 8 + (((size_t)4 + (n + br_q / 2 + 1) * 2 + 15) & ~(size_t)15);
+  }
 };
-static size_t fft_smem_bytes(u32 br_q, u32 n) {
-  return FFT_WORDS * 8 + (((size_t)4 + (n + br_q / 2 + 1) * 2 + 15) & ~(size_t)15);
-}
-__device__ __forceinline__ void load_twiddles(const BrParams &P, const Smem &S) {
-  for (int i = threadIdx.x; i < TW_WORDS; i += T) S.tw[i] = ldc((const cplx *)P.fft_tw + i);
+template <Form F>
+struct Smem {
+  typedef Shape<F> H;
+  u64 *x;  // the groups' buffers
+  __device__ __forceinline__ explicit Smem(u64 *s) : x(s) {}
+  __device__ __forceinline__ cplx *buffer(int g, u32 q) const {
+    return (cplx *)(x + (F == SPLIT ? (u32)g : 2 * g + q) * (2 * M));
+  }
+  __device__ __forceinline__ cplx *key(int g) const { return (cplx *)(x + H::X_WORDS + H::PASS_WORDS + g * 4 * M); }
+  // what passes to operation i, before whose first transform the group's next buffer is q: an
+  // automorphism's permuted b, or the digits of b; the digits of a
+  __device__ __forceinline__ long long *ub(u32 i, u32 q) const {
+    return F == QUAD ? (long long *)buffer(0, q ^ 1) : (long long *)(x + H::X_WORDS + (i & 1) * (N + N / 2));
+  }
+  __device__ __forceinline__ int *db(u32 i, u32 q) const { return (int *)ub(i, q); }
+  __device__ __forceinline__ int *da(u32 i) const {
+    return F == QUAD ? (int *)(x + H::X_WORDS) : (int *)(x + H::X_WORDS + (i & 1) * (N + N / 2) + N);
+  }
+  __device__ __forceinline__ cplx *tw() const { return (cplx *)(x + H::X_WORDS + H::PASS_WORDS + H::KEY_WORDS); }
+  __device__ __forceinline__ u32 *nops() const { return (u32 *)(x + H::WORDS); }
+  __device__ __forceinline__ unsigned short *ops() const { return (unsigned short *)(nops() + 1); }
+};
+
+namespace cg = cooperative_groups;
+template <int V>
+struct Int {
+  static constexpr int value = V;
+};
+// Barrier of the CTA that also orders tensor memory between warps.
+__device__ __forceinline__ void op_sync() {
+  tmem_wait_store();
+  tmem_before_barrier();
+  __syncthreads();
+  tmem_after_barrier();
 }
 
-// One operation `op` on what S holds for it, leaving there what the next one,
-// `nx`, reads: the digits of both polynomials for an external product; a's
-// digits and b, both under X -> X^k, for an automorphism; after the last
-// operation (OP_END) emit(o, i, v) gets coefficient i of output o (0: a, 1: b)
-// in [0, Q).  q: the buffer the next transform writes (b is in the other one).
-// tm: this warp's tensor memory.
-// The body is kept small (one copy of each transform): larger forms, with two
-// polynomials at a time, spent a third of their issue slots waiting for
-// instructions.
+// The digits of one polynomial (half 0: a's, or their low halves under an
+// automorphism; half 1: b's, or the high halves of a's).
+template <Form F>
+__device__ __forceinline__ void load_digits(int (&v)[16], int half, u32 i, u32 q, bool is_auto, const Smem<F> &S,
+                                            const Place &p) {
+  const int *d = half == 0 || is_auto ? S.da(i) : S.db(i, q);
+#pragma unroll
+  for (int m = 0; m < 16; m++) v[m] = d[p.t + T * m];
+  if (is_auto) {
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+      const int hi = (v[m] + (1 << (AUTO_CUT - 1))) >> AUTO_CUT;
+      v[m] = half ? hi : v[m] - (hi << AUTO_CUT);
+    }
+  }
+}
+__device__ __forceinline__ void to_complex(cplx (&z)[8], const int (&v)[16]) {
+#pragma unroll
+  for (int m = 0; m < 16; m++) (m < 8 ? z[m & 7].r : z[m & 7].i) = i2d(v[m]);
+}
+
+// points r and r + 1: the transformed digits (tensor memory) times the keys
+__device__ __forceinline__ void products(cplx (&z)[8], int r, u32 spec, const cplx &a0, const cplx &b0, const cplx &a1,
+                                         const cplx &b1) {
+  cplx u0, u1, v0, v1;
+  tmem_load4(spec + 8 * r, u0, u1, v0, v1);
+  z[r].r = fma(u0.r, a0.r, fma(-u0.i, a0.i, fma(v0.r, b0.r, -(v0.i * b0.i))));
+  z[r].i = fma(u0.r, a0.i, fma(u0.i, a0.r, fma(v0.r, b0.i, v0.i * b0.r)));
+  z[r + 1].r = fma(u1.r, a1.r, fma(-u1.i, a1.i, fma(v1.r, b1.r, -(v1.i * b1.i))));
+  z[r + 1].i = fma(u1.r, a1.i, fma(u1.i, a1.r, fma(v1.r, b1.i, v1.i * b1.r)));
+}
+
+// What becomes of output o of an operation: `nx` (the next one, i + 1) reads
+// digits, an automorphism X -> X^k those of a and b itself, permuted; after
+// the last operation (OP_END) emit(o, c, v) gets coefficient c in [0, Q).
+struct Next {
+  bool end, is_auto;
+  u32 k;
+  __device__ __forceinline__ Next(u32 nx, const BrParams &P)
+      : end(nx == OP_END), is_auto(!end && (nx & OP_AUTO)), k(is_auto ? P.auto_k[nx & OP_SLOT] : 1u) {}
+};
+// C values of output o: coefficients t + T (m0 + m), as sums of the limbs.  q:
+// the group's next buffer after the operation.  far_bar: the other CTA's barrier
+// for the digits sent there.
+template <int C, Form F, class Emit>
+__device__ __forceinline__ void pass_on(const u64 (&acc)[C], int m0, int o, u32 i, u32 q, const Next &nx,
+                                        const Smem<F> &S, u32 far_bar, int rank, const Place &p, const Emit &emit) {
+  long long c[C];
+  u32 worst = 0, at = (u32)(p.t + T * m0) * nx.k;
+#pragma unroll
+  for (int m = 0; m < C; m++, at += T * nx.k) {
+    c[m] = settle(acc[m]);
+    if (at & N) c[m] = -c[m];  // X^N = -1
+    worst = max(worst, edge(c[m]));
+  }
+  at = (u32)(p.t + T * m0) * nx.k;
+  if (nx.end) {
+#pragma unroll
+    for (int m = 0; m < C; m++) {
+      const long long v = centre(c[m]);
+      emit(o, p.t + T * (m0 + m), (u64)(v < 0 ? v + (long long)Q_N2048 : v));
+    }
+  } else if (o == 1 && nx.is_auto) {
+    long long *dst = S.ub(i + 1, q);
+#pragma unroll
+    for (int m = 0; m < C; m++, at += T * nx.k) dst[at & (N - 1)] = c[m];
+  } else {
+    if (worst > EDGE) {
+#pragma unroll
+      for (int m = 0; m < C; m++) c[m] = centre(c[m]);
+    }
+    // (c + half) >> 37 or 30, see digit()
+    const long long half = nx.is_auto ? 1ll << (AUTO_IGN - 1) : 1ll << (RLRG_IGN - 1);
+    const int more = nx.is_auto ? 0 : RLRG_IGN - AUTO_IGN;
+    int *dst = o ? S.db(i + 1, q) : S.da(i + 1);
+    const u32 far = F == SPLIT ? cluster_addr(dst, rank ^ 1) : 0;
+#pragma unroll
+    for (int m = 0; m < C; m++, at += T * nx.k) {
+      const int d = (int)((c[m] + half) >> AUTO_IGN) >> more;
+      dst[at & (N - 1)] = d;
+      if (F == SPLIT) remote_store(far + 4 * (at & (N - 1)), d, far_bar);
+    }
+  }
+}
+
+// Operation i, `op`, on what S holds for it, leaving there what the next one
+// reads.  q: the exchange buffer the group's next transform writes.  tm: this
+// warp's tensor memory.  The bodies are kept small (one copy of each
+// transform): with larger ones, two polynomials at a time, a third of the issue
+// slots waited for instructions.
 template <class Emit>
-__device__ __forceinline__ void fft_op(u32 op, u32 nx, const cplx *key, const cplx *next_key, const BrParams &P,
-                                       const Smem &S, u32 &q, u32 tm, const Place &p,
-                                       const Emit &emit) {
+__device__ __forceinline__ void op_quad(u32 i, u32 op, u32 nx_op, const cplx *key, const cplx *next_key,
+                                        const BrParams &P, const Smem<QUAD> &S, u32 &q, u32 tm, const Place &p,
+                                        const Emit &emit) {
+  typedef Shape<QUAD> H;
   const int t = p.t;
   const bool is_auto = (op & OP_AUTO) != 0;
   cplx z[8];
   {
     int y[16];
-    if (is_auto) {
-      const u64 *ub = S.buffer(q ^ 1);
+    load_digits(y, 0, i, q, is_auto, S, p);
+    to_complex(z, y);
+    load_digits(y, 1, i, q, is_auto, S, p);
+    if (is_auto) {  // b, before its buffer is written
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         u64 b[8];
 #pragma unroll
-        for (int m = 0; m < 8; m++) b[m] = ub[t + T * (8 * h + m)];
-        tmem_store8(tm + SPEC_COLS + 16 * h, b);
-      }
-#pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const int d = S.da[t + T * m];
-        y[m] = (d + (1 << (AUTO_CUT - 1))) >> AUTO_CUT;
-        (m < 8 ? z[m & 7].r : z[m & 7].i) = i2d(d - (y[m] << AUTO_CUT));
-      }
-    } else {
-      const int *db = (const int *)S.buffer(q ^ 1);
-#pragma unroll
-      for (int m = 0; m < 16; m++) {
-        (m < 8 ? z[m & 7].r : z[m & 7].i) = i2d(S.da[t + T * m]);
-        y[m] = db[t + T * m];
+        for (int m = 0; m < 8; m++) b[m] = (u64)S.ub(i, q)[t + T * (8 * h + m)];
+        tmem_store8(tm + H::PART + 16 * h, b);
       }
     }
 #pragma unroll 1
-    for (int i = 0; i < 2; i++) {
-      forward(z, (cplx *)S.buffer(q), S.tw, p);
+    for (int half = 0; half < 2; half++) {
+      forward<H::GROUPS>(z, S.buffer(0, q), S.tw(), p);
       q ^= 1;
 #pragma unroll
-      for (int c = 0; c < 4; c++) tmem_store2(tm + 16 * c + 8 * i, z[2 * c], z[2 * c + 1]);
-#pragma unroll
-      for (int m = 0; m < 16; m++) (m < 8 ? z[m & 7].r : z[m & 7].i) = i2d(y[m]);
+      for (int c = 0; c < 4; c++) tmem_store2(tm + H::SPEC + 16 * c + 8 * half, z[2 * c], z[2 * c + 1]);
+      to_complex(z, y);
     }
     tmem_wait_store();
   }
-  const bool end = nx == OP_END, nx_auto = !end && (nx & OP_AUTO);
-  const u32 k = nx_auto ? P.auto_k[nx & OP_SLOT] : 1u;
+  const Next nx(nx_op, P);
   const cplx *kp = key + t;
 #pragma unroll 1
   for (int o = 0; o < 2; o++) {
@@ -194,7 +314,7 @@ __device__ __forceinline__ void fft_op(u32 op, u32 nx, const cplx *key, const cp
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         u64 b[8];
-        tmem_load8(tm + SPEC_COLS + 16 * h, b);
+        tmem_load8(tm + H::PART + 16 * h, b);
 #pragma unroll
         for (int m = 0; m < 8; m++) acc[8 * h + m] = b[m];
       }
@@ -218,17 +338,10 @@ __device__ __forceinline__ void fft_op(u32 op, u32 nx, const cplx *key, const cp
 #pragma unroll
       for (int c = 0; c < 4; c++) {
         if (c < 3) fetch(c + 1);
-        cplx px[2], py[2];
-        tmem_load4(tm + 16 * c, px[0], px[1], py[0], py[1]);
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const cplx &u = px[e], &v = py[e], &a = kx[c & 1][e], &b = ky[c & 1][e];
-          z[2 * c + e].r = fma(u.r, a.r, fma(-u.i, a.i, fma(v.r, b.r, -(v.i * b.i))));
-          z[2 * c + e].i = fma(u.r, a.i, fma(u.i, a.r, fma(v.r, b.i, v.i * b.r)));
-        }
+        products(z, 2 * c, tm + H::SPEC, kx[c & 1][0], ky[c & 1][0], kx[c & 1][1], ky[c & 1][1]);
       }
       kp += 2 * M;
-      inverse(z, (cplx *)S.buffer(q), S.tw, p);
+      inverse<H::GROUPS>(z, S.buffer(0, q), S.tw(), p);
       q ^= 1;
       if (l == 0) {
 #pragma unroll
@@ -241,39 +354,158 @@ __device__ __forceinline__ void fft_op(u32 op, u32 nx, const cplx *key, const cp
         for (int m = 0; m < 16; m++) add_limb2(acc[m], m < 8 ? z[m & 7].r : z[m & 7].i);
       }
     }
-    long long c[16];
-    u32 worst = 0, at = (u32)t * k;
-#pragma unroll
-    for (int m = 0; m < 16; m++, at += T * k) {
-      c[m] = settle(acc[m]);
-      if (at & N) c[m] = -c[m];  // X^N = -1
-      worst = max(worst, edge(c[m]));
-    }
-    at = (u32)t * k;
-    if (end) {
-#pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const long long v = centre(c[m]);
-        emit(o, t + T * m, (u64)(v < 0 ? v + (long long)Q_N2048 : v));
-      }
-    } else if (o == 1 && nx_auto) {
-      long long *dst = (long long *)S.buffer(q);
-#pragma unroll
-      for (int m = 0; m < 16; m++, at += T * k) dst[at & (N - 1)] = c[m];
-    } else {
-      if (worst > EDGE) {
-#pragma unroll
-        for (int m = 0; m < 16; m++) c[m] = centre(c[m]);
-      }
-      // (c + half) >> 37 or 30, see digit()
-      const long long half = nx_auto ? 1ll << (AUTO_IGN - 1) : 1ll << (RLRG_IGN - 1);
-      const int more = nx_auto ? 0 : RLRG_IGN - AUTO_IGN;
-      int *dst = o ? (int *)S.buffer(q) : S.da;
-#pragma unroll
-      for (int m = 0; m < 16; m++, at += T * k) dst[at & (N - 1)] = (int)((c[m] + half) >> AUTO_IGN) >> more;
-    }
+    // the operation's eight transforms leave q as it was; the next operation
+    // starts with the other buffer
+    pass_on(acc, 0, o, i, q ^ 1, nx, S, 0u, 0, p, emit);
   }
   q ^= 1;
+}
+
+// The waits of SPLIT, each bounded (about a second): one that runs out
+// sets DEVERR_MBAR_TIMEOUT, and the CTA goes on without waiting any more (its
+// results are not valid), so every barrier is met and the kernel ends.
+struct Waits {
+  u64 *key;   // one per group: its block of the key has arrived
+  u64 *msg;   // SPLIT, by parity of the operation: the other CTA's digits for it
+  int *lost;  // shared: a wait ran out
+  u32 *err;
+  u32 key_phase, msg_phase;  // completed phases (msg: bit per barrier)
+  bool fresh;                // the item's first operation: no message
+  int rank;
+  __device__ __forceinline__ void ran_out() const {
+    *(volatile int *)lost = 1;
+    atomicOr(err, DEVERR_MBAR_TIMEOUT);
+  }
+  // the group's block of the key
+  __device__ __forceinline__ void wait_key(int g) {
+    if (!*(volatile int *)lost && !mbar_wait(key + g, key_phase & 1)) ran_out();
+    key_phase++;
+  }
+  __device__ __forceinline__ void first_key(const cplx *k, const Smem<SPLIT> &S, const Place &p) const {
+    __syncthreads();  // the barriers are there; the last item's blocks have been used
+    if (p.t == 0) {
+      fence_proxy_async_smem();
+      bulk_load(S.key(p.g), k + (size_t)(rank * LIMBS + p.g) * 2 * M, 2 * M * (u32)sizeof(cplx),
+                key + p.g);
+    }
+  }
+  // SPLIT, before operation i = the one whose parity `at` is: the other CTA's
+  // digits.  Rank 0 sends a's digits for every operation, rank 1 b's for an
+  // external product and one word for an automorphism, so that neither gets two
+  // operations ahead.
+  __device__ __forceinline__ void message(u32 i, u32 op) {
+    const u32 b = i & 1;
+    if (!fresh) {
+      if (threadIdx.x == 0) mbar_expect(msg + b, rank == 1 || !(op & OP_AUTO) ? N * 4u : 4u);
+      if (!*(volatile int *)lost && !mbar_wait_cluster(msg + b, (msg_phase >> b) & 1)) ran_out();
+      msg_phase ^= 1u << b;
+    }
+    fresh = false;
+  }
+};
+
+template <Form F, class Emit>
+__device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, const cplx *key, const cplx *next_key,
+                                        const BrParams &P, const Smem<F> &S, Waits &W, int rank, u32 &q, u32 tm,
+                                        const Place &p, const Emit &emit) {
+  typedef Shape<F> H;
+  const int t = p.t, g = p.g;
+  const bool is_auto = (op & OP_AUTO) != 0;
+  // the next operation's key, into L2 while this one is worked on
+  if (threadIdx.x == 0 && next_key) {
+    if (F == SPLIT) prefetch_l2(next_key + (size_t)rank * LIMBS * 2 * M, LIMBS * 2 * M * (u32)sizeof(cplx));
+    else prefetch_l2(next_key, (u32)(KEY_BLOCK * sizeof(cplx)));
+  }
+  cplx z[8];
+  if (g < 2) {
+    int v[16];
+    load_digits(v, g, i, q, is_auto, S, p);
+    to_complex(z, v);
+  }
+  // this group's limb of the key for the first output
+  const cplx *kp = key + (size_t)g * 2 * M + t;
+  cplx kx[8], ky[8];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      kx[r] = ld_key(kp + (2 * r) * T);
+      ky[r] = ld_key(kp + (2 * r + 1) * T);
+    }
+  };
+  if (F == TRIO) fetch();
+  if (g < 2) {
+    forward<H::GROUPS>(z, S.buffer(g, q), S.tw(), p);
+    if (F == TRIO) q ^= 1;
+#pragma unroll
+    for (int c = 0; c < 4; c++) tmem_store2(tm + H::SPEC + 16 * c + 8 * g, z[2 * c], z[2 * c + 1]);
+  }
+  op_sync();
+#pragma unroll 1
+  for (int o = F == SPLIT ? rank : 0; o < (F == SPLIT ? rank + 1 : 2); o++) {
+    if constexpr (F == SPLIT) {
+      W.wait_key(g);
+      const cplx *sp = S.key(g) + t;
+#pragma unroll
+      for (int r = 0; r < 8; r += 2)
+        products(z, r, tm + H::SPEC, sp[2 * r * T], sp[(2 * r + 1) * T], sp[(2 * r + 2) * T], sp[(2 * r + 3) * T]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 8; r += 2) products(z, r, tm + H::SPEC, kx[r], ky[r], kx[r + 1], ky[r + 1]);
+      if (o == 0) {
+        kp += (size_t)LIMBS * 2 * M;
+        fetch();
+      }
+    }
+    if constexpr (F == SPLIT) {
+      group_sync<H::GROUPS>(p);  // the exchange buffer and the block of the key have been used
+      if (t == 0 && next_key) {
+        fence_proxy_async_smem();
+        bulk_load(S.key(g), next_key + (size_t)(rank * LIMBS + g) * 2 * M, 2 * M * (u32)sizeof(cplx), W.key + g);
+      }
+    }
+    inverse<H::GROUPS>(z, S.buffer(g, q), S.tw(), p);
+    if (F == TRIO) q ^= 1;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      u64 v[8];
+#pragma unroll
+      for (int m = 0; m < 8; m++) v[m] = 0;
+      if (g == 0) {
+#pragma unroll
+        for (int m = 0; m < 8; m++) add_limb0(v[m], h ? z[m].i : z[m].r);
+      } else if (g == 1) {
+#pragma unroll
+        for (int m = 0; m < 8; m++) add_limb1(v[m], h ? z[m].i : z[m].r);
+      } else {
+#pragma unroll
+        for (int m = 0; m < 8; m++) add_limb2(v[m], h ? z[m].i : z[m].r);
+      }
+      tmem_store8(tm + H::PART + 32 * (3 * o + g) + 16 * h, v);
+    }
+  }
+  op_sync();
+  // the sums, dealt out to the groups: SPLIT values 0-7, 8-11, 12-15 of the
+  // output, TRIO the 16 of a and then those of b, 12, 12 and 8
+  const Next nx(nx_op, P);
+  const u32 far_bar = F == SPLIT ? cluster_addr(W.msg + ((i + 1) & 1), rank ^ 1) : 0;
+  auto finish = [&](auto count, int o, int m0) {
+    constexpr int C = decltype(count)::value;
+    u64 acc[C];
+    tmem_sum3<C>(tm + H::PART + 32 * 3 * o + 2 * m0, acc);
+    if (o == 1 && is_auto) {
+#pragma unroll
+      for (int m = 0; m < C; m++) acc[m] += (u64)S.ub(i, q)[t + T * (m0 + m)];
+    }
+    pass_on(acc, m0, o, i, q, nx, S, far_bar, rank, p, emit);
+  };
+  if (F == SPLIT) {
+    if (g == 0) finish(Int<8>(), rank, 0);
+    else finish(Int<4>(), rank, 4 + 4 * g);
+    if (rank == 1 && nx.is_auto && threadIdx.x == 0) remote_store(cluster_addr(S.db(i + 1, q), 0), 0, far_bar);
+  } else {
+#pragma unroll 1
+    for (int u = 3 * g; u < min(3 * g + 3, 8); u++) finish(Int<4>(), u >> 2, 4 * (u & 3));
+  }
 }
 
 __device__ __forceinline__ const cplx *op_key(const BrParams &P, u32 op) {
@@ -282,37 +514,39 @@ __device__ __forceinline__ const cplx *op_key(const BrParams &P, u32 op) {
 }
 
 // One gate bootstrap.
+template <Form F>
 __device__ __forceinline__ void fft_item(const BrParams &P, int ct, const u32 *kso, u32 gcode, u64 *out, u64 *rlwe_dbg,
-                                         u64 *smem, u32 tm) {
-  const int t = threadIdx.x;
-  const Smem S(smem);
-  const Place p(t, tm + SPEC_COLS + B_COLS);
+                                         u64 *smem, Waits &W, int rank, u32 tm) {
+  typedef Shape<F> H;
+  const Smem<F> S(smem);
+  const Place p(threadIdx.x % T, threadIdx.x / T, tm + H::TURN + 32 * (threadIdx.x / T));
   // the bucket arrays are only needed while the schedule is built: they, like
-  // its scratch (the first 2 N words), share the exchange buffers; the counters
-  // and keys take less than 10 KB of the first N words, the buckets' starts and
-  // members fit behind them
+  // its scratch (the first 2 N words), share the exchange buffers; of the first
+  // N words the counters and keys take less than 10 KB, and QUAD has the
+  // buckets' starts and members behind them
   SchedSmem sched;
-  sched.start = (unsigned short *)((char *)S.x + 10240);
+  sched.start = (unsigned short *)(F == QUAD ? smem + 1280 : smem + 2 * N);
   sched.list = sched.start + (P.br_q >> 1) + 1;
-  sched.ops = S.ops;
-  sched.nops = S.nops;
-  build_schedule<11, T>(P, kso, smem, sched);
+  sched.ops = S.ops();
+  sched.nops = S.nops();
+  build_schedule<11, H::THREADS>(P, kso, smem, sched);
   __syncthreads();
-  const u32 nops = *S.nops;
+  const u32 nops = *S.nops();
+  const unsigned short *ops = S.ops();
   u32 i = 0, q = 0;
   {
     // b: the rotated test polynomial, and the automorphisms of the trivial
     // RLWE (runtime.rs:625-642), which only permute it; a = 0
-    long long *from = (long long *)S.buffer(0), *to = (long long *)S.buffer(1);
+    long long *from = (long long *)smem, *to = from + N;
     const TestRotation tr(P, kso, gcode);
 #pragma unroll 1
-    for (int c = t; c < N; c += T) from[c] = (long long)tr.at((u32)c);
+    for (int c = threadIdx.x; c < N; c += H::THREADS) from[c] = (long long)tr.at((u32)c);
 #pragma unroll 1
-    for (; S.ops[i] & OP_AUTO; i++) {
-      const u32 k = P.auto_k[S.ops[i] & OP_SLOT];
+    for (; ops[i] & OP_AUTO; i++) {
+      const u32 k = P.auto_k[ops[i] & OP_SLOT];
       __syncthreads();
 #pragma unroll 1
-      for (int c = t; c < N; c += T) {
+      for (int c = threadIdx.x; c < N; c += H::THREADS) {
         const u32 at = (u32)c * k;
         to[at & (N - 1)] = (at & N) ? -from[c] : from[c];
       }
@@ -321,74 +555,97 @@ __device__ __forceinline__ void fft_item(const BrParams &P, int ct, const u32 *k
       to = x;
     }
     __syncthreads();
-    int d[N / T];
+    constexpr int PER = (N + H::THREADS - 1) / H::THREADS;
+    int d[PER];
 #pragma unroll
-    for (int m = 0; m < N / T; m++) d[m] = digit<RLRG_IGN>(centre(from[t + T * m]));
-    __syncthreads();  // the digits go where b was, or beside it
-    int *db = (int *)S.buffer(q ^ 1);
+    for (int m = 0; m < PER; m++) {
+      const int c = threadIdx.x + H::THREADS * m;
+      if (c < N) d[m] = digit<RLRG_IGN>(centre(from[c]));
+    }
+    if (F == QUAD) __syncthreads();  // b's digits go where b was, or beside it
 #pragma unroll
-    for (int m = 0; m < N / T; m++) {
-      db[t + T * m] = d[m];
-      S.da[t + T * m] = 0;
+    for (int m = 0; m < PER; m++) {
+      const int c = threadIdx.x + H::THREADS * m;
+      if (c < N) {
+        S.db(i, q)[c] = d[m];
+        S.da(i)[c] = 0;
+      }
     }
   }
   u64 *dst = out + (size_t)(P.out_idx ? P.out_idx[ct] : (u32)ct) * (N + 1);
+  auto emit = [&](int o, int c, u64 v) {
+    // sample extract at index 0 (pbs.rs:423-449)
+    if (o == 0) dst[c == 0 ? 1 : 1 + N - c] = c == 0 ? v : Q_N2048 - v;
+    else if (c == 0) dst[0] = v;
+    if (rlwe_dbg) rlwe_dbg[((size_t)ct * 2 + o) * N + c] = v;
+  };
+  if constexpr (F == SPLIT) {
+    W.first_key(op_key(P, ops[i]), S, p);
+    cg::this_cluster().sync();  // the other CTA is ready for what it is sent, too
+  }
+  W.fresh = true;
 #pragma unroll 1
   for (; i < nops; i++) {
-    const u32 op = S.ops[i], nx = i + 1 < nops ? (u32)S.ops[i + 1] : OP_END;
-    __syncthreads();
-    fft_op(op, nx, op_key(P, op), nx != OP_END ? op_key(P, nx) : nullptr, P, S, q, tm, p, [&](int o, int c, u64 v) {
-      // sample extract at index 0 (pbs.rs:423-449)
-      if (o == 0) dst[c == 0 ? 1 : 1 + N - c] = c == 0 ? v : Q_N2048 - v;
-      else if (c == 0) dst[0] = v;
-      if (rlwe_dbg) rlwe_dbg[((size_t)ct * 2 + o) * N + c] = v;
-    });
+    const u32 op = ops[i], nx = i + 1 < nops ? (u32)ops[i + 1] : OP_END;
+    const cplx *key = op_key(P, op), *next_key = nx != OP_END ? op_key(P, nx) : nullptr;
+    if constexpr (F == SPLIT) W.message(i, op);
+    op_sync();
+    if constexpr (F == QUAD) op_quad(i, op, nx, key, next_key, P, S, q, tm, p, emit);
+    else op_trio(i, op, nx, key, next_key, P, S, W, rank, q, tm, p, emit);
   }
 }
 
 // Tensor memory of the CTA: this warp's address of its lanes.
+template <Form F>
 __device__ __forceinline__ u32 tmem_begin(u32 *slot) {
-  if (threadIdx.x < 32) tmem_alloc(slot);
+  if (threadIdx.x < 32) tmem_alloc<Shape<F>::COLS>(slot);
   __syncthreads();
-  return *slot + ((threadIdx.x >> 5) << 21);  // lane 32 w in bits 16 and up
+  return *slot + (((threadIdx.x >> 5) & 3) << 21);  // lane 32 (w mod 4) in bits 16 and up
 }
+template <Form F>
 __device__ __forceinline__ void tmem_end(u32 *slot) {
   __syncthreads();
-  if (threadIdx.x < 32) tmem_free(*slot);
+  if (threadIdx.x < 32) tmem_free<Shape<F>::COLS>(*slot);
 }
 
-__global__ void __launch_bounds__(T, 4)
-    pbs_fft_kernel(BrParams P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out, int count,
-                   u64 *rlwe_dbg) {
-  extern __shared__ __align__(128) u64 smem[];
-  __shared__ u32 tmem_slot;
-  load_twiddles(P, Smem(smem));
-  const u32 tm = tmem_begin(&tmem_slot);
-  for (int ct = blockIdx.x; ct < count; ct += gridDim.x)
-    fft_item(P, ct, ks + (size_t)ct * ks_stride, gates[ct], out, rlwe_dbg, smem, tm);
-  tmem_end(&tmem_slot);
-}
-
-// Ragged batch: ciphertext ct uses the parameter set and server key of
-// descriptor item_desc[ct]; outputs scatter to out_idx[ct].
-__global__ void __launch_bounds__(T, 4)
-    pbs_fft_ragged_kernel(const BrParams *descs, const u32 *item_desc, const u32 *ks, u32 ks_stride,
-                          const unsigned char *gates, u64 *out, const u32 *out_idx, int count) {
+// The batch (gates of one key; descs and item_desc null), or a ragged one:
+// ciphertext ct uses the parameter set and server key of descriptor
+// item_desc[ct] and its output goes to out_idx[ct].  SPLIT: launched in
+// clusters of two, both on the same items.
+template <Form F>
+__global__ void __launch_bounds__(Shape<F>::THREADS, Shape<F>::CTAS)
+    pbs_fft_kernel(const __grid_constant__ BrParams P, const BrParams *descs, const u32 *item_desc, const u32 *out_idx,
+                   const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out, int count, u64 *rlwe_dbg) {
   extern __shared__ __align__(128) u64 smem[];
   __shared__ BrParams sp;
   __shared__ u32 tmem_slot;
-  const u32 tm = tmem_begin(&tmem_slot);
-  for (int ct = blockIdx.x; ct < count; ct += gridDim.x) {
+  const u32 tm = tmem_begin<F>(&tmem_slot);
+  const int rank = F == SPLIT ? (int)cg::this_cluster().block_rank() : 0;
+  __shared__ u64 bars[5];
+  __shared__ int lost;
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < 5; b++) mbar_init(bars + b, 1);
+    lost = 0;
+    mbar_init_fence();
+  }
+  Waits W{bars, bars + 3, &lost, nullptr, 0, 0, false, rank};
+  const int first = F == SPLIT ? blockIdx.x / 2 : blockIdx.x, step = F == SPLIT ? gridDim.x / 2 : gridDim.x;
+  for (int ct = first; ct < count; ct += step) {
     __syncthreads();  // the previous item is done with sp
     if (threadIdx.x == 0) {
-      sp = descs[item_desc[ct]];
-      sp.out_idx = out_idx;
+      sp = descs ? descs[item_desc[ct]] : P;
+      if (descs) sp.out_idx = out_idx;
     }
     __syncthreads();
-    if (ct == (int)blockIdx.x) load_twiddles(sp, Smem(smem));
-    fft_item(sp, ct, ks + (size_t)ct * ks_stride, gates[ct], out, nullptr, smem, tm);
+    if (ct == first) {
+      cplx *tw = Smem<F>(smem).tw();
+      for (int i = threadIdx.x; i < TW_WORDS; i += Shape<F>::THREADS) tw[i] = ldc((const cplx *)sp.fft_tw + i);
+    }
+    W.err = sp.err;
+    fft_item<F>(sp, ct, ks + (size_t)ct * ks_stride, gates[ct], out, rlwe_dbg, smem, W, rank, tm);
   }
-  tmem_end(&tmem_slot);
+  if (F == SPLIT) cg::this_cluster().sync();  // nobody leaves while the other may still send
+  tmem_end<F>(&tmem_slot);
 }
 
 }  // namespace fft
@@ -455,30 +712,68 @@ cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const
   return cudaGetLastError();
 }
 
+// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 6.6 up to 74 ciphertexts;
+// TRIO 8.8 for 148, 17.4 for 296; QUAD 15.1, 18.6, 24.4 and 30.6 for 148, 296, 444
+// and 592, and from there by the number of ciphertexts (20.7 k/s).
+static fft::Form fft_form(size_t resident, bool split) {
+  if (split) return fft::SPLIT;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return resident <= (size_t)sms ? fft::TRIO : fft::QUAD;
+}
+
 cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas) {
-  const size_t smem = fft::fft_smem_bytes(br_q, n);
-  const cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel, smem);
-  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, fft::pbs_fft_kernel, fft::T, smem);
+  typedef fft::Shape<fft::QUAD> H;
+  const size_t smem = H::smem_bytes(br_q, n);
+  const cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel<fft::QUAD>, smem);
+  return e != cudaSuccess ? e
+                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, fft::pbs_fft_kernel<fft::QUAD>,
+                                                                          H::THREADS, smem);
+}
+
+template <fft::Form F>
+static cudaError_t launch_form(const BrParams &P, const BrParams *d_descs, const u32 *item_desc, const u32 *out_idx,
+                               u32 br_q, u32 n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
+                               size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s) {
+  typedef fft::Shape<F> H;
+  const size_t smem = H::smem_bytes(br_q, n);
+  cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel<F>, smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(F == fft::SPLIT ? 2 * grid : grid));
+  cfg.blockDim = dim3(H::THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {2, 1, 1};
+  cfg.attrs = attr;
+  cfg.numAttrs = F == fft::SPLIT ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, fft::pbs_fft_kernel<F>, P, d_descs, item_desc, out_idx, ks, ks_stride, gates, out,
+                         (int)count, rlwe_dbg);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+static cudaError_t launch_fft(const BrParams &P, const BrParams *d_descs, const u32 *item_desc, const u32 *out_idx,
+                              u32 br_q, u32 n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
+                              size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split) {
+  switch (fft_form((size_t)grid, split)) {
+    case fft::SPLIT: return launch_form<fft::SPLIT>(P, d_descs, item_desc, out_idx, br_q, n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
+    case fft::TRIO: return launch_form<fft::TRIO>(P, d_descs, item_desc, out_idx, br_q, n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
+    default: return launch_form<fft::QUAD>(P, d_descs, item_desc, out_idx, br_q, n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
+  }
 }
 
 cudaError_t launch_pbs_fft(const BrParams &P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
-                           size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s) {
-  const size_t smem = fft::fft_smem_bytes(P.br_q, P.n);
-  const cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel, smem);
-  if (e != cudaSuccess) return e;
-  fft::pbs_fft_kernel<<<grid, fft::T, smem, s>>>(P, ks, ks_stride, gates, out, (int)count, rlwe_dbg);
-  return cudaGetLastError();
+                           size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split) {
+  return launch_fft(P, nullptr, nullptr, nullptr, P.br_q, P.n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s,
+                    split);
 }
 
 cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc, u32 max_br_q, u32 max_n, const u32 *ks,
                                   u32 ks_stride, const unsigned char *gates, u64 *out, const u32 *out_idx,
-                                  size_t count, int grid, cudaStream_t s) {
-  const size_t smem = fft::fft_smem_bytes(max_br_q, max_n);
-  const cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_ragged_kernel, smem);
-  if (e != cudaSuccess) return e;
-  fft::pbs_fft_ragged_kernel<<<grid, fft::T, smem, s>>>(d_descs, item_desc, ks, ks_stride, gates, out, out_idx,
-                                                        (int)count);
-  return cudaGetLastError();
+                                  size_t count, int grid, cudaStream_t s, bool split) {
+  return launch_fft(BrParams{}, d_descs, item_desc, out_idx, max_br_q, max_n, ks, ks_stride, gates, out, count, nullptr,
+                    grid, s, split);
 }
 
 }  // namespace pz

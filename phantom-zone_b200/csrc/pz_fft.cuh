@@ -30,7 +30,7 @@ namespace pz {
 namespace fft {
 
 constexpr int M = 1024;          // complex length
-constexpr int T = 128;           // threads per polynomial, 8 complex values each
+constexpr int T = 128;           // threads per polynomial (a group), 8 complex values each
 constexpr int LIMBS = 3, LIMB_BITS = 18;
 constexpr int POLY_W = M;        // complex words (16 bytes) of one transformed limb
 // One key block = the operand of one operation: [output a, b][limb][point 0..7]
@@ -126,20 +126,52 @@ __device__ __forceinline__ void inv4(cplx &a, cplx &b, cplx &c, cplx &d, double 
   ibf(b, d, w1r, w1i);
 }
 
-// Tensor memory, per warp: 64 columns as storage of the transformed digit
-// polynomials of its threads while the key is worked through, 32 for the
-// permuted b of an automorphism until its turn, 32 for the turns below.  That
-// is 96 registers less per thread: four CTAs share an SM.
-constexpr u32 SPEC_COLS = 64, B_COLS = 32, TURN_COLS = 32, TMEM_COLS = SPEC_COLS + B_COLS + TURN_COLS;
+// Tensor memory.  Warps of equal number in the groups of a CTA share 32 lanes
+// of it, and their threads of equal number hold the same positions of their
+// polynomials, so it is where the groups meet without the shared-memory pipe,
+// besides saving registers.
+template <u32 COLS>
 __device__ __forceinline__ void tmem_alloc(u32 *slot) {  // one warp; slot in shared memory
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)),
-               "r"(TMEM_COLS)
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)), "r"(COLS)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
 }
+template <u32 COLS>
 __device__ __forceinline__ void tmem_free(u32 base) {  // the same warp
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(TMEM_COLS));
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(COLS));
 }
+// One 32-bit word into the other CTA's shared memory, counted there on *bar.
+__device__ __forceinline__ void remote_store(u32 addr, int v, u32 bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
+               : "memory");
+}
+// this CTA's shared address in CTA `rank` of the cluster
+__device__ __forceinline__ u32 cluster_addr(const void *p, u32 rank) {
+  u32 a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+  return a;
+}
+// mbar_wait for writes of the cluster
+__device__ __forceinline__ bool mbar_wait_cluster(u64 *bar, u32 parity, long long limit = MBAR_WAIT_LIMIT) {
+  const u32 a = smem_addr(bar);
+  const long long t0 = clock64();
+  for (;;) {
+    u32 done;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (clock64() - t0 > limit) return false;
+  }
+}
+__device__ __forceinline__ void mbar_expect(u64 *bar, u32 bytes) {  // one arrival
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+// around a barrier between one warp's accesses and another's
+__device__ __forceinline__ void tmem_before_barrier() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_after_barrier() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // two complex values -> 8 columns
 __device__ __forceinline__ void tmem_store2(u32 addr, const cplx &a, const cplx &b) {
@@ -193,6 +225,37 @@ __device__ __forceinline__ void tmem_load8(u32 addr, u64 (&v)[8]) {
       : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7])
       : "r"(addr)
       : "memory");
+}
+
+// three groups of 2 C columns -> the sums of C 64-bit words
+template <int C>
+__device__ __forceinline__ void tmem_sum3(u32 addr, u64 (&v)[C]) {
+  static_assert(C == 4 || C == 8, "");
+  if constexpr (C == 4)
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 r<24>;\n\t.reg .u64 a, b, c;\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0, r1, r2, r3, r4, r5, r6, r7}, [%4];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {r8, r9, r10, r11, r12, r13, r14, r15}, [%5];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {r16, r17, r18, r19, r20, r21, r22, r23}, [%6];\n\t"
+        "tcgen05.wait::ld.sync.aligned;\n\t"
+        "mov.b64 a, {r0, r1};\n\tmov.b64 b, {r8, r9};\n\tmov.b64 c, {r16, r17};\n\tadd.u64 a, a, b;\n\tadd.u64 %0, a, c;\n\t"
+        "mov.b64 a, {r2, r3};\n\tmov.b64 b, {r10, r11};\n\tmov.b64 c, {r18, r19};\n\tadd.u64 a, a, b;\n\tadd.u64 %1, a, c;\n\t"
+        "mov.b64 a, {r4, r5};\n\tmov.b64 b, {r12, r13};\n\tmov.b64 c, {r20, r21};\n\tadd.u64 a, a, b;\n\tadd.u64 %2, a, c;\n\t"
+        "mov.b64 a, {r6, r7};\n\tmov.b64 b, {r14, r15};\n\tmov.b64 c, {r22, r23};\n\tadd.u64 a, a, b;\n\tadd.u64 %3, a, c;\n\t"
+        "}"
+        : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+        : "r"(addr), "r"(addr + 32), "r"(addr + 64)
+        : "memory");
+  else {
+    u64 w[4];
+    tmem_sum3<4>(addr, w);
+#pragma unroll
+    for (int m = 0; m < 4; m++) v[m] = w[m];
+    tmem_sum3<4>(addr + 8, w);
+#pragma unroll
+    for (int m = 0; m < 4; m++) v[4 + m] = w[m];
+  }
 }
 
 // Two lane bits and two register bits change places through tensor memory,
@@ -376,31 +439,41 @@ __device__ __forceinline__ void turn_take_back(u32 addr, cplx (&x)[8]) {
 //   2      p9 p8       p1 p0 p7 p6 p5     p4 p3 p2    levels 6, 7
 //   E      p9 p8       p7 p6 p5 p3 p2     p4 p1 p0    levels 8, 9, evaluation order
 // C <-> 1 goes through shared memory (M words of 16 bytes); p7 is XORed into
-// address bit 2, so that neither side has bank conflicts.  Two such buffers
-// take turns: a transform writes the one that everybody finished reading
-// before the barrier of the transform in between, so one barrier per transform
-// is enough.  1 <-> 2 <-> E stay inside a warp and go through tensor memory:
+// address bit 2, so that neither side has bank conflicts.  A group's two
+// buffers take turns: a transform writes the one that the whole group finished
+// reading before the barrier of the transform in between, so one barrier per
+// transform is enough.  (SPLIT has another barrier between any two transforms of a
+// group, and one buffer.)  1 <-> 2 <-> E stay inside a warp and go through tensor memory:
 // the shared-memory pipe, which also delivers the keys, was the busiest unit
 // with them.
 struct Place {
-  int t, c, b;  // thread; buffer index of its register 0 in layouts C and 1
-  u32 turn;     // this warp's tensor memory for the turns
-  __device__ __forceinline__ explicit Place(int t_, u32 turn_) : t(t_), turn(turn_) {
+  int t, g, c, b;  // thread of group g; buffer index of its register 0 in layouts C and 1
+  u32 turn;        // this warp's tensor memory for the turns
+  __device__ __forceinline__ Place(int t_, int g_, u32 turn_) : t(t_), g(g_), turn(turn_) {
     const int w = t >> 5, l = t & 31;
     c = t;
     b = ((w << 8) | ((l & 1) << 7) | (l >> 1)) ^ ((l & 1) << 2);
   }
 };
+// The barrier of one of GROUPS groups (0 is the block's).
+template <int GROUPS>
+__device__ __forceinline__ void group_sync(const Place &p) {
+  if (GROUPS == 1) __syncthreads();
+  else if (p.g == 0) asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+  else if (p.g == 1) asm volatile("bar.sync 2, %0;" ::"n"(T) : "memory");
+  else asm volatile("bar.sync 3, %0;" ::"n"(T) : "memory");
+}
 // register r of layout C is at p.c + 128 r, with the XOR for odd r
 __device__ __forceinline__ int at_c(const Place &p, int r) { return (p.c ^ ((r & 1) << 2)) + 128 * r; }
 __device__ __forceinline__ int at_1(const Place &p, int r) { return p.b + 16 * r; }
 
 // Forward transform, layout C -> E, through buffer X.
+template <int GROUPS>
 __device__ __forceinline__ void forward(cplx (&x)[8], cplx *X, const cplx *tw, const Place &p) {
   fwd8(x, PZ_FFT_C0);
 #pragma unroll
   for (int r = 0; r < 8; r++) X[at_c(p, r)] = x[r];
-  __syncthreads();
+  group_sync<GROUPS>(p);
 #pragma unroll
   for (int r = 0; r < 8; r++) x[r] = X[at_1(p, r)];
   const int w = p.t >> 5, l = p.t & 31;
@@ -429,6 +502,7 @@ __device__ __forceinline__ void forward(cplx (&x)[8], cplx *X, const cplx *tw, c
 }
 
 // Inverse transform (without the factor 1 / M, which the keys carry), E -> C.
+template <int GROUPS>
 __device__ __forceinline__ void inverse(cplx (&x)[8], cplx *X, const cplx *tw, const Place &p) {
   const int w = p.t >> 5, l = p.t & 31;
   {
@@ -455,7 +529,7 @@ __device__ __forceinline__ void inverse(cplx (&x)[8], cplx *X, const cplx *tw, c
   }
 #pragma unroll
   for (int r = 0; r < 8; r++) X[at_1(p, r)] = x[r];
-  __syncthreads();
+  group_sync<GROUPS>(p);
 #pragma unroll
   for (int r = 0; r < 8; r++) x[r] = X[at_c(p, r)];
   inv8(x, PZ_FFT_C0);

@@ -128,11 +128,11 @@ size_t fft_key_bytes(size_t keys);
 cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const RingConsts &rc, const void *tables,
                            void *out, cudaStream_t s);
 cudaError_t launch_pbs_fft(const BrParams &P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
-                           size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s);
+                           size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split);
 cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas);  // resident CTAs per SM
 cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc, u32 max_br_q, u32 max_n, const u32 *ks,
                                   u32 ks_stride, const unsigned char *gates, u64 *out, const u32 *out_idx,
-                                  size_t count, int grid, cudaStream_t s);
+                                  size_t count, int grid, cudaStream_t s, bool split);
 cudaError_t launch_not(const u64 *in, u64 *out, size_t words, u64 q, cudaStream_t s);
 cudaError_t launch_imad_probe(int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);
 cudaError_t launch_pipe_probe(int kind, int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);
