@@ -48,8 +48,8 @@ pz_status pz_aggregate_rgsw_device(pz_ctx *c, uint64_t *d_rgsw0, const uint64_t 
   u32 *d_idx = nullptr;
   std::vector<u32> idx(2 * chunk);
   for (size_t i = 0; i < 2 * chunk; i++) idx[i] = (u32)(i / 2);  // two RLWEs per leader RGSW
-  cudaError_t e = cudaMallocAsync(&d_eval, chunk * rows1 * N * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_idx, 2 * chunk * 4, st);
+  cudaError_t e = pz::pool_malloc(&d_eval, chunk * rows1 * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_idx, 2 * chunk * 4, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_idx, idx.data(), 2 * chunk * 4, cudaMemcpyHostToDevice, st);
   for (size_t t = 0; t < steps && e == cudaSuccess; t++) {  // the other users, in order
     for (size_t c0 = 0; c0 < count && e == cudaSuccess; c0 += chunk) {
@@ -111,12 +111,12 @@ pz_status pz_aggregate_device(pz_ctx *c, const pz_server_key_share_view *shares,
   }
   const u64 **d_src = nullptr;
   u64 *d_others = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&d_src, 2 * users * sizeof(u64 *), st);
+  cudaError_t e = pz::pool_malloc((void **)&d_src, 2 * users * sizeof(u64 *), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_src, src.data(), 2 * users * sizeof(u64 *), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
     e = pz::launch_sum_mod(d_src, (u32)users, (size_t)P.n_auto_keys * P.auto_d * N, P.rlwe_q, d_auto_b, st);
   if (e == cudaSuccess) e = pz::launch_sum_mod(d_src + users, (u32)users, (size_t)P.lwe_d * N, P.lwe_q, d_lwe_b, st);
-  if (e == cudaSuccess && users > 1) e = cudaMallocAsync(&d_others, (users - 1) * max_seg * rows1 * N * 8, st);
+  if (e == cudaSuccess && users > 1) e = pz::pool_malloc(&d_others, (users - 1) * max_seg * rows1 * N * 8, st);
   pz_status ps = PZ_OK;
   for (size_t L = 0; L < users && e == cudaSuccess && ps == PZ_OK; L++) {
     const size_t b = sb[L], cnt = se[L] - sb[L];
@@ -151,9 +151,9 @@ pz_status pz_aggregate_server_key(pz_ctx *c, const uint8_t crs[32], const pz_ser
   const size_t N = P.rlwe_n;
   PZ_CK(c, cudaSetDevice(c->device));
   u64 *d_rgsw = nullptr, *d_auto = nullptr, *d_lwe = nullptr;
-  cudaError_t e = cudaMalloc(&d_rgsw, (size_t)P.lwe_n * 4 * N * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_auto, (size_t)P.n_auto_keys * P.auto_d * N * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_lwe, (size_t)P.lwe_d * N * 8);
+  cudaError_t e = pz::dev_malloc(&d_rgsw, (size_t)P.lwe_n * 4 * N * 8);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_auto, (size_t)P.n_auto_keys * P.auto_d * N * 8);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_lwe, (size_t)P.lwe_d * N * 8);
   pz_status s = e == cudaSuccess ? PZ_OK : pz::cuda_fail(c, "pz_aggregate_server_key", e);
   if (s == PZ_OK) s = pz_aggregate_device(c, shares, users, d_rgsw, d_auto, d_lwe, c->stream);
   if (s == PZ_OK) {

@@ -324,13 +324,13 @@ pz_status bind_device(pz_ctx *ctx, pz_circuit *c) {
   c->free_device();
   const size_t G = c->gates.size(), L = (size_t)ctx->P.rlwe_n + 1;
   const size_t W = c->n_inputs + G;
-  PZ_CK(ctx, cudaMalloc(&c->d_wires, std::max<size_t>(W, 1) * L * 8));
-  PZ_CK(ctx, cudaMalloc(&c->d_type, std::max<size_t>(G, 1)));
-  PZ_CK(ctx, cudaMalloc(&c->d_in0, std::max<size_t>(G, 1) * 4));
-  PZ_CK(ctx, cudaMalloc(&c->d_in1, std::max<size_t>(G, 1) * 4));
-  PZ_CK(ctx, cudaMalloc(&c->d_out, std::max<size_t>(G, 1) * 4));
-  PZ_CK(ctx, cudaMalloc(&c->d_outref, std::max<size_t>(c->outputs.size(), 1) * 4));
-  PZ_CK(ctx, cudaMalloc(&c->d_ks, std::max<size_t>(c->max_width, 1) * pz::ks_stride(ctx->P) * 4));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_wires, std::max<size_t>(W, 1) * L * 8));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_type, std::max<size_t>(G, 1)));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_in0, std::max<size_t>(G, 1) * 4));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_in1, std::max<size_t>(G, 1) * 4));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_out, std::max<size_t>(G, 1) * 4));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_outref, std::max<size_t>(c->outputs.size(), 1) * 4));
+  PZ_CK(ctx, pz::dev_malloc(&c->d_ks, std::max<size_t>(c->max_width, 1) * pz::ks_stride(ctx->P) * 4));
   if (G) {
     PZ_CK(ctx, cudaMemcpy(c->d_type, c->h_type.data(), G, cudaMemcpyHostToDevice));
     PZ_CK(ctx, cudaMemcpy(c->d_in0, c->h_in0.data(), G * 4, cudaMemcpyHostToDevice));
@@ -607,7 +607,7 @@ pz_status pz_circuit_run(pz_ctx *ctx, const pz_key *k, pz_circuit *c, const uint
   if (s != PZ_OK) return s;
   const size_t L = (size_t)ctx->P.rlwe_n + 1;
   u64 *d_o = nullptr;
-  PZ_CK(ctx, cudaMallocAsync(&d_o, std::max<size_t>(c->outputs.size(), 1) * L * 8, ctx->stream));
+  PZ_CK(ctx, pz::pool_malloc(&d_o, std::max<size_t>(c->outputs.size(), 1) * L * 8, ctx->stream));
   // host inputs go straight into the input wire slots
   if (c->n_inputs)
     PZ_CK(ctx, cudaMemcpyAsync(c->d_wires, inputs, c->n_inputs * L * 8, cudaMemcpyHostToDevice, ctx->stream));

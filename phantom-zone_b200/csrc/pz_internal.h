@@ -10,6 +10,7 @@
 
 struct pz_ctx {
   int param_id = 0, device = 0;
+  bool pooled = false;  // holds a reference to the device's memory pool
   pz_params P{};
   pz::u32 logn = 0;
   pz::u64 root = 0;
@@ -65,6 +66,25 @@ struct pz_ni_ksk {
 };
 
 namespace pz {
+// Stream-ordered scratch comes from one memory pool per device, shared by the
+// contexts there, created with the first of them and destroyed with the last.
+// It keeps at most POOL_KEEP bytes between calls (the default pool gave all its
+// memory back at every synchronisation: three users' key aggregation, with 1.4 GB
+// of scratch, took 195 ms in a row of calls against 37 ms with the memory there).
+constexpr size_t POOL_KEEP = (size_t)2 << 30;
+cudaError_t pool_acquire(int device);
+void pool_release(int device);
+cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t st);  // on the current device
+template <typename T>
+cudaError_t pool_malloc(T **p, size_t bytes, cudaStream_t st) {
+  return pool_malloc((void **)p, bytes, st);
+}
+// cudaMalloc that, short of memory, gives back what the pool keeps and tries again
+cudaError_t dev_malloc(void **p, size_t bytes);
+template <typename T>
+cudaError_t dev_malloc(T **p, size_t bytes) {
+  return dev_malloc((void **)p, bytes);
+}
 // Build k->d_ksk8 from k->d_ksk (when the parameter set's digits fit s8 and
 // the rows come in whole 32-row blocks; otherwise, or when the device is out
 // of memory, the key keeps the IMAD key-switch kernels only).

@@ -303,7 +303,7 @@ pz_status seeded_fill(pz_ctx *c, const uint8_t (*seeds)[32], size_t streams, u64
   const size_t b_samples = group * nblocks * 64, b_off = group * (nblocks + 1) * 8, b_tot = group * 8,
                b_cnt = group * nblocks * 4, b_acc = group * nblocks;
   unsigned char *scratch = nullptr;
-  cudaError_t e = cudaMallocAsync(&scratch, b_samples + b_off + b_tot + b_cnt + b_acc, st);
+  cudaError_t e = pz::pool_malloc(&scratch, b_samples + b_off + b_tot + b_cnt + b_acc, st);
   u64 *samples = (u64 *)scratch, *off = (u64 *)(scratch + b_samples), *tot = (u64 *)(scratch + b_samples + b_off);
   u32 *cnt = (u32 *)(scratch + b_samples + b_off + b_tot);
   unsigned char *acc = scratch + b_samples + b_off + b_tot + b_cnt;
@@ -389,8 +389,8 @@ pz_status pz_ni_ksk_upload(pz_ctx *c, const uint64_t *ksk, pz_ni_ksk **out) {
   k->d = c->P.ni_ks_d;
   k->bytes = polys * N * 8;
   u64 *stage = nullptr;
-  cudaError_t e = cudaMalloc(&k->d_ksk, k->bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&stage, k->bytes);
+  cudaError_t e = pz::dev_malloc(&k->d_ksk, k->bytes);
+  if (e == cudaSuccess) e = pz::dev_malloc(&stage, k->bytes);
   if (e == cudaSuccess) e = cudaMemcpyAsync(stage, ksk, k->bytes, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = pz::launch_key_convert((int)c->logn, stage, k->d_ksk, polys, c->rc, c->ni_conv_c, c->ni_conv_cs, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -417,8 +417,8 @@ pz_status pz_ni_ksk_upload_seeded(pz_ctx *c, const uint64_t *ksk_b, const uint8_
   k->d = (u32)d;
   k->bytes = polys * N * 8;
   u64 *stage = nullptr;
-  cudaError_t e = cudaMalloc(&k->d_ksk, k->bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&stage, k->bytes);
+  cudaError_t e = pz::dev_malloc(&k->d_ksk, k->bytes);
+  if (e == cudaSuccess) e = pz::dev_malloc(&stage, k->bytes);
   // keys.rs:965-1000: d A rows from the user's stream, then the B rows
   if (e == cudaSuccess) s = pz::seeded_fill_u64(c, seed, c->P.rlwe_q, (u64)d * N, d * N, 2 * d * N, 0, stage, c->stream);
   if (e == cudaSuccess && s == PZ_OK)
@@ -481,7 +481,7 @@ pz_status pz_ni_key_switch_device(pz_ctx *c, const pz_ni_ksk *k, const uint64_t 
     return PZ_OK;
   }
   u64 *part = nullptr;
-  PZ_CK(c, cudaMallocAsync(&part, count * shares * 2 * c->P.rlwe_n * 8, st));
+  PZ_CK(c, pz::pool_malloc(&part, count * shares * 2 * c->P.rlwe_n * 8, st));
   ni_ks_partial_kernel<<<dim3((unsigned)count, (unsigned)shares), NI_T, smem, st>>>(c->rc, dp, k->d, k->d_ksk, d_in,
                                                                                    part, count);
   cudaError_t e = cudaGetLastError();
@@ -523,11 +523,11 @@ pz_status pz_ni_ingest(pz_ctx *c, const pz_ni_ksk *k, const uint8_t seed[32], co
   u32 *d_i = nullptr;
   std::vector<u32> idx(nbools);
   for (size_t i = 0; i < nbools; i++) idx[i] = (u32)i;
-  cudaError_t e = cudaMallocAsync(&d_b, rlwe_count * N * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_r, rlwe_count * 2 * N * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_k, rlwe_count * 2 * N * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_l, std::max<size_t>(nbools, 1) * (N + 1) * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_i, std::max<size_t>(nbools, 1) * 4, st);
+  cudaError_t e = pz::pool_malloc(&d_b, rlwe_count * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_r, rlwe_count * 2 * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_k, rlwe_count * 2 * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_l, std::max<size_t>(nbools, 1) * (N + 1) * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_i, std::max<size_t>(nbools, 1) * 4, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_b, b, rlwe_count * N * 8, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && nbools) e = cudaMemcpyAsync(d_i, idx.data(), nbools * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -281,10 +281,10 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   const u64 **d_src = nullptr;
   NiUser *d_users = nullptr;
   const size_t nsrc = users * users + 2 * users;  // ksk lists, auto list, lwe list
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_keys, users * 2 * d * N * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_stage, 2 * d * N * 8, st);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&d_src, nsrc * sizeof(u64 *), st);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_users, users * sizeof(NiUser), st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_keys, users * 2 * d * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_stage, 2 * d * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc((void **)&d_src, nsrc * sizeof(u64 *), st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_users, users * sizeof(NiUser), st);
   // ---- ui_to_s key B rows (evaluator.rs:1269-1294), auto and LWE KSK sums
   std::vector<const u64 *> src(nsrc);
   for (size_t j = 0; j < users; j++) {
@@ -344,11 +344,11 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
     chunk = std::max<size_t>(1, std::min(chunk, free_b / 2 / per_index));
   u64 *d_arows = nullptr, *d_vals = nullptr, *d_dig = nullptr, *d_others = nullptr;
-  if (e == cudaSuccess && ps == PZ_OK) e = cudaMallocAsync(&d_arows, chunk * max_d * N * 8, st);
-  if (e == cudaSuccess && ps == PZ_OK) e = cudaMallocAsync(&d_vals, chunk * R * N * 8, st);
-  if (e == cudaSuccess && ps == PZ_OK) e = cudaMallocAsync(&d_dig, chunk * R * d * N * 8, st);
+  if (e == cudaSuccess && ps == PZ_OK) e = pz::pool_malloc(&d_arows, chunk * max_d * N * 8, st);
+  if (e == cudaSuccess && ps == PZ_OK) e = pz::pool_malloc(&d_vals, chunk * R * N * 8, st);
+  if (e == cudaSuccess && ps == PZ_OK) e = pz::pool_malloc(&d_dig, chunk * R * d * N * 8, st);
   if (e == cudaSuccess && ps == PZ_OK && users > 1)
-    e = cudaMallocAsync(&d_others, (users - 1) * chunk * rows1 * N * 8, st);
+    e = pz::pool_malloc(&d_others, (users - 1) * chunk * rows1 * N * 8, st);
   const pz::Decomp dp = pz::decomposer(P.rlwe_q, P.ni_ks_logb, (u32)d);
   const size_t smem = 2 * N * 8;
   std::vector<uint8_t> seeds(chunk * 32);
@@ -394,10 +394,10 @@ pz_status pz_ni_aggregate_server_key(pz_ctx *c, const uint8_t crs[32], const pz_
   const size_t N = P.rlwe_n, d = P.ni_ks_d;
   PZ_CK(c, cudaSetDevice(c->device));
   u64 *d_ksk = nullptr, *d_rgsw = nullptr, *d_auto = nullptr, *d_lwe = nullptr;
-  cudaError_t e = cudaMalloc(&d_ksk, std::max<size_t>(users, 1) * d * N * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_rgsw, (size_t)P.lwe_n * 4 * N * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_auto, (size_t)P.n_auto_keys * P.auto_d * N * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_lwe, (size_t)P.lwe_d * N * 8);
+  cudaError_t e = pz::dev_malloc(&d_ksk, std::max<size_t>(users, 1) * d * N * 8);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_rgsw, (size_t)P.lwe_n * 4 * N * 8);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_auto, (size_t)P.n_auto_keys * P.auto_d * N * 8);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_lwe, (size_t)P.lwe_d * N * 8);
   pz_status s = e == cudaSuccess ? PZ_OK : pz::cuda_fail(c, "pz_ni_aggregate_server_key", e);
   if (s == PZ_OK) s = pz_ni_aggregate_device(c, crs, shares, users, d_ksk, d_rgsw, d_auto, d_lwe, c->stream);
   if (s == PZ_OK) {

@@ -103,6 +103,70 @@ pz::Decomp make_decomp(u64 q, u32 logb, u32 d) {  // decomposer.rs:158-178
 }  // namespace
 
 namespace pz {
+namespace {
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  int contexts = 0;
+};
+constexpr int MAX_POOLS = 64;
+std::mutex pool_mu;
+DevicePool pools[MAX_POOLS];
+}  // namespace
+
+cudaError_t pool_acquire(int device) {
+  if (device < 0 || device >= MAX_POOLS) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(pool_mu);
+  DevicePool &d = pools[device];
+  if (!d.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaError_t e = cudaMemPoolCreate(&d.pool, &props);
+    if (e != cudaSuccess) {
+      d.pool = nullptr;
+      return e;
+    }
+    uint64_t keep = POOL_KEEP;
+    if ((e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+      cudaMemPoolDestroy(d.pool);
+      d.pool = nullptr;
+      return e;
+    }
+  }
+  d.contexts++;
+  return cudaSuccess;
+}
+void pool_release(int device) {
+  if (device < 0 || device >= MAX_POOLS) return;
+  std::lock_guard<std::mutex> lock(pool_mu);
+  DevicePool &d = pools[device];
+  if (d.contexts > 0 && --d.contexts == 0 && d.pool) {
+    cudaMemPoolDestroy(d.pool);  // allocations still in flight end first
+    d.pool = nullptr;
+  }
+}
+static cudaMemPool_t current_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_POOLS) return nullptr;
+  std::lock_guard<std::mutex> lock(pool_mu);
+  return pools[dev].pool;
+}
+cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = current_pool();
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+}
+cudaError_t dev_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  cudaMemPool_t pool = e == cudaErrorMemoryAllocation ? current_pool() : nullptr;
+  if (pool) {
+    cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 Decomp decomposer(u64 q, u32 logb, u32 d) { return make_decomp(q, logb, d); }
 
 pz_status fail(pz_ctx *ctx, pz_status s, const std::string &msg) {
@@ -174,11 +238,11 @@ pz_status ensure_scratch(pz_ctx *c, size_t count) {
   cudaFree(c->d_c0); cudaFree(c->d_c1); cudaFree(c->d_out); cudaFree(c->d_gates); cudaFree(c->d_ks);
   c->d_c0 = c->d_c1 = c->d_out = nullptr; c->d_gates = nullptr; c->d_ks = nullptr;
   c->cap = 0;
-  PZ_CK(c, cudaMalloc(&c->d_c0, cap * L * 8));
-  PZ_CK(c, cudaMalloc(&c->d_c1, cap * L * 8));
-  PZ_CK(c, cudaMalloc(&c->d_out, cap * L * 8));
-  PZ_CK(c, cudaMalloc(&c->d_gates, cap));
-  PZ_CK(c, cudaMalloc(&c->d_ks, cap * ks_stride(c->P) * 4));
+  PZ_CK(c, pz::dev_malloc(&c->d_c0, cap * L * 8));
+  PZ_CK(c, pz::dev_malloc(&c->d_c1, cap * L * 8));
+  PZ_CK(c, pz::dev_malloc(&c->d_out, cap * L * 8));
+  PZ_CK(c, pz::dev_malloc(&c->d_gates, cap));
+  PZ_CK(c, pz::dev_malloc(&c->d_ks, cap * ks_stride(c->P) * 4));
   c->cap = cap;
   return PZ_OK;
 }
@@ -205,7 +269,7 @@ void build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s) {
   if (!k->d_ksk || rows % 32 || P.rlwe_n % 32 || P.lwe_d > 16 || P.lwe_logb > 7) return;
   const u32 planes = ksk8_planes(c->ks.mask), cols = ksk8_cols(P.lwe_n);
   const size_t bytes = (size_t)planes * rows * cols;
-  if (cudaMalloc(&k->d_ksk8, bytes) != cudaSuccess) {
+  if (pz::dev_malloc(&k->d_ksk8, bytes) != cudaSuccess) {
     cudaGetLastError();
     k->d_ksk8 = nullptr;
     return;
@@ -224,7 +288,7 @@ void build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s) {
   const pz_params &P = c->P;
   if (!c->d_fft) return;
   const size_t rg = fft_key_bytes(P.lwe_n), au = fft_key_bytes(P.n_auto_keys);
-  if (cudaMalloc(&k->d_fft_rgsw, rg) == cudaSuccess && cudaMalloc(&k->d_fft_autos, au) == cudaSuccess &&
+  if (pz::dev_malloc(&k->d_fft_rgsw, rg) == cudaSuccess && pz::dev_malloc(&k->d_fft_autos, au) == cudaSuccess &&
       launch_fft_key(k->d_rgsw, P.rgsw_rows, P.lwe_n, c->rc, c->d_fft, k->d_fft_rgsw, s) == cudaSuccess &&
       launch_fft_key(k->d_autos, P.auto_rows, P.n_auto_keys, c->rc, c->d_fft, k->d_fft_autos, s) == cudaSuccess &&
       cudaStreamSynchronize(s) == cudaSuccess) {
@@ -357,6 +421,8 @@ pz_status pz_ctx_create_ex(int id, int device, uint64_t root, pz_ctx **out) {
   c->root = root;
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) { delete c; return PZ_ERR_CUDA; }
+  if (pz::pool_acquire(device) != cudaSuccess) { delete c; return PZ_ERR_CUDA; }
+  c->pooled = true;
   // twiddles: psi^{bitrev(i)} and psi^{-bitrev(i)} (ntt.rs:337-369), each
   // interleaved with its companion: [w_0, ws_0, w_1, ws_1, ...] (the Shoup
   // companion, or w/Q as a double for the FP64-quotient butterflies)
@@ -382,14 +448,14 @@ pz_status pz_ctx_create_ex(int id, int device, uint64_t root, pz_ctx **out) {
     if (_e != cudaSuccess) { pz_ctx_destroy(c); return PZ_ERR_CUDA; } \
   } while (0)
   CK_CREATE(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  CK_CREATE(cudaMalloc(&c->d_tw, 4 * N * 8));
+  CK_CREATE(pz::dev_malloc(&c->d_tw, 4 * N * 8));
   CK_CREATE(cudaMemcpy(c->d_tw, tw.data(), 4 * N * 8, cudaMemcpyHostToDevice));
-  CK_CREATE(cudaMalloc(&c->d_dlog, dlog.size() * 2));
+  CK_CREATE(pz::dev_malloc(&c->d_dlog, dlog.size() * 2));
   CK_CREATE(cudaMemcpy(c->d_dlog, dlog.data(), dlog.size() * 2, cudaMemcpyHostToDevice));
   if (c->logn == 11 && P.rlrg_d_a == 1 && P.rlrg_d_b == 1 && P.auto_d == 1) CK_CREATE(pz::fft_tables(&c->d_fft));
-  CK_CREATE(cudaMalloc(&c->d_err, sizeof(u32)));
+  CK_CREATE(pz::dev_malloc(&c->d_err, sizeof(u32)));
   CK_CREATE(cudaMemset(c->d_err, 0, sizeof(u32)));
-  CK_CREATE(cudaMalloc(&c->d_tv, tv.size() * 8));
+  CK_CREATE(pz::dev_malloc(&c->d_tv, tv.size() * 8));
   CK_CREATE(cudaMemcpy(c->d_tv, tv.data(), tv.size() * 8, cudaMemcpyHostToDevice));
 #undef CK_CREATE
   // Montgomery constant -Q^{-1} mod 2^64 (Newton iteration)
@@ -459,6 +525,7 @@ void pz_ctx_destroy(pz_ctx *c) {
   cudaFree(c->d_tw); cudaFree(c->d_fft); cudaFree(c->d_dlog); cudaFree(c->d_tv); cudaFree(c->d_err);
   cudaFree(c->d_c0); cudaFree(c->d_c1); cudaFree(c->d_out); cudaFree(c->d_gates); cudaFree(c->d_ks);
   if (c->stream) cudaStreamDestroy(c->stream);
+  if (c->pooled) pz::pool_release(c->device);
   delete c;
 }
 
@@ -521,14 +588,14 @@ pz_status pz_key_upload(pz_ctx *c, const pz_server_key_view *v, pz_key **out) {
     return fail(c, s, m);
   };
   cudaError_t e;
-  if ((e = cudaMalloc(&k->d_rgsw, rgsw_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "rgsw alloc");
-  if ((e = cudaMalloc(&k->d_autos, auto_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "auto alloc");
-  if ((e = cudaMalloc(&k->d_ksk, ksk_rows * stride * 4)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "ksk alloc");
+  if ((e = pz::dev_malloc(&k->d_rgsw, rgsw_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "rgsw alloc");
+  if ((e = pz::dev_malloc(&k->d_autos, auto_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "auto alloc");
+  if ((e = pz::dev_malloc(&k->d_ksk, ksk_rows * stride * 4)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "ksk alloc");
   k->bytes = (rgsw_polys + auto_polys) * N * 8 + ksk_rows * stride * 4;
   // coefficient rows -> device staging -> forward NTT + key form (br_conv_c) + device layout
   const size_t chunk = 1024;  // polynomials per staging copy
   u64 *d_stage = nullptr;
-  if ((e = cudaMalloc(&d_stage, chunk * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "staging alloc");
+  if ((e = pz::dev_malloc(&d_stage, chunk * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "staging alloc");
   auto convert = [&](const u64 *src, u64 *dst, size_t polys) -> cudaError_t {
     for (size_t p0 = 0; p0 < polys; p0 += chunk) {
       size_t m = std::min(chunk, polys - p0);
@@ -584,10 +651,10 @@ pz_status pz_key_upload_seeded(pz_ctx *c, const pz_seeded_server_key_view *v, pz
   };
   cudaError_t e;
   const size_t chunk = 1024;  // polynomials per staging copy (>= the auto keys)
-  if ((e = cudaMalloc(&k->d_rgsw, rgsw_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "rgsw alloc");
-  if ((e = cudaMalloc(&k->d_autos, auto_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "auto alloc");
-  if ((e = cudaMalloc(&k->d_ksk, ksk_rows * stride * 4)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "ksk alloc");
-  if ((e = cudaMalloc(&d_stage, std::max(chunk, auto_polys) * N * 8)) != cudaSuccess)
+  if ((e = pz::dev_malloc(&k->d_rgsw, rgsw_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "rgsw alloc");
+  if ((e = pz::dev_malloc(&k->d_autos, auto_polys * N * 8)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "auto alloc");
+  if ((e = pz::dev_malloc(&k->d_ksk, ksk_rows * stride * 4)) != cudaSuccess) return cleanup(PZ_ERR_OUT_OF_MEMORY, "ksk alloc");
+  if ((e = pz::dev_malloc(&d_stage, std::max(chunk, auto_polys) * N * 8)) != cudaSuccess)
     return cleanup(PZ_ERR_OUT_OF_MEMORY, "staging alloc");
   k->bytes = (rgsw_polys + auto_polys) * N * 8 + ksk_rows * stride * 4;
   // RGSW ciphertexts: as pz_key_upload (keys.rs:738-757)
@@ -674,7 +741,7 @@ static pz_status gate_device_common(pz_ctx *c, const pz_key *k, const uint8_t *d
   PZ_CK(c, cudaSetDevice(c->device));
   cudaStream_t st = pick(c, stream);
   u32 *d_ks = nullptr;
-  if (!d_ks_out) PZ_CK(c, cudaMallocAsync(&d_ks, count * ks_stride(c->P) * 4, st));
+  if (!d_ks_out) PZ_CK(c, pz::pool_malloc(&d_ks, count * ks_stride(c->P) * 4, st));
   s = run_gates(c, k, d_gates, d_c0, d_c1, d_out, count, d_ks_out, d_rlwe, st, d_ks, raw);
   if (d_ks) cudaFreeAsync(d_ks, st);
   return s;
@@ -735,9 +802,9 @@ pz_status pz_ctx_autotune(pz_ctx *c, const pz_key *k, size_t batch, int *variant
   unsigned char *d_g = nullptr;
   u64 *d_out = nullptr;
   cudaEvent_t a = nullptr, b = nullptr;
-  cudaError_t e = cudaMalloc(&d_ks, ks.size() * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&d_g, batch);
-  if (e == cudaSuccess) e = cudaMalloc(&d_out, batch * (c->P.rlwe_n + 1) * 8);
+  cudaError_t e = pz::dev_malloc(&d_ks, ks.size() * 4);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_g, batch);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_out, batch * (c->P.rlwe_n + 1) * 8);
   if (e == cudaSuccess) e = cudaMemcpy(d_ks, ks.data(), ks.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d_g, g.data(), batch, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaEventCreate(&a);
@@ -775,7 +842,7 @@ pz_status pz_ctx_autotune(pz_ctx *c, const pz_key *k, size_t batch, int *variant
   int bct = c->ks_ct;
   u64 *d_c01 = nullptr;
   const size_t L = (size_t)c->P.rlwe_n + 1;
-  if (e == cudaSuccess) e = cudaMalloc(&d_c01, 2 * batch * L * 8);
+  if (e == cudaSuccess) e = pz::dev_malloc(&d_c01, 2 * batch * L * 8);
   if (e == cudaSuccess) {
     std::vector<u64> c01(2 * batch * L);
     for (auto &v : c01) { st ^= st << 13; st ^= st >> 7; st ^= st << 17; v = st % c->P.rlwe_q; }
@@ -856,7 +923,7 @@ pz_status pz_probe_imad_rate(int device, double *imad_per_second) {
   const u32 iters = 2048;
   u32 *sink = nullptr;
   cudaEvent_t e0, e1;
-  if (cudaMalloc(&sink, blocks * 4) != cudaSuccess) return PZ_ERR_OUT_OF_MEMORY;
+  if (pz::dev_malloc(&sink, blocks * 4) != cudaSuccess) return PZ_ERR_OUT_OF_MEMORY;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   pz_status st = PZ_OK;
@@ -886,7 +953,7 @@ pz_status pz_probe_pipe_rates(int device, double *rates, size_t n) {
   const int blocks = sms * 8, threads = 256;
   const u32 iters = 1024;
   u32 *sink = nullptr;
-  if (cudaMalloc(&sink, blocks * 4) != cudaSuccess) return PZ_ERR_OUT_OF_MEMORY;
+  if (pz::dev_malloc(&sink, blocks * 4) != cudaSuccess) return PZ_ERR_OUT_OF_MEMORY;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

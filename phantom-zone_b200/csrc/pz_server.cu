@@ -247,8 +247,8 @@ pz_status upload_descs(pz_server *s) {
   cudaFree(s->d_ksp);
   s->d_br = nullptr;
   s->d_ksp = nullptr;
-  if ((e = cudaMalloc(&s->d_br, br.size() * sizeof(pz::BrParams))) != cudaSuccess) return s->cuda("cudaMalloc", e);
-  if ((e = cudaMalloc(&s->d_ksp, ks.size() * sizeof(pz::KsParams))) != cudaSuccess) return s->cuda("cudaMalloc", e);
+  if ((e = pz::dev_malloc(&s->d_br, br.size() * sizeof(pz::BrParams))) != cudaSuccess) return s->cuda("cudaMalloc", e);
+  if ((e = pz::dev_malloc(&s->d_ksp, ks.size() * sizeof(pz::KsParams))) != cudaSuccess) return s->cuda("cudaMalloc", e);
   if ((e = cudaMemcpy(s->d_br, br.data(), br.size() * sizeof(pz::BrParams), cudaMemcpyHostToDevice)) != cudaSuccess)
     return s->cuda("cudaMemcpy", e);
   if ((e = cudaMemcpy(s->d_ksp, ks.data(), ks.size() * sizeof(pz::KsParams), cudaMemcpyHostToDevice)) != cudaSuccess)
@@ -299,7 +299,7 @@ pz_status ensure_arena(pz_server *s, size_t arena_bytes) {
   s->free_ranges.clear();
   s->free_ranges[0] = s->arena_slots;
   if (s->dry) return PZ_OK;
-  cudaError_t e = cudaMalloc(&s->d_arena, s->arena_slots * s->L * 8);
+  cudaError_t e = pz::dev_malloc(&s->d_arena, s->arena_slots * s->L * 8);
   if (e != cudaSuccess) {
     s->arena_slots = 0;
     return s->cuda("arena cudaMalloc", e);
@@ -368,7 +368,7 @@ pz_status ensure_device_buffers(pz_server *s) {
     cudaFree(s->d_ksout);
     s->d_ksout = nullptr;
     s->ksout_stride = 0;
-    cudaError_t e = cudaMalloc(&s->d_ksout, s->max_items * (size_t)s->ks_stride * 4);
+    cudaError_t e = pz::dev_malloc(&s->d_ksout, s->max_items * (size_t)s->ks_stride * 4);
     if (e != cudaSuccess) return s->cuda("cudaMalloc", e);
     s->ksout_stride = s->ks_stride;
   }
@@ -536,7 +536,7 @@ pz_status finish_outputs(pz_server *s, const std::vector<pz_server::Job *> &fin)
     cudaFree(s->d_outref);
     s->d_outref = nullptr;
     s->outref_cap = 0;
-    if ((e = cudaMalloc(&s->d_outref, refs * 4)) != cudaSuccess) return s->cuda("cudaMalloc", e);
+    if ((e = pz::dev_malloc(&s->d_outref, refs * 4)) != cudaSuccess) return s->cuda("cudaMalloc", e);
     s->outref_cap = refs;
   }
   if (host_outs > s->gather_cap) {
@@ -544,7 +544,7 @@ pz_status finish_outputs(pz_server *s, const std::vector<pz_server::Job *> &fin)
     cudaFree(s->d_gather);
     s->d_gather = nullptr;
     s->gather_cap = 0;
-    if ((e = cudaMalloc(&s->d_gather, host_outs * s->L * 8)) != cudaSuccess) return s->cuda("cudaMalloc", e);
+    if ((e = pz::dev_malloc(&s->d_gather, host_outs * s->L * 8)) != cudaSuccess) return s->cuda("cudaMalloc", e);
     s->gather_cap = host_outs;
   }
   std::vector<u32> h(refs);
@@ -595,7 +595,7 @@ pz_status pz_server_create(int device, size_t arena_bytes, size_t max_items, pz_
     }
     const pz_server::Layout lay = s->layout(max_items);
     for (int b = 0; b < 2; b++) {
-      if (cudaMallocHost(&s->h_buf[b], lay.total) != cudaSuccess || cudaMalloc(&s->d_buf[b], lay.total) != cudaSuccess ||
+      if (cudaMallocHost(&s->h_buf[b], lay.total) != cudaSuccess || pz::dev_malloc(&s->d_buf[b], lay.total) != cudaSuccess ||
           cudaEventCreateWithFlags(&s->buf_free[b], cudaEventDisableTiming) != cudaSuccess ||
           cudaEventRecord(s->buf_free[b], s->stream) != cudaSuccess) {
         delete s;
@@ -840,8 +840,8 @@ pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid
     if (e != cudaSuccess && st == PZ_OK) st = s->cuda(w, e);
     return e == cudaSuccess;
   };
-  if (CK(cudaMalloc(&d_ks, ks.size() * 4), "cudaMalloc") && CK(cudaMalloc(&d_desc, batch * 4), "cudaMalloc") &&
-      CK(cudaMalloc(&d_out, batch * 4), "cudaMalloc") && CK(cudaMalloc(&d_g, batch), "cudaMalloc") &&
+  if (CK(pz::dev_malloc(&d_ks, ks.size() * 4), "cudaMalloc") && CK(pz::dev_malloc(&d_desc, batch * 4), "cudaMalloc") &&
+      CK(pz::dev_malloc(&d_out, batch * 4), "cudaMalloc") && CK(pz::dev_malloc(&d_g, batch), "cudaMalloc") &&
       CK(cudaMemcpy(d_ks, ks.data(), ks.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy") &&
       CK(cudaMemcpy(d_desc, desc.data(), batch * 4, cudaMemcpyHostToDevice), "cudaMemcpy") &&
       CK(cudaMemcpy(d_out, outi.data(), batch * 4, cudaMemcpyHostToDevice), "cudaMemcpy") &&

@@ -98,9 +98,9 @@ pz_status pz_key_import(pz_ctx *c, const void *buf, size_t size, pz_key **out) {
   k->ctx = c;
   k->bytes = rg + au + ks;
   const unsigned char *p = (const unsigned char *)buf + sizeof h;
-  cudaError_t e = cudaMalloc(&k->d_rgsw, rg);
-  if (e == cudaSuccess) e = cudaMalloc(&k->d_autos, au);
-  if (e == cudaSuccess) e = cudaMalloc(&k->d_ksk, ks);
+  cudaError_t e = pz::dev_malloc(&k->d_rgsw, rg);
+  if (e == cudaSuccess) e = pz::dev_malloc(&k->d_autos, au);
+  if (e == cudaSuccess) e = pz::dev_malloc(&k->d_ksk, ks);
   if (e == cudaSuccess) e = cudaMemcpy(k->d_rgsw, p, rg, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(k->d_autos, p + rg, au, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(k->d_ksk, p + rg + au, ks, cudaMemcpyHostToDevice);
