@@ -648,6 +648,53 @@ __global__ void __launch_bounds__(Shape<F>::THREADS, Shape<F>::CTAS)
   tmem_end<F>(&tmem_slot);
 }
 
+// External products (AUTO: automorphisms) by themselves: one operation per
+// ciphertext, QUAD's, CTAs taking ciphertexts in turn.  An index out of range
+// leaves its ciphertext unchanged.  Inputs need not be canonical: the digits
+// are the decomposer's for any word.
+template <bool AUTO>
+__global__ void __launch_bounds__(T, 4)
+    op_fft_kernel(const __grid_constant__ BrParams P, u64 *rlwe, const u32 *idx, size_t count, int trivial) {
+  extern __shared__ __align__(128) u64 smem[];
+  __shared__ u32 tmem_slot;
+  const u32 tm = tmem_begin<QUAD>(&tmem_slot);
+  const Smem<QUAD> S(smem);
+  const int t = threadIdx.x;
+  const Place p(t, 0, tm + Shape<QUAD>::TURN);
+  for (int i = t; i < TW_WORDS; i += T) S.tw()[i] = ldc((const cplx *)P.fft_tw + i);
+  u32 q = 0;
+  for (size_t c = blockIdx.x; c < count; c += gridDim.x) {
+    const u32 i = idx[c];
+    if (AUTO ? i > P.w : i >= P.n) continue;  // uniform
+    const u32 op = AUTO ? OP_AUTO | i : i;
+    const cplx *key = op_key(P, op);
+    if (t == 0) prefetch_l2(key, 2 * M * (u32)sizeof(cplx));
+    u64 *x = rlwe + c * 2 * N;
+    __syncthreads();  // the last ciphertext's use of S
+    int *da = S.da(0), *db = S.db(0, q);
+    long long *ub = S.ub(0, q);
+    if (AUTO) {
+      u32 at = (u32)t * P.auto_k[i];
+#pragma unroll
+      for (int m = 0; m < 16; m++, at += T * P.auto_k[i]) {
+        const u64 a = x[t + T * m];
+        const long long b = (long long)reduce_n2048(x[N + t + T * m]);
+        da[at & (N - 1)] = digit_any<AUTO_LOGB, AUTO_IGN>((at & N) ? Q_N2048 - a : a);
+        ub[at & (N - 1)] = (at & N) ? -b : b;
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < 16; m++) {
+        da[t + T * m] = trivial ? 0 : digit_any<RLRG_LOGB, RLRG_IGN>(x[t + T * m]);  // a = 0 (runtime.rs:790)
+        db[t + T * m] = digit_any<RLRG_LOGB, RLRG_IGN>(x[N + t + T * m]);
+      }
+    }
+    op_sync();
+    op_quad(0, op, OP_END, key, nullptr, P, S, q, tm, p, [&](int o, int e, u64 v) { x[o * N + e] = v; });
+  }
+  tmem_end<QUAD>(&tmem_slot);
+}
+
 }  // namespace fft
 
 using fft::cplx;
@@ -774,6 +821,25 @@ cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc,
                                   size_t count, int grid, cudaStream_t s, bool split) {
   return launch_fft(BrParams{}, d_descs, item_desc, out_idx, max_br_q, max_n, ks, ks_stride, gates, out, count, nullptr,
                     grid, s, split);
+}
+
+template <bool AUTO>
+static cudaError_t launch_op(const BrParams &P, u64 *rlwe, const u32 *idx, size_t count, int trivial, cudaStream_t s) {
+  constexpr size_t smem = fft::Shape<fft::QUAD>::WORDS * 8;
+  const cudaError_t e = opt_in_smem((const void *)fft::op_fft_kernel<AUTO>, smem);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const unsigned grid = (unsigned)std::min<size_t>(count, (size_t)4 * sms);
+  fft::op_fft_kernel<AUTO><<<grid, fft::T, smem, s>>>(P, rlwe, idx, count, trivial);
+  return cudaGetLastError();
+}
+cudaError_t launch_fft_product(const BrParams &P, u64 *rlwe, const u32 *idx, size_t count, int trivial,
+                               cudaStream_t s) {
+  return launch_op<false>(P, rlwe, idx, count, trivial, s);
+}
+cudaError_t launch_fft_auto(const BrParams &P, u64 *rlwe, const u32 *slot, size_t count, cudaStream_t s) {
+  return launch_op<true>(P, rlwe, slot, count, 0, s);
 }
 
 }  // namespace pz

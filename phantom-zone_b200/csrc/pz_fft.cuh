@@ -583,6 +583,16 @@ template <int IGN>
 __device__ __forceinline__ int digit(long long c) {
   return (int)((c + (1ll << (IGN - 1))) >> IGN);
 }
+// The decomposer's signed digit of any 64-bit word (one outside [0, Q) may
+// round above half the base).
+template <int LOGB, int IGN>
+__device__ __forceinline__ int digit_any(u64 v) {
+  if (v >= (Q_N2048 >> 1)) v = v - Q_N2048;
+  const u32 r = (u32)(v >> IGN) + (u32)((v >> (IGN - 1)) & 1ull);
+  const u32 k = r & ((1u << LOGB) - 1u), half = 1u << (LOGB - 1);
+  const bool c = k > half || (k == half && ((r >> LOGB) & 1u));
+  return (int)k - (c ? (1 << LOGB) : 0);
+}
 static_assert(RLRG_LOGB + RLRG_IGN == 54 && AUTO_LOGB + AUTO_IGN == 54, "one digit covers Q");
 
 }  // namespace fft

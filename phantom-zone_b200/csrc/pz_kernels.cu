@@ -1110,18 +1110,15 @@ cudaError_t launch_ntt_inv(int logn, u64 *polys, size_t count, const RingConsts 
 }
 
 cudaError_t launch_ext_product(int logn, bool d1, const BrParams &P, u64 *rlwe, const u32 *idx,
-                               size_t count, int trivial, cudaStream_t s, int variant) {
+                               size_t count, int trivial, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
+  if (logn == 11 && d1 && P.fft_rgsw) return launch_fft_product(P, rlwe, idx, count, trivial, s);
   const size_t N = (size_t)1 << logn, smem = OP_REGIONS * N * 8;
   cudaError_t e;
 #define PZ_LAUNCH(LN, DD, MB, TH)                                                                  \
   if ((e = set_smem(ext_product_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;              \
   ext_product_kernel<LN, DD, MB><<<grid_for(count), TH, smem, s>>>(P, rlwe, idx, count, trivial);
-  if (logn == 11 && d1) {
-    if (variant == 0) { PZ_LAUNCH(11, true, 2, 256) }
-    else if (variant == 2) { PZ_LAUNCH(11, true, 4, 256) }
-    else { PZ_LAUNCH(11, true, 3, 256) }
-  }
+  if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }
   else if (logn == 11) { PZ_LAUNCH(11, false, 1, 256) }
   else if (logn == 9 && d1) { PZ_LAUNCH(9, true, 1, 64) }
   else if (logn == 9) { PZ_LAUNCH(9, false, 1, 64) }
@@ -1131,18 +1128,15 @@ cudaError_t launch_ext_product(int logn, bool d1, const BrParams &P, u64 *rlwe, 
 }
 
 cudaError_t launch_auto(int logn, bool d1, const BrParams &P, u64 *rlwe, const u32 *slot, size_t count,
-                        int trivial, cudaStream_t s, int variant) {
+                        int trivial, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
+  if (logn == 11 && d1 && P.fft_autos && !trivial) return launch_fft_auto(P, rlwe, slot, count, s);
   const size_t N = (size_t)1 << logn, smem = OP_REGIONS * N * 8;
   cudaError_t e;
 #define PZ_LAUNCH(LN, DD, MB, TH)                                                           \
   if ((e = set_smem(auto_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;              \
   auto_kernel<LN, DD, MB><<<grid_for(count), TH, smem, s>>>(P, rlwe, slot, count, trivial);
-  if (logn == 11 && d1) {
-    if (variant == 0) { PZ_LAUNCH(11, true, 2, 256) }
-    else if (variant == 2) { PZ_LAUNCH(11, true, 4, 256) }
-    else { PZ_LAUNCH(11, true, 3, 256) }
-  }
+  if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }
   else if (logn == 11) { PZ_LAUNCH(11, false, 1, 256) }
   else if (logn == 9 && d1) { PZ_LAUNCH(9, true, 1, 64) }
   else if (logn == 9) { PZ_LAUNCH(9, false, 1, 64) }

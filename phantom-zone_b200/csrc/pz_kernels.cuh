@@ -73,12 +73,10 @@ cudaError_t launch_key_convert(int logn, const u64 *in, u64 *out, size_t npolys,
 // err: the context's device error word (DEVERR_* bits)
 cudaError_t launch_ntt_fwd(int logn, u64 *polys, size_t count, const RingConsts &rc, u32 *err, cudaStream_t s);
 cudaError_t launch_ntt_inv(int logn, u64 *polys, size_t count, const RingConsts &rc, u32 *err, cudaStream_t s);
-// variant: register cap of the one-digit forms as the blind rotation's
-// launch shapes 0 / 1 / 2 (2 / 3 / 4 CTAs per SM; other values: 3)
 cudaError_t launch_ext_product(int logn, bool d1, const BrParams &P, u64 *rlwe, const u32 *idx,
-                               size_t count, int trivial, cudaStream_t s, int variant = 1);
+                               size_t count, int trivial, cudaStream_t s);
 cudaError_t launch_auto(int logn, bool d1, const BrParams &P, u64 *rlwe, const u32 *slot, size_t count,
-                        int trivial, cudaStream_t s, int variant = 1);
+                        int trivial, cudaStream_t s);
 // reduce_output: leave every output word reduced mod q_ks (otherwise the
 // words may carry multiples of q_ks, and consumers mask with q_ks - 1)
 // ct: ciphertexts per CTA (8, 16 or 32)
@@ -133,6 +131,9 @@ cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas);  // resident CTAs per SM
 cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc, u32 max_br_q, u32 max_n, const u32 *ks,
                                   u32 ks_stride, const unsigned char *gates, u64 *out, const u32 *out_idx,
                                   size_t count, int grid, cudaStream_t s, bool split);
+cudaError_t launch_fft_product(const BrParams &P, u64 *rlwe, const u32 *idx, size_t count, int trivial,
+                               cudaStream_t s);
+cudaError_t launch_fft_auto(const BrParams &P, u64 *rlwe, const u32 *slot, size_t count, cudaStream_t s);
 cudaError_t launch_not(const u64 *in, u64 *out, size_t words, u64 q, cudaStream_t s);
 cudaError_t launch_imad_probe(int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);
 cudaError_t launch_pipe_probe(int kind, int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);
