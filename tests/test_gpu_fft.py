@@ -1,0 +1,90 @@
+"""The FFT products at the edges of their exactness bound, and the forms of the
+blind rotation at the batch sizes where one takes over from another."""
+import numpy as np
+import pytest
+
+from conftest import oracle, oracle_setup, pz, to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+
+def _extremes(Q):
+    """Key words whose three 18-bit limbs are all as large as they get, and the
+    ends of the centred range."""
+    low = -((1 << 17) + (1 << 35) + (((1 << 17) - 1) << 36))  # limbs -2^17, -2^17, 1 - 2^17
+    high = ((1 << 17) - 1) * (1 + (1 << 18) + (1 << 36))
+    return [v % Q for v in (low, high, Q // 2, Q // 2 + 1, Q - 1, 0, 1 << 35, 1 << 17)]
+
+
+@pytest.mark.parametrize("signs", ["same", "alternating", "random"])
+def test_products_of_extreme_words(gpu_available, signs):
+    """Digits of +-2^16 (products) and +-2^23 (automorphisms) in every coefficient
+    against keys with every limb at its largest: the largest sums there are,
+    exact word for word."""
+    O = oracle()
+    ev = O.Evaluator("NI_2P")
+    i, N, Q = ev.info, ev.N, ev.Q
+    g = np.random.default_rng(7)
+    words = _extremes(Q)
+
+    def pattern(v, shape):
+        s = {"same": np.zeros(shape, bool), "alternating": np.arange(np.prod(shape)).reshape(shape) % 2 == 1,
+             "random": g.integers(0, 2, shape).astype(bool)}[signs]
+        return np.where(s, np.uint64((Q - v) % Q), np.uint64(v))
+
+    rgsw = np.zeros((ev.n, i.rgsw_rows, N), np.uint64)
+    autos = np.zeros((i.w + 1, i.auto_rows, N), np.uint64)
+    for k, v in enumerate(words):
+        rgsw[k] = pattern(v, rgsw[k].shape)
+        autos[k] = pattern(v, autos[k].shape)
+    ksk = np.zeros((i.lwe_d * N, ev.n + 1), np.uint64)
+    okey = O.OracleKey(ev, O.ServerKeyCoeff(rgsw, autos, ksk))
+    eng = pz().Engine("NI_2P")
+    key = eng.upload_key(rgsw, autos, ksk)
+    inputs = np.stack([pattern(v, (2, N)) for v in (Q // 2 - 1, Q // 2, Q // 2 + 1, (1 << 36) - 1, 1 << 36, 0)])
+    idx = np.repeat(np.arange(len(words)), len(inputs)).astype(np.uint32)
+    rl = np.concatenate([inputs] * len(words))
+    for device, host in ((eng.rlwe_by_rgsw_device, okey.rlwe_by_rgsw), (eng.rlwe_auto_device, okey.rlwe_auto)):
+        t = to_dev(rl)
+        device(key, t, to_dev(idx))
+        want = np.stack([host(r.reshape(-1), int(k)) for r, k in zip(rl, idx)])
+        assert np.array_equal(to_host(t).reshape(len(rl), -1), want)
+
+
+@pytest.mark.parametrize("param", ["I_2P_LB_SR", "NI_8P"])
+def test_forms_agree(gpu_available, param):
+    """The same key-switched ciphertexts in batches on either side of each form's
+    range, with more ciphertexts than a form has places, and with few CTAs:
+    the same words, and the oracle's for some."""
+    import torch
+    ev, _, coeff, okey = oracle_setup(param)
+    eng = pz().Engine(param)
+    key = eng.upload_key(coeff.rgsw, coeff.autos, coeff.ksk)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    most = 4 * sms + 3
+    r = oracle().Rng(b"\x5f" * 32)
+    ks = r.uniform_mod(ev.info.lwe_q, most * (ev.n + 1)).reshape(most, -1).astype(np.uint32)
+    gates = (np.arange(most) % 6).astype(np.uint8)
+
+    def run(count, limit=0, split=-1):
+        eng.set_split_threshold(split)
+        eng.set_pbs_grid_limit(limit)
+        out = to_dev(np.zeros((count, ev.L), np.uint64))
+        eng.blind_rotate_device(key, to_dev(ks[:count]), to_dev(gates[:count]), out)
+        return to_host(out)
+
+    try:
+        full = run(most)
+        for count, limit, split in [(1, 0, -1), (sms // 2, 0, -1), (sms // 2 + 1, 0, -1), (sms, 0, 0), (sms + 1, 0, -1),
+                                    (13, 5, 74), (13, 5, 0), (2, 0, 0)]:
+            assert np.array_equal(run(count, limit, split), full[:count]), (count, limit, split)
+        # one gate through the debug entry point: the rotated RLWE is the oracle's
+        c0 = r.uniform_mod(ev.Q, 2 * ev.L).reshape(2, ev.L)
+        c1 = r.uniform_mod(ev.Q, 2 * ev.L).reshape(2, ev.L)
+        out = to_dev(np.zeros((2, ev.L), np.uint64))
+        eng.gate_batch_device(key, to_dev(gates[:2]), to_dev(c0), to_dev(c1), out)
+        assert np.array_equal(to_host(out), okey.gate_batch(gates[:2], c0, c1, threads=2))
+        assert eng.device_error() == 0
+    finally:
+        eng.set_split_threshold(-1)
+        eng.set_pbs_grid_limit(0)
