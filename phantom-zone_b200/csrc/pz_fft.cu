@@ -16,92 +16,20 @@ namespace fft {
 constexpr int N = 2048;
 constexpr u32 OP_END = 0xffffffffu;
 
-// ---------------------------------------------------------------------------
-// Key form: the device rows (evaluation domain, K N^{-1}) back to
-// coefficients, cut into limbs, and each limb transformed in double-double
-// arithmetic, scaled by 1 / M (exact) and rounded once.
-// ---------------------------------------------------------------------------
-struct dd {
-  double h, l;
-};
-__device__ __forceinline__ dd dd_norm(double a, double b) {  // |a| >= |b|
-  const double s = a + b;
-  return {s, b - (s - a)};
-}
-__device__ __forceinline__ dd dd_add(dd a, dd b) {
-  const double s = a.h + b.h, bb = s - a.h;
-  const double e = (a.h - (s - bb)) + (b.h - bb);
-  return dd_norm(s, e + (a.l + b.l));
-}
-__device__ __forceinline__ dd dd_neg(dd a) { return {-a.h, -a.l}; }
-__device__ __forceinline__ dd dd_mul(dd a, dd b) {
-  const double p = a.h * b.h;
-  const double e = fma(a.h, b.h, -p);
-  return dd_norm(p, e + (a.h * b.l + a.l * b.h));
-}
-
-// One CTA per (key block, row).  rows_per_key device rows per key: 4 for RGSW
-// (A(-sm), B(-sm), A(m), B(m)), 2 for automorphism keys (A, B), whose second
-// digit half uses 2^AUTO_CUT times the row.
+// Key form of the blind rotation.  One CTA per (key block, row).  rows_per_key
+// device rows per key: 4 for RGSW (A(-sm), B(-sm), A(m), B(m)), 2 for
+// automorphism keys (A, B), whose second digit half uses 2^AUTO_CUT times the row.
 __global__ void __launch_bounds__(256)
     fft_key_kernel(const u64 *rows, cplx *out, u32 rows_per_key, RingConsts rc, const double4 *tw) {
   __shared__ u64 coef[N];
   extern __shared__ double dyn[];
-  double *re_h = dyn, *re_l = dyn + M, *im_h = dyn + 2 * M, *im_l = dyn + 3 * M;
-  const int j = threadIdx.x;
   const u32 key = blockIdx.x >> 2, in = (blockIdx.x >> 1) & 1, o = blockIdx.x & 1;
   const u32 row = rows_per_key == 4 ? 2 * in + o : o;
-  const u64 *src = rows + ((size_t)key * rows_per_key + row) * N;
-  u64 x[8];
-#pragma unroll
-  for (int r = 0; r < 8; r++) x[r] = src[dev_index<11>(j, r)];
-  ntt_inv<11>(x, coef, rc);
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    u64 v = reduce2(x[r], Q_N2048);
-    if (rows_per_key == 2 && in)  // 2^12 v mod Q
-      v = reduce2(reduce_n2048(((v & ((1ull << (54 - AUTO_CUT)) - 1)) << AUTO_CUT) + 77823ull * (v >> (54 - AUTO_CUT))),
-                  Q_N2048);
-    coef[pos_coef<11>(j, r)] = v;
-  }
+  key_coefficients(rows + ((size_t)key * rows_per_key + row) * N, coef, rc, rows_per_key == 2 && in ? AUTO_CUT : 0);
   for (int limb = 0; limb < LIMBS; limb++) {
-    __syncthreads();
-    auto cut = [&](u64 u) -> double {
-      long long v = u > (Q_N2048 >> 1) ? (long long)(u - Q_N2048) : (long long)u;
-      long long k = 0;
-      for (int l = 0; l <= limb; l++) {
-        k = l + 1 < LIMBS ? ((v + (1 << (LIMB_BITS - 1))) & ((1 << LIMB_BITS) - 1)) - (1 << (LIMB_BITS - 1)) : v;
-        v = (v - k) >> LIMB_BITS;
-      }
-      return (double)k;
-    };
-    for (int e = j; e < M; e += 256) {
-      re_h[e] = cut(coef[e]);
-      im_h[e] = cut(coef[e + M]);
-      re_l[e] = im_l[e] = 0;
-    }
-    for (int s = 0; s < 10; s++) {
-      const int half = M >> (s + 1);
-      __syncthreads();
-      for (int e = j; e < M / 2; e += 256) {
-        const int k = e / half, a = k * 2 * half + e % half, b = a + half;
-        const double4 w = tw[(1 << s) + k];  // y(s, k): re hi, re lo, im hi, im lo
-        const dd wr{w.x, w.y}, wi{w.z, w.w};
-        const dd ar{re_h[a], re_l[a]}, ai{im_h[a], im_l[a]}, br{re_h[b], re_l[b]}, bi{im_h[b], im_l[b]};
-        const dd tr = dd_add(dd_mul(wr, br), dd_neg(dd_mul(wi, bi)));
-        const dd ti = dd_add(dd_mul(wr, bi), dd_mul(wi, br));
-        const dd pr = dd_add(ar, tr), pi = dd_add(ai, ti), mr = dd_add(ar, dd_neg(tr)), mi = dd_add(ai, dd_neg(ti));
-        re_h[a] = pr.h; re_l[a] = pr.l; im_h[a] = pi.h; im_l[a] = pi.l;
-        re_h[b] = mr.h; re_l[b] = mr.l; im_h[b] = mi.h; im_l[b] = mi.l;
-      }
-    }
-    __syncthreads();
+    key_limb<LIMBS, LIMB_BITS>(coef, limb, dyn, tw);
     cplx *dst = out + (size_t)key * KEY_BLOCK + (size_t)(o * LIMBS + limb) * 2 * M;
-    for (int e = j; e < M; e += 256) {  // evaluation position e, layout E
-      const int t = ((e >> 8) << 5) | (((e >> 5) & 7) << 2) | ((e >> 2) & 3), r = (((e >> 4) & 1) << 2) | (e & 3);
-      dst[(2 * r + in) * T + t] = cplx{re_h[e] * (1.0 / M), im_h[e] * (1.0 / M)};
-    }
+    for (int e = threadIdx.x; e < M; e += 256) dst[(2 * eval_register(e) + in) * T + eval_thread(e)] = key_value(dyn, e);
   }
 }
 
@@ -755,7 +683,7 @@ cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const
                            void *out, cudaStream_t s) {
   if (keys == 0) return cudaSuccess;
   const double4 *tw = (const double4 *)((const cplx *)tables + fft::TW_WORDS);
-  fft::fft_key_kernel<<<(unsigned)(4 * keys), 256, 4 * fft::M * 8, s>>>(rows, (cplx *)out, rows_per_key, rc, tw);
+  fft::fft_key_kernel<<<(unsigned)(4 * keys), 256, fft::KEY_SMEM, s>>>(rows, (cplx *)out, rows_per_key, rc, tw);
   return cudaGetLastError();
 }
 

@@ -560,11 +560,11 @@ __device__ __forceinline__ void add_limb2(u64 &acc, double z) {
 }
 // The sum of the limbs (in (-2^47, 2^56) once ROUND_SUM is taken off) -> a
 // representative mod Q in [-2^53 - 2^20, 2^53 + 2^20].
-__device__ __forceinline__ long long settle(u64 acc) {
-  acc -= ROUND_SUM;
+__device__ __forceinline__ long long settle_sum(u64 acc) {
   const int h = ((int)(acc >> 32) + (1 << 21)) >> 22;
   return (long long)(acc - ((u64)((u32)h << 22) << 32)) + (long long)h * 77823ll;
 }
+__device__ __forceinline__ long long settle(u64 acc) { return settle_sum(acc - ROUND_SUM); }
 // The decomposer's centred form, [-(Q + 1)/2, (Q - 3)/2] (decomposer.rs:217-234:
 // v >= Q >> 1 -> v - Q), of a representative in (-1.5 Q, 1.5 Q).
 __device__ __forceinline__ long long centre(long long c) {
@@ -594,6 +594,90 @@ __device__ __forceinline__ int digit_any(u64 v) {
   return (int)k - (c ? (1 << LOGB) : 0);
 }
 static_assert(RLRG_LOGB + RLRG_IGN == 54 && AUTO_LOGB + AUTO_IGN == 54, "one digit covers Q");
+
+// ---------------------------------------------------------------------------
+// Key form: device rows (evaluation domain, K N^{-1}) back to coefficients, cut
+// into limbs, and each limb transformed in double-double arithmetic, scaled by
+// 1 / M (exact) and rounded once.  CTAs of 256 threads.
+// ---------------------------------------------------------------------------
+struct dd {
+  double h, l;
+};
+__device__ __forceinline__ dd dd_norm(double a, double b) {  // |a| >= |b|
+  const double s = a + b;
+  return {s, b - (s - a)};
+}
+__device__ __forceinline__ dd dd_add(dd a, dd b) {
+  const double s = a.h + b.h, bb = s - a.h;
+  const double e = (a.h - (s - bb)) + (b.h - bb);
+  return dd_norm(s, e + (a.l + b.l));
+}
+__device__ __forceinline__ dd dd_neg(dd a) { return {-a.h, -a.l}; }
+__device__ __forceinline__ dd dd_mul(dd a, dd b) {
+  const double p = a.h * b.h;
+  const double e = fma(a.h, b.h, -p);
+  return dd_norm(p, e + (a.h * b.l + a.l * b.h));
+}
+
+constexpr size_t KEY_SMEM = 4 * M * sizeof(double);  // re, im: high and low parts
+// position e in layout E
+__device__ __forceinline__ int eval_thread(int e) { return ((e >> 8) << 5) | (((e >> 5) & 7) << 2) | ((e >> 2) & 3); }
+__device__ __forceinline__ int eval_register(int e) { return (((e >> 4) & 1) << 2) | (e & 3); }
+
+// coef (shared, N words) = the row's coefficients times 2^up mod Q
+__device__ __forceinline__ void key_coefficients(const u64 *row, u64 *coef, const RingConsts &rc, int up) {
+  const int j = threadIdx.x;
+  u64 x[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) x[r] = row[dev_index<11>(j, r)];
+  ntt_inv<11>(x, coef, rc);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    u64 v = reduce2(x[r], Q_N2048);
+    if (up) v = reduce2(reduce_n2048(((v & ((1ull << (54 - up)) - 1)) << up) + 77823ull * (v >> (54 - up))), Q_N2048);
+    coef[pos_coef<11>(j, r)] = v;
+  }
+}
+// work (shared) = the transform of limb `limb` of LIMBS_ limbs of BITS bits
+template <int LIMBS_, int BITS>
+__device__ __forceinline__ void key_limb(const u64 *coef, int limb, double *work, const double4 *tw) {
+  double *re_h = work, *re_l = work + M, *im_h = work + 2 * M, *im_l = work + 3 * M;
+  const int j = threadIdx.x;
+  auto cut = [&](u64 u) -> double {
+    long long v = u > (Q_N2048 >> 1) ? (long long)(u - Q_N2048) : (long long)u, k = 0;
+    for (int l = 0; l <= limb; l++) {
+      k = l + 1 < LIMBS_ ? ((v + (1 << (BITS - 1))) & ((1 << BITS) - 1)) - (1 << (BITS - 1)) : v;
+      v = (v - k) >> BITS;
+    }
+    return (double)k;
+  };
+  __syncthreads();
+  for (int e = j; e < M; e += 256) {
+    re_h[e] = cut(coef[e]);
+    im_h[e] = cut(coef[e + M]);
+    re_l[e] = im_l[e] = 0;
+  }
+  for (int s = 0; s < 10; s++) {
+    const int half = M >> (s + 1);
+    __syncthreads();
+    for (int e = j; e < M / 2; e += 256) {
+      const int k = e >> (9 - s), a = k * 2 * half + (e & (half - 1)), b = a + half;
+      const double4 w = tw[(1 << s) + k];  // y(s, k): re hi, re lo, im hi, im lo
+      const dd wr{w.x, w.y}, wi{w.z, w.w};
+      const dd ar{re_h[a], re_l[a]}, ai{im_h[a], im_l[a]}, br{re_h[b], re_l[b]}, bi{im_h[b], im_l[b]};
+      const dd tr = dd_add(dd_mul(wr, br), dd_neg(dd_mul(wi, bi)));
+      const dd ti = dd_add(dd_mul(wr, bi), dd_mul(wi, br));
+      const dd pr = dd_add(ar, tr), pi = dd_add(ai, ti), mr = dd_add(ar, dd_neg(tr)), mi = dd_add(ai, dd_neg(ti));
+      re_h[a] = pr.h; re_l[a] = pr.l; im_h[a] = pi.h; im_l[a] = pi.l;
+      re_h[b] = mr.h; re_l[b] = mr.l; im_h[b] = mi.h; im_l[b] = mi.l;
+    }
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ cplx key_value(const double *work, int e) {
+  return cplx{work[e] * (1.0 / M), work[2 * M + e] * (1.0 / M)};
+}
 
 }  // namespace fft
 }  // namespace pz

@@ -134,6 +134,38 @@ cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc,
 cudaError_t launch_fft_product(const BrParams &P, u64 *rlwe, const u32 *idx, size_t count, int trivial,
                                cudaStream_t s);
 cudaError_t launch_fft_auto(const BrParams &P, u64 *rlwe, const u32 *slot, size_t count, cudaStream_t s);
+// Non-interactive key switch over FFT products (pz_fft_ni.cu; one-bit digits,
+// d = NI_FFT_D).  Bytes of a user's key form, of `rows` values' transformed
+// digits (and what may be read beyond them) and of one (value, user)'s sums;
+// `keys`: device array of the users' key forms.
+constexpr u32 NI_FFT_D = 50;
+size_t ni_fft_key_bytes(u32 d);
+size_t ni_fft_digit_bytes(u32 d, size_t rows);
+size_t ni_fft_sum_bytes();
+cudaError_t launch_ni_fft_key(const u64 *rows, u32 d, const void *tables, void *out,
+                              cudaStream_t s);  // rows: [2 d][N] coefficients
+// out = rlwe_key_switch(in), [rows][2][N]
+cudaError_t launch_ni_fft_switch(const u64 *in, u64 *out, size_t rows, u32 d, const Decomp &dp,
+                                 const void *const *keys, const void *tables, void *digits, void *sums, u32 *err,
+                                 cudaStream_t s);
+// Key aggregation: row v = row % (ra + rb) of LWE index idx0 + row / (ra + rb),
+// switched for every user, the user's NI RGSW row added and stored into the
+// leader's RGSW (rlwe x rgsw shape: rows A(-sm), B(-sm), A(m), B(m); only its
+// last zero-encryption and last -a value) or, for every other user t in
+// increasing id, into others[t][index]: rows v / ra + v for zero-encryption
+// values, 2 ra + r / 2 ra + rb + r for -a values.
+struct NiRowUser {
+  const u64 *self_leader, *not_leader;
+  u32 seg_b, seg_e;
+};
+struct NiRows {
+  u32 ra, rb, max_d, max_l, per_user, idx0, cnt;
+  const NiRowUser *users;
+  u64 *leader, *others;
+};
+cudaError_t launch_ni_fft_rows(const u64 *vals, size_t rows, u32 users, u32 d, const Decomp &dp, const NiRows &R,
+                               const void *const *keys, const void *tables, void *digits, void *sums, u32 *err,
+                               cudaStream_t s);
 cudaError_t launch_not(const u64 *in, u64 *out, size_t words, u64 q, cudaStream_t s);
 cudaError_t launch_imad_probe(int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);
 cudaError_t launch_pipe_probe(int kind, int blocks, int threads, u32 iters, u32 *sink, cudaStream_t s);

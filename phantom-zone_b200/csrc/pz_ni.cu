@@ -13,11 +13,8 @@
 //                exactly the order of the sequential stream, rejections
 //                included.  Also used to expand seeded server keys.
 //   key switch   rlwe_key_switch (runtime.rs:1001-1063) from the user's RLWE
-//                secret u_j to the ideal secret s: the 50 one-bit signed
-//                digits of -A are transformed two at a time and accumulated
-//                against the user's ui_to_s key rows (N^{-1} folded in;
-//                sums folded with 2^54 = 77823, see ni_mac), then one
-//                inverse transform of both outputs and B' += B.
+//                secret u_j to the ideal secret s, over FFT products
+//                (pz_fft_ni.cu).
 //   extract      BatchedFheBools::extract (ni_mp_api.rs:217-236): bool i is
 //                sample_extract (pbs.rs:423-449) at coefficient i % N of
 //                RLWE i / N.
@@ -36,9 +33,7 @@ namespace {
 using pz::ni::ChaChaKey;
 using pz::ni::chacha8_block;
 using pz::ni::uniform_from_word;
-using pz::ni::ni_mac;
 using pz::ni::NI_LOGN;
-using pz::ni::NI_T;
 constexpr u64 UNSEED_MARGIN = 1024;  // keystream words generated beyond the samples needed
 
 // Block b of stream blockIdx.y: the 8 u64 words 8b..8b+7 of the stream (two
@@ -121,148 +116,49 @@ __global__ void seeded_place_kernel(const u64 *samples, const unsigned char *acc
   }
 }
 
-// One RLWE per CTA: rlwe_key_switch of in[c] with the user's key rows.
-__global__ void __launch_bounds__(NI_T, 2)
-    ni_key_switch_kernel(pz::RingConsts rc, pz::Decomp dp, u32 d, const u64 *ksk, const u64 *in, u64 *out,
-                         size_t count) {
-  constexpr int N = 1 << NI_LOGN;
-  extern __shared__ u64 sm[];  // 2N words: exchange buffer of the two-polynomial transforms
-  const int j = threadIdx.x;
-  const u64 q = rc.q;
-  for (size_t c = blockIdx.x; c < count; c += gridDim.x) {
-    const u64 *p = in + c * 2 * N;
-    u64 st[8], oa[8], ob[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      st[r] = pz::decomp_init(q - p[pz::pos_coef<NI_LOGN>(j, r)], dp);  // elwise_neg_mut, then decompose
-      oa[r] = 0;
-      ob[r] = 0;
-    }
-#pragma unroll 1
-    for (u32 jd = 0; jd < d; jd += 2) {
-      const bool two = jd + 1 < d;  // uniform
-      u64 x[8], y[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        x[r] = pz::decomp_next(st[r], dp);
-        y[r] = two ? pz::decomp_next(st[r], dp) : 0;
-      }
-      if (two) pz::ntt_fwd<NI_LOGN, true>(x, y, sm, rc);
-      else pz::ntt_fwd<NI_LOGN, false>(x, x, sm, rc);
-      ni_mac(oa, ob, x, y, ksk + (size_t)jd * N, ksk + (size_t)(d + jd) * N, ksk + (size_t)(jd + 1) * N,
-             ksk + (size_t)(d + jd + 1) * N, two, rc);
-    }
-    pz::ntt_inv<NI_LOGN, true>(oa, ob, sm, rc);
-    u64 *o = out + c * 2 * N;
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int pc = pz::pos_coef<NI_LOGN>(j, r);
-      o[pc] = pz::reduce2(oa[r], q);
-      o[N + pc] = pz::add_mod(pz::reduce2(ob[r], q), p[N + pc], q);  // elwise_add_mut(B', B)
-    }
-    __syncthreads();
-  }
-}
-
-// Small batches: the digits of one RLWE split over gridDim.y CTAs.  CTA
-// (c, s) runs the decomposition through digit pair `pend` of its share (the
-// signed digits carry from low to high, so every share walks the digits
-// before its own) and transforms and accumulates only pairs [pbeg, pend);
-// its partial (A, B) sums, evaluation domain in [0, 2q), go to
-// part[c][s][2][N] in the thread-major order ni_ks_finish_kernel reads.
-__global__ void __launch_bounds__(NI_T, 2)
-    ni_ks_partial_kernel(pz::RingConsts rc, pz::Decomp dp, u32 d, const u64 *ksk, const u64 *in, u64 *part,
-                         size_t count) {
-  constexpr int N = 1 << NI_LOGN;
-  extern __shared__ u64 sm[];
-  const int j = threadIdx.x;
-  const u64 q = rc.q;
-  const u32 pairs = (d + 1) / 2, share = (pairs + gridDim.y - 1) / gridDim.y;
-  const u32 pbeg = blockIdx.y * share, pend = min(pairs, pbeg + share);
-  for (size_t c = blockIdx.x; c < count; c += gridDim.x) {
-    const u64 *p = in + c * 2 * N;
-    u64 st[8], oa[8], ob[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      st[r] = pz::decomp_init(q - p[pz::pos_coef<NI_LOGN>(j, r)], dp);  // elwise_neg_mut, then decompose
-      oa[r] = 0;
-      ob[r] = 0;
-    }
-#pragma unroll 1
-    for (u32 pi = 0; pi < pbeg; pi++) {  // digits of the earlier shares: carries only
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        pz::decomp_next(st[r], dp);
-        if (2 * pi + 1 < d) pz::decomp_next(st[r], dp);
-      }
-    }
-#pragma unroll 1
-    for (u32 pi = pbeg; pi < pend; pi++) {
-      const u32 jd = 2 * pi;
-      const bool two = jd + 1 < d;  // uniform
-      u64 x[8], y[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        x[r] = pz::decomp_next(st[r], dp);
-        y[r] = two ? pz::decomp_next(st[r], dp) : 0;
-      }
-      if (two) pz::ntt_fwd<NI_LOGN, true>(x, y, sm, rc);
-      else pz::ntt_fwd<NI_LOGN, false>(x, x, sm, rc);
-      ni_mac(oa, ob, x, y, ksk + (size_t)jd * N, ksk + (size_t)(d + jd) * N, ksk + (size_t)(jd + 1) * N,
-             ksk + (size_t)(d + jd + 1) * N, two, rc);
-    }
-    u64 *o = part + (c * gridDim.y + blockIdx.y) * 2 * N;
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      o[r * NI_T + j] = oa[r];
-      o[N + r * NI_T + j] = ob[r];
-    }
-    __syncthreads();
-  }
-}
-
-// Sum of the `shares` partials (each < 2q, so the sum is reduced with the
-// special form of Q once), one inverse transform of both outputs, B' += B.
-__global__ void __launch_bounds__(NI_T, 2)
-    ni_ks_finish_kernel(pz::RingConsts rc, const u64 *part, u32 shares, const u64 *in, u64 *out, size_t count) {
-  constexpr int N = 1 << NI_LOGN;
-  extern __shared__ u64 sm[];
-  const int j = threadIdx.x;
-  const u64 q = rc.q;
-  for (size_t c = blockIdx.x; c < count; c += gridDim.x) {
-    u64 oa[8], ob[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) oa[r] = ob[r] = 0;
-    for (u32 sh = 0; sh < shares; sh++) {
-      const u64 *src = part + (c * shares + sh) * 2 * N;
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        oa[r] += src[r * NI_T + j];
-        ob[r] += src[N + r * NI_T + j];
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      oa[r] = pz::reduce_n2048(oa[r]);
-      ob[r] = pz::reduce_n2048(ob[r]);
-    }
-    pz::ntt_inv<NI_LOGN, true>(oa, ob, sm, rc);
-    const u64 *p = in + c * 2 * N;
-    u64 *o = out + c * 2 * N;
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int pc = pz::pos_coef<NI_LOGN>(j, r);
-      o[pc] = pz::reduce2(oa[r], q);
-      o[N + pc] = pz::add_mod(pz::reduce2(ob[r], q), p[N + pc], q);  // elwise_add_mut(B', B)
-    }
-    __syncthreads();
-  }
-}
-
 // out[c] = sample_extract(rlwe[idx[c] / N], idx[c] % N); an index past the
-// batch leaves out[c] unchanged.
-__global__ void extract_kernel(const u64 *rlwe, size_t rlwe_count, const u32 *idx, u64 *out, size_t count, u32 N,
-                               u64 q) {
+// batch leaves out[c] unchanged.  Bound by the writes (16 KB per bool): a CTA
+// takes EXTRACT_RUN entries in a row, keeps their RLWE in shared memory while it
+// stays the same, and stores 16 bytes per thread from the row's first 16-byte
+// boundary (rows are N + 1 words, so every other one starts off it).  49,152
+// bools of 24 RLWEs: 160 -> 129 us (6.2 TB/s).
+constexpr int EXTRACT_RUN = 8;
+__global__ void __launch_bounds__(256)
+    extract_kernel(const u64 *rlwe, size_t rlwe_count, const u32 *idx, u64 *out, size_t count, u64 q) {
+  constexpr int N = 1 << NI_LOGN;
+  __shared__ u64 ab[2 * N];  // a, b
+  size_t have = rlwe_count;  // the RLWE in ab
+  for (size_t c0 = (size_t)blockIdx.x * EXTRACT_RUN; c0 < count; c0 += (size_t)gridDim.x * EXTRACT_RUN) {
+    for (size_t c = c0; c < c0 + EXTRACT_RUN && c < count; c++) {
+      const u32 i = idx[c];
+      const size_t ct = i / N;
+      const int k = (int)(i % N);
+      if (ct >= rlwe_count) continue;  // uniform over the CTA
+      if (ct != have) {
+        __syncthreads();  // the last RLWE has been read
+        for (int t = threadIdx.x; t < 2 * N; t += 256) ab[t] = rlwe[ct * 2 * N + t];
+        __syncthreads();
+        have = ct;
+      }
+      auto word = [&](int t) -> u64 {
+        if (t == 0) return ab[N + k];
+        return t - 1 <= k ? ab[k + 1 - t] : q - ab[N + k + 1 - t];  // neg = q - x (modulus_u64.rs:147-149)
+      };
+      u64 *o = out + c * (size_t)(N + 1);
+      const int first = ((size_t)o & 8) ? 1 : 0;  // the row's words up to a 16-byte boundary
+      if (threadIdx.x == 0) o[first ? 0 : N] = word(first ? 0 : N);
+#pragma unroll
+      for (int p = 0; p < N / 512; p++) {
+        const int t = first + 2 * (threadIdx.x + 256 * p);
+        *(ulonglong2 *)(o + t) = make_ulonglong2(word(t), word(t + 1));
+      }
+    }
+  }
+}
+
+// ... for any ring size, one entry per CTA
+__global__ void extract_any_kernel(const u64 *rlwe, size_t rlwe_count, const u32 *idx, u64 *out, size_t count, u32 N,
+                                   u64 q) {
   for (size_t c = blockIdx.x; c < count; c += gridDim.x) {
     const u32 i = idx[c];
     const size_t ct = i / N, k = i % N;
@@ -274,7 +170,7 @@ __global__ void extract_kernel(const u64 *rlwe, size_t rlwe_count, const u32 *id
         o[0] = b[k];
       } else {
         const size_t ii = t - 1;
-        o[t] = ii <= k ? a[k - ii] : q - a[N + k - ii];  // neg = q - x (modulus_u64.rs:147-149)
+        o[t] = ii <= k ? a[k - ii] : q - a[N + k - ii];
       }
     }
   }
@@ -285,7 +181,23 @@ pz_status ni_check(pz_ctx *c) {
   if (c->P.variant != 2 || c->P.ni_ks_d == 0)
     return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "not a non-interactive parameter set");
   if (c->logn != NI_LOGN) return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "ring dimension other than 2048");
+  // the FFT products' exactness bound is for these (every non-interactive set)
+  if (c->P.ni_ks_logb != 1 || c->P.ni_ks_d != pz::NI_FFT_D || !c->d_fft)
+    return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "key-switch decomposition other than 50 one-bit digits");
   return PZ_OK;
+}
+
+// k's key form from its coefficient rows (device).  Synchronous.
+cudaError_t key_form(pz_ctx *c, pz_ni_ksk *k, const u64 *rows) {
+  const size_t bytes = pz::ni_fft_key_bytes(k->d);
+  cudaError_t e = pz::dev_malloc(&k->d_fft, bytes + sizeof(void *));
+  if (e == cudaSuccess) k->bytes = bytes + sizeof(void *);
+  const void *self = k->d_fft;
+  if (e == cudaSuccess) e = pz::launch_ni_fft_key(rows, k->d, c->d_fft, k->d_fft, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(k->d_fft + bytes, &self, sizeof self, cudaMemcpyHostToDevice, c->stream);
+  const cudaError_t e2 = cudaStreamSynchronize(c->stream);
+  return e != cudaSuccess ? e : e2;
 }
 
 int grid_of(size_t n, int cap) { return (int)std::min<size_t>(std::max<size_t>(n, 1), (size_t)cap); }
@@ -387,16 +299,13 @@ pz_status pz_ni_ksk_upload(pz_ctx *c, const uint64_t *ksk, pz_ni_ksk **out) {
   pz_ni_ksk *k = new pz_ni_ksk();
   k->ctx = c;
   k->d = c->P.ni_ks_d;
-  k->bytes = polys * N * 8;
   u64 *stage = nullptr;
-  cudaError_t e = pz::dev_malloc(&k->d_ksk, k->bytes);
-  if (e == cudaSuccess) e = pz::dev_malloc(&stage, k->bytes);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(stage, ksk, k->bytes, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = pz::launch_key_convert((int)c->logn, stage, k->d_ksk, polys, c->rc, c->ni_conv_c, c->ni_conv_cs, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaError_t e = pz::dev_malloc(&stage, polys * N * 8);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(stage, ksk, polys * N * 8, cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = key_form(c, k, stage);
   cudaFree(stage);
   if (e != cudaSuccess) {
-    cudaFree(k->d_ksk);
+    cudaFree(k->d_fft);
     delete k;
     return pz::cuda_fail(c, "pz_ni_ksk_upload", e);
   }
@@ -415,20 +324,16 @@ pz_status pz_ni_ksk_upload_seeded(pz_ctx *c, const uint64_t *ksk_b, const uint8_
   pz_ni_ksk *k = new pz_ni_ksk();
   k->ctx = c;
   k->d = (u32)d;
-  k->bytes = polys * N * 8;
   u64 *stage = nullptr;
-  cudaError_t e = pz::dev_malloc(&k->d_ksk, k->bytes);
-  if (e == cudaSuccess) e = pz::dev_malloc(&stage, k->bytes);
+  cudaError_t e = pz::dev_malloc(&stage, polys * N * 8);
   // keys.rs:965-1000: d A rows from the user's stream, then the B rows
   if (e == cudaSuccess) s = pz::seeded_fill_u64(c, seed, c->P.rlwe_q, (u64)d * N, d * N, 2 * d * N, 0, stage, c->stream);
   if (e == cudaSuccess && s == PZ_OK)
     e = cudaMemcpyAsync(stage + d * N, ksk_b, d * N * 8, cudaMemcpyDefault, c->stream);
-  if (e == cudaSuccess && s == PZ_OK)
-    e = pz::launch_key_convert((int)c->logn, stage, k->d_ksk, polys, c->rc, c->ni_conv_c, c->ni_conv_cs, c->stream);
-  if (e == cudaSuccess && s == PZ_OK) e = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess && s == PZ_OK) e = key_form(c, k, stage);
   cudaFree(stage);
   if (e != cudaSuccess || s != PZ_OK) {
-    cudaFree(k->d_ksk);
+    cudaFree(k->d_fft);
     delete k;
     return s != PZ_OK ? s : pz::cuda_fail(c, "pz_ni_ksk_upload_seeded", e);
   }
@@ -439,7 +344,7 @@ pz_status pz_ni_ksk_upload_seeded(pz_ctx *c, const uint64_t *ksk_b, const uint8_
 void pz_ni_ksk_release(pz_ni_ksk *k) {
   if (!k) return;
   cudaSetDevice(k->ctx->device);
-  cudaFree(k->d_ksk);
+  cudaFree(k->d_fft);
   delete k;
 }
 
@@ -468,28 +373,24 @@ pz_status pz_ni_key_switch_device(pz_ctx *c, const pz_ni_ksk *k, const uint64_t 
   if (count == 0) return PZ_OK;
   PZ_CK(c, cudaSetDevice(c->device));
   const pz::Decomp dp = pz::decomposer(c->P.rlwe_q, c->P.ni_ks_logb, c->P.ni_ks_d);
-  const size_t smem = 2 * (size_t)c->P.rlwe_n * 8;
   cudaStream_t st = (cudaStream_t)stream;
-  // fewer RLWEs than two per SM: split each one's digit pairs over CTAs
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  const u32 pairs = (k->d + 1) / 2;
-  const size_t shares = std::min<size_t>(std::min<size_t>(8, pairs), (2 * (size_t)sms + count - 1) / count);
-  if (shares <= 1) {
-    ni_key_switch_kernel<<<grid_of(count, 65535), NI_T, smem, st>>>(c->rc, dp, k->d, k->d_ksk, d_in, d_out, count);
-    PZ_CK(c, cudaGetLastError());
-    return PZ_OK;
+  // scratch: the transformed digits (0.8 MB per RLWE) and the sums, for at most
+  // 512 RLWEs at a time, fewer when there is no memory for that many
+  const size_t N = c->P.rlwe_n;
+  size_t chunk = std::min<size_t>(count, 512);
+  unsigned char *scratch = nullptr;
+  cudaError_t e;
+  while ((e = pz::pool_malloc(&scratch, pz::ni_fft_digit_bytes(k->d, chunk) + chunk * pz::ni_fft_sum_bytes(), st)) ==
+             cudaErrorMemoryAllocation &&
+         chunk > 1) {
+    cudaGetLastError();
+    chunk = (chunk + 1) / 2;
   }
-  u64 *part = nullptr;
-  PZ_CK(c, pz::pool_malloc(&part, count * shares * 2 * c->P.rlwe_n * 8, st));
-  ni_ks_partial_kernel<<<dim3((unsigned)count, (unsigned)shares), NI_T, smem, st>>>(c->rc, dp, k->d, k->d_ksk, d_in,
-                                                                                   part, count);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) {
-    ni_ks_finish_kernel<<<grid_of(count, 65535), NI_T, smem, st>>>(c->rc, part, (u32)shares, d_in, d_out, count);
-    e = cudaGetLastError();
-  }
-  cudaFreeAsync(part, st);
+  for (size_t i = 0; i < count && e == cudaSuccess; i += chunk)
+    e = pz::launch_ni_fft_switch(d_in + i * 2 * N, d_out + i * 2 * N, std::min(chunk, count - i), k->d, dp,
+                                 (const void *const *)(k->d_fft + pz::ni_fft_key_bytes(k->d)), c->d_fft, scratch,
+                                 scratch + pz::ni_fft_digit_bytes(k->d, chunk), c->d_err, st);
+  if (scratch) cudaFreeAsync(scratch, st);
   if (e != cudaSuccess) return pz::cuda_fail(c, "pz_ni_key_switch_device", e);
   return PZ_OK;
 }
@@ -500,8 +401,13 @@ pz_status pz_sample_extract_device(pz_ctx *c, const uint64_t *d_rlwe, size_t rlw
   if (count && (!d_rlwe || !d_index || !d_lwe)) return pz::fail(c, PZ_ERR_INVALID_ARGUMENT, "NULL argument");
   if (count == 0) return PZ_OK;
   PZ_CK(c, cudaSetDevice(c->device));
-  extract_kernel<<<grid_of(count, 65535), 256, 0, (cudaStream_t)stream>>>(d_rlwe, rlwe_count, d_index, d_lwe, count,
-                                                                          c->P.rlwe_n, c->P.rlwe_q);
+  if (c->logn != NI_LOGN) {
+    extract_any_kernel<<<grid_of(count, 65535), 256, 0, (cudaStream_t)stream>>>(d_rlwe, rlwe_count, d_index, d_lwe,
+                                                                                count, c->P.rlwe_n, c->P.rlwe_q);
+  } else {
+    extract_kernel<<<grid_of((count + EXTRACT_RUN - 1) / EXTRACT_RUN, 65535), 256, 0, (cudaStream_t)stream>>>(
+        d_rlwe, rlwe_count, d_index, d_lwe, count, c->P.rlwe_q);
+  }
   PZ_CK(c, cudaGetLastError());
   return PZ_OK;
 }

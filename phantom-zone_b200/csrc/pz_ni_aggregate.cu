@@ -10,22 +10,16 @@
 //   RGSWs          per LWE index l, in chunks of indices: the a_{l,i} rows
 //                  from the index's CRS stream (all chunk streams in one
 //                  batched seeded fill), the zero encryptions summed over
-//                  users; each of these d_a + d_b values is decomposed (50
-//                  one-bit digits) and transformed ONCE into HBM (the digit
-//                  kernel), then every (value, user) pair is one CTA of the
-//                  multiply-accumulate kernel: 50-digit MAC against that
-//                  user's key, one inverse transform of both outputs, the
-//                  user's NI RGSW row added (produce_rgsw_ciphertext_from_
-//                  ni_rgsw, :480-608) and the row stored straight into its
+//                  users; each of these d_a + d_b values is key-switched
+//                  for every user (pz_fft_ni.cu: its 50 one-bit digits
+//                  transformed ONCE), the user's NI RGSW row added
+//                  (produce_rgsw_ciphertext_from_ni_rgsw, :480-608) and the
+//                  row stored straight into its
 //                  place in the leader's RGSW (rlwe x rgsw shape) or in the
 //                  other users' RGSWs (rgsw x rgsw shape).  Then the batched
 //                  RGSW x RGSW products (pz_aggregate_rgsw_device) multiply
 //                  the leader's RGSW by the other users' in increasing id.
 //
-// Bytes per LWE index (NI_8P: d_a 20, d_b 18, 8 users): digits 38 x 50 x 16 KiB
-// = 31 MB written once and read by 8 users (L2-resident when the users of one
-// value run together, the grid's fastest index); key rows 1.6 MB per user,
-// shared by every index.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -36,20 +30,15 @@
 using pz::u32;
 using pz::u64;
 using pz::ni::NI_LOGN;
-using pz::ni::NI_T;
 
 namespace {
 
-struct NiUser {            // device view of one user's RGSW inputs
-  const u64 *ksk;          // [2 d][N] device key form (A rows, then B rows)
-  const u64 *self_leader;  // [segment][max_l][N]
-  const u64 *not_leader;   // [n - segment][max_d][N]
-  const u64 *zero_encs;    // [n][ra][N]
-  u32 seg_b, seg_e;        // multi_party_user_id_lwe_segment
+struct NiUser {          // device view of one user's values
+  const u64 *zero_encs;  // [n][ra][N]
 };
 
 struct NiShape {
-  u32 users, per_user, ra, rb, max_d, max_l, d;
+  u32 users, ra, rb, max_d;
 };
 
 // out[i] = sum_t src[t][i] mod q (elwise_add_mut over canonical rows)
@@ -86,108 +75,6 @@ __global__ void ni_values_kernel(const NiUser *users, NiShape sh, const u64 *aro
       x = q - arows[((size_t)c * sh.max_d + sh.max_d - sh.rb + (v - sh.ra)) * N + k];
     }
     vals[i] = x;
-  }
-}
-
-// One value row per CTA: its d one-bit digits, transformed two at a time,
-// stored [row][digit][N] in the thread-major order the MAC kernel reads back.
-__global__ void __launch_bounds__(NI_T, 2)
-    ni_digits_kernel(pz::RingConsts rc, pz::Decomp dp, u32 d, const u64 *vals, u64 *dig, size_t rows) {
-  constexpr int N = 1 << NI_LOGN;
-  extern __shared__ u64 sm[];  // 2N words: exchange buffer of the two-polynomial transforms
-  const int j = threadIdx.x;
-  for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    const u64 *p = vals + row * N;
-    u64 st[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) st[r] = pz::decomp_init(p[pz::pos_coef<NI_LOGN>(j, r)], dp);
-#pragma unroll 1
-    for (u32 jd = 0; jd < d; jd += 2) {
-      const bool two = jd + 1 < d;  // uniform
-      u64 x[8], y[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        x[r] = pz::decomp_next(st[r], dp);
-        y[r] = two ? pz::decomp_next(st[r], dp) : 0;
-      }
-      if (two) pz::ntt_fwd<NI_LOGN, true>(x, y, sm, rc);
-      else pz::ntt_fwd<NI_LOGN, false>(x, x, sm, rc);
-      u64 *o = dig + (row * d + jd) * N;
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        o[r * NI_T + j] = x[r];
-        if (two) o[N + r * NI_T + j] = y[r];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// One (index, value, user) item per CTA, user fastest.  The leader of an
-// index only needs the last zero-enc value (ra - 1) and the last -a value
-// (R - 1): its RGSW is in the rlwe x rgsw shape (d_a = d_b = 1), rows
-// [A(-sm), B(-sm), A(m), B(m)] in leader_out[c].  Every other user t (in
-// increasing id, the leader skipped) gets all R values: rows v / ra + v of
-// others[t][c] for zero-enc values, 2 ra + r / 2 ra + rb + r for -a values.
-__global__ void __launch_bounds__(NI_T, 2)
-    ni_agg_mac_kernel(pz::RingConsts rc, NiShape sh, const u64 *dig, const NiUser *users, u32 idx0, u32 cnt,
-                      u64 *leader_out, u64 *others) {
-  constexpr int N = 1 << NI_LOGN;
-  extern __shared__ u64 sm[];
-  const int j = threadIdx.x;
-  const u64 q = rc.q;
-  const u32 R = sh.ra + sh.rb, rows1 = 2 * R, d = sh.d;
-  const size_t items = (size_t)cnt * R * sh.users;
-  for (size_t it = blockIdx.x; it < items; it += gridDim.x) {
-    const u32 u = (u32)(it % sh.users), v = (u32)((it / sh.users) % R), c = (u32)(it / ((size_t)sh.users * R));
-    const u32 idx = idx0 + c, L = idx / sh.per_user;
-    const bool lead = u == L;
-    if (lead && v != sh.ra - 1 && v != R - 1) continue;  // uniform over the CTA
-    const NiUser U = users[u];
-    const u64 *kk = U.ksk;
-    const u64 *dv = dig + ((size_t)c * R + v) * d * N;
-    u64 oa[8], ob[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) oa[r] = ob[r] = 0;
-#pragma unroll 1
-    for (u32 jd = 0; jd < d; jd += 2) {
-      const bool two = jd + 1 < d;
-      u64 x[8], y[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        x[r] = dv[(size_t)jd * N + r * NI_T + j];
-        y[r] = two ? dv[(size_t)(jd + 1) * N + r * NI_T + j] : 0;
-      }
-      pz::ni::ni_mac(oa, ob, x, y, kk + (size_t)jd * N, kk + (size_t)(d + jd) * N, kk + (size_t)(jd + 1) * N,
-                     kk + (size_t)(d + jd + 1) * N, two, rc);
-    }
-    pz::ntt_inv<NI_LOGN, true>(oa, ob, sm, rc);
-    const bool to_a = v < sh.ra;  // -sm rows add the NI row to A, m rows to B
-    const u64 *ct;
-    u64 *oA, *oB;
-    if (lead) {
-      ct = U.self_leader + ((size_t)(idx - U.seg_b) * sh.max_l + (sh.max_l - 1)) * N;
-      oA = leader_out + ((size_t)c * 4 + (to_a ? 0 : 2)) * N;
-      oB = oA + N;
-    } else {
-      const u32 pos = idx < U.seg_b ? idx : idx - (U.seg_e - U.seg_b);
-      const u32 ctrow = to_a ? sh.max_d - sh.ra + v : sh.max_d - sh.rb + (v - sh.ra);
-      ct = U.not_leader + ((size_t)pos * sh.max_d + ctrow) * N;
-      const u32 t = u < L ? u : u - 1;
-      u64 *base = others + ((size_t)t * cnt + c) * rows1 * N;
-      oA = base + (size_t)(to_a ? v : 2 * sh.ra + (v - sh.ra)) * N;
-      oB = base + (size_t)(to_a ? sh.ra + v : 2 * sh.ra + sh.rb + (v - sh.ra)) * N;
-    }
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int pc = pz::pos_coef<NI_LOGN>(j, r);
-      u64 a = pz::reduce2(oa[r], q), b = pz::reduce2(ob[r], q);
-      if (to_a) a = pz::add_mod(a, ct[pc], q);
-      else b = pz::add_mod(b, ct[pc], q);
-      oA[pc] = a;
-      oB[pc] = b;
-    }
-    __syncthreads();
   }
 }
 
@@ -259,6 +146,8 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   if (P.variant != 2 || P.ni_ks_d == 0 || !P.rgrg_logb)
     return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "not a non-interactive parameter set");
   if (c->logn != NI_LOGN) return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "ring dimension other than 2048");
+  if (P.ni_ks_logb != 1 || P.ni_ks_d != pz::NI_FFT_D || !c->d_fft)
+    return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "key-switch decomposition other than 50 one-bit digits");
   if (P.rlrg_d_a != 1 || P.rlrg_d_b != 1)
     return pz::fail(c, PZ_ERR_NOT_SUPPORTED, "rlwe x rgsw decomposition count other than 1");
   if (!crs || !shares || users == 0 || !d_ksk_b || !d_rgsw || !d_auto_b || !d_lwe_b)
@@ -273,18 +162,22 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   const size_t N = P.rlwe_n, n = P.lwe_n, d = P.ni_ks_d;
   const u32 ra = P.rgrg_d_a, rb = P.rgrg_d_b, max_d = std::max(ra, rb), R = ra + rb;
   const size_t rows1 = 2 * (size_t)R;
-  NiShape sh{(u32)users, (u32)((n + users - 1) / users), ra, rb, max_d, 1, (u32)d};
+  NiShape sh{(u32)users, ra, rb, max_d};
   pz_status ps = PZ_OK;
   cudaError_t e = cudaSuccess;
   // ---- device buffers that live through the call
-  u64 *d_keys = nullptr, *d_stage = nullptr;
+  u64 *d_stage = nullptr;
+  unsigned char *d_keys = nullptr;  // the users' key forms, then their addresses
+  pz::NiRowUser *d_rows = nullptr;
+  const size_t key_bytes = pz::ni_fft_key_bytes((u32)d);
   const u64 **d_src = nullptr;
   NiUser *d_users = nullptr;
   const size_t nsrc = users * users + 2 * users;  // ksk lists, auto list, lwe list
-  if (e == cudaSuccess) e = pz::pool_malloc(&d_keys, users * 2 * d * N * 8, st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_keys, users * (key_bytes + sizeof(void *)), st);
   if (e == cudaSuccess) e = pz::pool_malloc(&d_stage, 2 * d * N * 8, st);
   if (e == cudaSuccess) e = pz::pool_malloc((void **)&d_src, nsrc * sizeof(u64 *), st);
   if (e == cudaSuccess) e = pz::pool_malloc(&d_users, users * sizeof(NiUser), st);
+  if (e == cudaSuccess) e = pz::pool_malloc(&d_rows, users * sizeof(pz::NiRowUser), st);
   // ---- ui_to_s key B rows (evaluator.rs:1269-1294), auto and LWE KSK sums
   std::vector<const u64 *> src(nsrc);
   for (size_t j = 0; j < users; j++) {
@@ -322,52 +215,73 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
     ps = pz::seeded_fill_u64(c, seed, P.rlwe_q, (u64)d * N, d * N, 2 * d * N, 0, d_stage, st);
     if (ps == PZ_OK) e = cudaMemcpyAsync(d_stage + d * N, d_ksk_b + j * d * N, d * N * 8, cudaMemcpyDeviceToDevice, st);
     if (ps == PZ_OK && e == cudaSuccess)
-      e = pz::launch_key_convert(NI_LOGN, d_stage, d_keys + j * 2 * d * N, 2 * d, c->rc, c->ni_conv_c, c->ni_conv_cs, st);
+      e = pz::launch_ni_fft_key(d_stage, (u32)d, c->d_fft, d_keys + j * key_bytes, st);
   }
   std::vector<NiUser> hu(users);
+  std::vector<pz::NiRowUser> hr(users);
+  std::vector<const void *> hk(users);
   for (size_t u = 0; u < users; u++) {
-    hu[u].ksk = d_keys + u * 2 * d * N;
-    hu[u].self_leader = shares[u].self_leader_cts;
-    hu[u].not_leader = shares[u].not_leader_cts;
+    hk[u] = d_keys + u * key_bytes;
     hu[u].zero_encs = shares[u].rgsw_zero_encs;
-    segment(u, users, n, &hu[u].seg_b, &hu[u].seg_e);
-    if ((hu[u].seg_e > hu[u].seg_b && !hu[u].self_leader) || (hu[u].seg_e - hu[u].seg_b < n && !hu[u].not_leader))
+    hr[u].self_leader = shares[u].self_leader_cts;
+    hr[u].not_leader = shares[u].not_leader_cts;
+    segment(u, users, n, &hr[u].seg_b, &hr[u].seg_e);
+    if ((hr[u].seg_e > hr[u].seg_b && !hr[u].self_leader) || (hr[u].seg_e - hr[u].seg_b < n && !hr[u].not_leader))
       ps = pz::fail(c, PZ_ERR_INVALID_ARGUMENT, "pz_ni_aggregate_device: NULL NI RGSW ciphertexts");
   }
   if (e == cudaSuccess && ps == PZ_OK)
     e = cudaMemcpyAsync(d_users, hu.data(), users * sizeof(NiUser), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && ps == PZ_OK) e = cudaStreamSynchronize(st);  // hu, src leave scope only after this
-  // ---- RGSWs, chunk by chunk of LWE indices
-  const size_t per_index = ((size_t)R * d + R + max_d + (users - 1) * rows1) * N * 8;
-  size_t chunk = std::min<size_t>(n, 64);
+  if (e == cudaSuccess && ps == PZ_OK)
+    e = cudaMemcpyAsync(d_rows, hr.data(), users * sizeof(pz::NiRowUser), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && ps == PZ_OK)
+    e = cudaMemcpyAsync(d_keys + users * key_bytes, hk.data(), users * sizeof(void *), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && ps == PZ_OK) e = cudaStreamSynchronize(st);  // the host arrays are read until here
+  // ---- RGSWs, in groups whose products (two leader RLWEs per index, one CTA
+  // per SM) fill the chip once: 620 indices of three users take 18 launches of
+  // 91 us; 22 of 24 indices each took 54 launches of 91 us.  The digits of a group
+  // are made in equal chunks of at most 1 GiB with their sums, so that the
+  // scratch stays within what the pool keeps.
+  const size_t sum_bytes = users * pz::ni_fft_sum_bytes();
+  const size_t per_index = R * ((size_t)d * N * 8 + sum_bytes) + ((size_t)R + max_d) * N * 8;
+  const size_t per_product = (users - 1) * rows1 * N * 8;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  size_t group = std::min<size_t>(n, std::max(1, sms / 2)), room = (size_t)1 << 30;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
-    chunk = std::max<size_t>(1, std::min(chunk, free_b / 2 / per_index));
-  u64 *d_arows = nullptr, *d_vals = nullptr, *d_dig = nullptr, *d_others = nullptr;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+    room = std::min(room, free_b / 4);
+    group = std::max<size_t>(1, std::min(group, free_b / 4 / std::max<size_t>(1, per_product)));
+  }
+  const size_t chunks = std::max<size_t>(1, std::min(group, (group * per_index + room) / (room + 1)));
+  const size_t chunk = (group + chunks - 1) / chunks;
+  u64 *d_arows = nullptr, *d_vals = nullptr, *d_others = nullptr;
+  unsigned char *d_dig = nullptr;
   if (e == cudaSuccess && ps == PZ_OK) e = pz::pool_malloc(&d_arows, chunk * max_d * N * 8, st);
   if (e == cudaSuccess && ps == PZ_OK) e = pz::pool_malloc(&d_vals, chunk * R * N * 8, st);
-  if (e == cudaSuccess && ps == PZ_OK) e = pz::pool_malloc(&d_dig, chunk * R * d * N * 8, st);
-  if (e == cudaSuccess && ps == PZ_OK && users > 1)
-    e = pz::pool_malloc(&d_others, (users - 1) * chunk * rows1 * N * 8, st);
+  if (e == cudaSuccess && ps == PZ_OK)
+    e = pz::pool_malloc(&d_dig, pz::ni_fft_digit_bytes((u32)d, chunk * R) + chunk * R * sum_bytes, st);
+  if (e == cudaSuccess && ps == PZ_OK && users > 1) e = pz::pool_malloc(&d_others, group * per_product, st);
   const pz::Decomp dp = pz::decomposer(P.rlwe_q, P.ni_ks_logb, (u32)d);
-  const size_t smem = 2 * N * 8;
   std::vector<uint8_t> seeds(chunk * 32);
-  for (size_t i0 = 0; i0 < n && e == cudaSuccess && ps == PZ_OK; i0 += chunk) {
-    const size_t cnt = std::min(chunk, n - i0);
-    for (size_t c0 = 0; c0 < cnt; c0++) pz_ni_crs_seed(crs, PZ_CRS_NI_RGSW, i0 + c0, &seeds[c0 * 32]);
-    ps = pz::seeded_fill_batch_u64(c, (const uint8_t(*)[32])seeds.data(), cnt, P.rlwe_q, (u64)max_d * N, d_arows,
-                                   (u64)max_d * N, st);
-    if (ps != PZ_OK) break;
-    ni_values_kernel<<<grid_cap(cnt * R * N / 256, 4736), 256, 0, st>>>(d_users, sh, d_arows, (u32)i0, (u32)cnt,
-                                                                       P.rlwe_q, d_vals);
-    if ((e = cudaGetLastError()) != cudaSuccess) break;
-    ni_digits_kernel<<<grid_cap(cnt * R, 65535), NI_T, smem, st>>>(c->rc, dp, (u32)d, d_vals, d_dig, cnt * R);
-    if ((e = cudaGetLastError()) != cudaSuccess) break;
-    u64 *lead = d_rgsw + i0 * 4 * N;
-    ni_agg_mac_kernel<<<grid_cap(cnt * R * users, 65535), NI_T, smem, st>>>(c->rc, sh, d_dig, d_users, (u32)i0,
-                                                                           (u32)cnt, lead, d_others);
-    if ((e = cudaGetLastError()) != cudaSuccess) break;
-    if (users > 1) ps = pz_aggregate_rgsw_device(c, lead, d_others, users - 1, cnt, st);
+  for (size_t g0 = 0; g0 < n && e == cudaSuccess && ps == PZ_OK; g0 += group) {
+    const size_t gcnt = std::min(group, n - g0);
+    for (size_t o0 = 0; o0 < gcnt && e == cudaSuccess; o0 += chunk) {
+      const size_t i0 = g0 + o0, cnt = std::min(chunk, gcnt - o0);
+      for (size_t c0 = 0; c0 < cnt; c0++) pz_ni_crs_seed(crs, PZ_CRS_NI_RGSW, i0 + c0, &seeds[c0 * 32]);
+      ps = pz::seeded_fill_batch_u64(c, (const uint8_t(*)[32])seeds.data(), cnt, P.rlwe_q, (u64)max_d * N, d_arows,
+                                     (u64)max_d * N, st);
+      if (ps != PZ_OK) break;
+      ni_values_kernel<<<grid_cap(cnt * R * N / 256, 4736), 256, 0, st>>>(d_users, sh, d_arows, (u32)i0, (u32)cnt,
+                                                                         P.rlwe_q, d_vals);
+      if ((e = cudaGetLastError()) != cudaSuccess) break;
+      const pz::NiRows rows{ra, rb, max_d, 1, (u32)((n + users - 1) / users), (u32)i0, (u32)gcnt, d_rows,
+                            d_rgsw + i0 * 4 * N, d_others ? d_others + o0 * rows1 * N : nullptr};
+      e = pz::launch_ni_fft_rows(d_vals, cnt * R, (u32)users, (u32)d, dp, rows,
+                                 (const void *const *)(d_keys + users * key_bytes), c->d_fft, d_dig,
+                                 d_dig + pz::ni_fft_digit_bytes((u32)d, chunk * R), c->d_err, st);
+    }
+    if (e == cudaSuccess && ps == PZ_OK && users > 1)
+      ps = pz_aggregate_rgsw_device(c, d_rgsw + g0 * 4 * N, d_others, users - 1, gcnt, st);
   }
   if (e == cudaSuccess && ps == PZ_OK) e = cudaStreamSynchronize(st);
   cudaFreeAsync(d_arows, st);
@@ -378,6 +292,7 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   cudaFreeAsync(d_stage, st);
   cudaFreeAsync((void *)d_src, st);
   cudaFreeAsync(d_users, st);
+  cudaFreeAsync(d_rows, st);
   cudaStreamSynchronize(st);
   if (ps != PZ_OK) return ps;
   if (e != cudaSuccess) return pz::cuda_fail(c, "pz_ni_aggregate_device", e);

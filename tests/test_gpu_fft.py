@@ -88,3 +88,55 @@ def test_forms_agree(gpu_available, param):
     finally:
         eng.set_split_threshold(-1)
         eng.set_pbs_grid_limit(0)
+
+
+@pytest.mark.parametrize("count", [1, 3, 9, 287, 288, 290, 513])
+def test_ni_key_switch_of_extreme_words(gpu_available, count):
+    """Keys with both 27-bit limbs at their largest and values with as many
+    non-zero digits as there can be, at counts around four rows to a warp and
+    around a launch's largest batch."""
+    O = oracle()
+    ev = O.Evaluator("NI_8P")
+    i, N, Q = ev.info, ev.N, ev.Q
+    g = np.random.default_rng(11)
+    low = -(1 << 26) - (((1 << 26) - 1) << 27)
+    high = ((1 << 26) - 1) * (1 + (1 << 27))
+    words = np.array([v % Q for v in (low, high, Q // 2, Q // 2 + 1, Q - 1, 1 << 26)], np.uint64)
+    ksk = words[g.integers(0, len(words), (2 * i.ni_ks_d, N))]
+    ksk[::3] = words[0]
+    dense = ((1 << 50) - 1) // 3 << 3
+    values = np.array([v % Q for v in (dense, -dense, dense << 1, Q // 2, Q // 2 + 1, 0, Q - 1)], np.uint64)
+    rows = values[g.integers(0, len(values), (7, 2, N))]
+    rows[0, 0] = values[0]
+    rows[1, 0] = np.where(np.arange(N) % 2, values[0], values[1])
+    want = np.stack([ev.ni_key_switch(ksk, r) for r in rows])
+    pick = np.arange(count) % len(rows)
+    eng = pz().Engine("NI_8P")
+    d_out = to_dev(np.zeros((count, 2, N), np.uint64))
+    eng.ni_key_switch_device(eng.upload_ni_ksk(ksk), to_dev(rows[pick]), d_out)
+    assert np.array_equal(to_host(d_out).reshape(count, -1), want.reshape(len(rows), -1)[pick])
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_sample_extract_rows_off_16_bytes(gpu_available, shift):
+    """Rows that start on and off a 16-byte boundary, runs that end in a launch's
+    last CTA, RLWEs that change within a run, and an index past the batch."""
+    eng = pz().Engine("NI_2P")
+    N, Q, count = eng.N, eng.Q, 45
+    g = np.random.default_rng(13)
+    rl = g.integers(0, Q, (3, 2, N), dtype=np.uint64)
+    idx = g.integers(0, 3 * N, count).astype(np.uint32)
+    idx[:6] = [0, N - 1, N, 2 * N - 1, 2 * N, 3 * N - 1]
+    idx[20] = 3 * N
+    out = to_dev(np.full(shift + count * (N + 1), 5, np.uint64))
+    eng.sample_extract_device(to_dev(rl), to_dev(idx), out[shift:])
+    got = to_host(out)
+    assert (got[:shift] == 5).all()
+    for row, k in zip(got[shift:].reshape(count, N + 1), idx):
+        if k >= 3 * N:
+            assert (row == 5).all()
+            continue
+        a, b = rl[k // N]
+        k = int(k) % N
+        want = np.concatenate([b[k:k + 1], a[k::-1], np.uint64(Q) - a[:k:-1]])
+        assert np.array_equal(row, want)
