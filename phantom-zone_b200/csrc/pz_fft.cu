@@ -109,14 +109,38 @@ __device__ __forceinline__ void op_sync() {
   tmem_after_barrier();
 }
 
+// SPLIT's digits wait in their own order, those of coefficients t + T m and t +
+// T (m + 1) for even m side by side, and an automorphism reads them permuted:
+// what goes to the other CTA goes by 8-byte stores to neighbouring places (one
+// gate 6.67 -> 6.01 ms against 4-byte stores to permuted ones; as bulk copies 6.16).
+__device__ __forceinline__ int pair_place(int e) {
+  const int m = e / T;
+  return m / 2 * 2 * T + 2 * (e % T) + (m & 1);
+}
+
 // The digits of one polynomial (half 0: a's, or their low halves under an
 // automorphism; half 1: b's, or the high halves of a's).
 template <Form F>
-__device__ __forceinline__ void load_digits(int (&v)[16], int half, u32 i, u32 q, bool is_auto, const Smem<F> &S,
+__device__ __forceinline__ void load_digits(int (&v)[16], int half, u32 i, u32 q, bool is_auto, u32 k, const Smem<F> &S,
                                             const Place &p) {
   const int *d = half == 0 || is_auto ? S.da(i) : S.db(i, q);
+  if (F != SPLIT) {
 #pragma unroll
-  for (int m = 0; m < 16; m++) v[m] = d[p.t + T * m];
+    for (int m = 0; m < 16; m++) v[m] = d[p.t + T * m];
+  } else if (is_auto) {
+    u32 inv = k * (2 - k * k);  // of k mod 2^6, then 2^12 = 2 N
+    inv *= 2 - k * inv;
+    u32 e = (u32)p.t * inv;
+#pragma unroll
+    for (int m = 0; m < 16; m++, e += T * inv) v[m] = d[pair_place(e & (N - 1))];
+  } else {
+#pragma unroll
+    for (int m = 0; m < 16; m += 2) {
+      const int2 x = ((const int2 *)d)[m / 2 * T + p.t];
+      v[m] = x.x;
+      v[m + 1] = x.y;
+    }
+  }
   if (is_auto) {
 #pragma unroll
     for (int m = 0; m < 16; m++) {
@@ -184,12 +208,19 @@ __device__ __forceinline__ void pass_on(const u64 (&acc)[C], int m0, int o, u32 
     const long long half = nx.is_auto ? 1ll << (AUTO_IGN - 1) : 1ll << (RLRG_IGN - 1);
     const int more = nx.is_auto ? 0 : RLRG_IGN - AUTO_IGN;
     int *dst = o ? S.db(i + 1, q) : S.da(i + 1);
-    const u32 far = F == SPLIT ? cluster_addr(dst, rank ^ 1) : 0;
+    auto digit_of = [&](long long v) { return (int)((v + half) >> AUTO_IGN) >> more; };
+    if constexpr (F == SPLIT) {
+      dst += 2 * (m0 / 2 * T + p.t);
+      const u32 far = cluster_addr(dst, rank ^ 1);
 #pragma unroll
-    for (int m = 0; m < C; m++, at += T * nx.k) {
-      const int d = (int)((c[m] + half) >> AUTO_IGN) >> more;
-      dst[at & (N - 1)] = d;
-      if (F == SPLIT) remote_store(far + 4 * (at & (N - 1)), d, far_bar);
+      for (int m = 0; m < C; m += 2) {
+        const int2 d = make_int2(digit_of(c[m]), digit_of(c[m + 1]));
+        remote_store2(far + 4 * m * T, d.x, d.y, far_bar);
+        *(int2 *)(dst + m * T) = d;
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < C; m++, at += T * nx.k) dst[at & (N - 1)] = digit_of(c[m]);
     }
   }
 }
@@ -209,9 +240,9 @@ __device__ __forceinline__ void op_quad(u32 i, u32 op, u32 nx_op, const cplx *ke
   cplx z[8];
   {
     int y[16];
-    load_digits(y, 0, i, q, is_auto, S, p);
+    load_digits(y, 0, i, q, is_auto, 1u, S, p);
     to_complex(z, y);
-    load_digits(y, 1, i, q, is_auto, S, p);
+    load_digits(y, 1, i, q, is_auto, 1u, S, p);
     if (is_auto) {  // b, before its buffer is written
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -333,12 +364,14 @@ struct Waits {
 };
 
 template <Form F, class Emit>
-__device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, const cplx *key, const cplx *next_key,
+__device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, Next &now, const cplx *key, const cplx *next_key,
                                         const BrParams &P, const Smem<F> &S, Waits &W, int rank, u32 &q, u32 tm,
                                         const Place &p, const Emit &emit) {
   typedef Shape<F> H;
   const int t = p.t, g = p.g;
   const bool is_auto = (op & OP_AUTO) != 0;
+  Next nx = now;
+  if (F == SPLIT) nx = Next(nx_op, P);
   // the next operation's key, into L2 while this one is worked on
   if (threadIdx.x == 0 && next_key) {
     if (F == SPLIT) prefetch_l2(next_key + (size_t)rank * LIMBS * 2 * M, LIMBS * 2 * M * (u32)sizeof(cplx));
@@ -347,7 +380,7 @@ __device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, const cplx *ke
   cplx z[8];
   if (g < 2) {
     int v[16];
-    load_digits(v, g, i, q, is_auto, S, p);
+    load_digits(v, g, i, q, is_auto, now.k, S, p);
     to_complex(z, v);
   }
   // this group's limb of the key for the first output
@@ -360,22 +393,41 @@ __device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, const cplx *ke
       ky[r] = ld_key(kp + (2 * r + 1) * T);
     }
   };
+  // SPLIT: half of the block into registers while the digits are transformed
+  // (the products would wait for all of it otherwise, 96 KB in 770 cycles: one
+  // gate 5.96 -> 5.78 ms together with the sums dealt out 6, 6 and 4)
+  constexpr int EARLY = 4;
+  const cplx *const sk = F == SPLIT ? S.key(g) + t : nullptr;
+  auto take = [&]() {
+    if constexpr (F == SPLIT) {
+      W.wait_key(g);
+#pragma unroll
+      for (int r = 0; r < EARLY; r++) {
+        kx[r] = sk[2 * r * T];
+        ky[r] = sk[(2 * r + 1) * T];
+      }
+    }
+  };
   if (F == TRIO) fetch();
   if (g < 2) {
-    forward<H::GROUPS>(z, S.buffer(g, q), S.tw(), p);
+    forward<H::GROUPS>(z, S.buffer(g, q), S.tw(), p, take);
     if (F == TRIO) q ^= 1;
 #pragma unroll
     for (int c = 0; c < 4; c++) tmem_store2(tm + H::SPEC + 16 * c + 8 * g, z[2 * c], z[2 * c + 1]);
+  } else {
+    take();
   }
   op_sync();
 #pragma unroll 1
   for (int o = F == SPLIT ? rank : 0; o < (F == SPLIT ? rank + 1 : 2); o++) {
     if constexpr (F == SPLIT) {
-      W.wait_key(g);
-      const cplx *sp = S.key(g) + t;
 #pragma unroll
-      for (int r = 0; r < 8; r += 2)
-        products(z, r, tm + H::SPEC, sp[2 * r * T], sp[(2 * r + 1) * T], sp[(2 * r + 2) * T], sp[(2 * r + 3) * T]);
+      for (int r = EARLY; r < 8; r++) {
+        kx[r] = sk[2 * r * T];
+        ky[r] = sk[(2 * r + 1) * T];
+      }
+#pragma unroll
+      for (int r = 0; r < 8; r += 2) products(z, r, tm + H::SPEC, kx[r], ky[r], kx[r + 1], ky[r + 1]);
     } else {
 #pragma unroll
       for (int r = 0; r < 8; r += 2) products(z, r, tm + H::SPEC, kx[r], ky[r], kx[r + 1], ky[r + 1]);
@@ -412,9 +464,9 @@ __device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, const cplx *ke
     }
   }
   op_sync();
-  // the sums, dealt out to the groups: SPLIT values 0-7, 8-11, 12-15 of the
-  // output, TRIO the 16 of a and then those of b, 12, 12 and 8
-  const Next nx(nx_op, P);
+  if (F == TRIO) nx = Next(nx_op, P);
+  // the sums, dealt out to the groups: SPLIT values 0-5, 6-11, 12-15 of the
+  // output (limb 2 takes its group longest), TRIO the 16 of a and then those of b, 12, 12 and 8
   const u32 far_bar = F == SPLIT ? cluster_addr(W.msg + ((i + 1) & 1), rank ^ 1) : 0;
   auto finish = [&](auto count, int o, int m0) {
     constexpr int C = decltype(count)::value;
@@ -427,13 +479,14 @@ __device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, const cplx *ke
     pass_on(acc, m0, o, i, q, nx, S, far_bar, rank, p, emit);
   };
   if (F == SPLIT) {
-    if (g == 0) finish(Int<8>(), rank, 0);
-    else finish(Int<4>(), rank, 4 + 4 * g);
+    if (g < 2) finish(Int<6>(), rank, 6 * g);
+    else finish(Int<4>(), rank, 12);
     if (rank == 1 && nx.is_auto && threadIdx.x == 0) remote_store(cluster_addr(S.db(i + 1, q), 0), 0, far_bar);
   } else {
 #pragma unroll 1
     for (int u = 3 * g; u < min(3 * g + 3, 8); u++) finish(Int<4>(), u >> 2, 4 * (u & 3));
   }
+  now = nx;
 }
 
 __device__ __forceinline__ const cplx *op_key(const BrParams &P, u32 op) {
@@ -495,7 +548,7 @@ __device__ __forceinline__ void fft_item(const BrParams &P, int ct, const u32 *k
     for (int m = 0; m < PER; m++) {
       const int c = threadIdx.x + H::THREADS * m;
       if (c < N) {
-        S.db(i, q)[c] = d[m];
+        S.db(i, q)[F == SPLIT ? pair_place(c) : c] = d[m];
         S.da(i)[c] = 0;
       }
     }
@@ -512,14 +565,17 @@ __device__ __forceinline__ void fft_item(const BrParams &P, int ct, const u32 *k
     cg::this_cluster().sync();  // the other CTA is ready for what it is sent, too
   }
   W.fresh = true;
+  u32 op = ops[i];
+  Next now(op, P);
 #pragma unroll 1
   for (; i < nops; i++) {
-    const u32 op = ops[i], nx = i + 1 < nops ? (u32)ops[i + 1] : OP_END;
-    const cplx *key = op_key(P, op), *next_key = nx != OP_END ? op_key(P, nx) : nullptr;
+    const u32 nx_op = i + 1 < nops ? (u32)ops[i + 1] : OP_END;
+    const cplx *key = op_key(P, op), *next_key = nx_op != OP_END ? op_key(P, nx_op) : nullptr;
     if constexpr (F == SPLIT) W.message(i, op);
     op_sync();
-    if constexpr (F == QUAD) op_quad(i, op, nx, key, next_key, P, S, q, tm, p, emit);
-    else op_trio(i, op, nx, key, next_key, P, S, W, rank, q, tm, p, emit);
+    if constexpr (F == QUAD) op_quad(i, op, nx_op, key, next_key, P, S, q, tm, p, emit);
+    else op_trio(i, op, nx_op, now, key, next_key, P, S, W, rank, q, tm, p, emit);
+    op = nx_op;
   }
 }
 
@@ -687,7 +743,7 @@ cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const
   return cudaGetLastError();
 }
 
-// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 6.6 up to 74 ciphertexts;
+// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 5.8 up to 74 ciphertexts;
 // TRIO 8.8 for 148, 17.4 for 296; QUAD 15.1, 18.6, 24.4 and 30.6 for 148, 296, 444
 // and 592, and from there by the number of ciphertexts (20.7 k/s).
 static fft::Form fft_form(size_t resident, bool split) {

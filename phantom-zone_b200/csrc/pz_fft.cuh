@@ -145,6 +145,12 @@ __device__ __forceinline__ void remote_store(u32 addr, int v, u32 bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
                : "memory");
 }
+// ... two of them (8-byte aligned)
+__device__ __forceinline__ void remote_store2(u32 addr, int a, int b, u32 bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(a),
+               "r"(b), "r"(bar)
+               : "memory");
+}
 // this CTA's shared address in CTA `rank` of the cluster
 __device__ __forceinline__ u32 cluster_addr(const void *p, u32 rank) {
   u32 a;
@@ -227,11 +233,25 @@ __device__ __forceinline__ void tmem_load8(u32 addr, u64 (&v)[8]) {
       : "memory");
 }
 
-// three groups of 2 C columns -> the sums of C 64-bit words
+// three groups of 2 C columns, 32 apart -> the sums of C 64-bit words
 template <int C>
 __device__ __forceinline__ void tmem_sum3(u32 addr, u64 (&v)[C]) {
-  static_assert(C == 4 || C == 8, "");
-  if constexpr (C == 4)
+  static_assert(C == 2 || C == 4 || C == 6, "");
+  if constexpr (C == 2)
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 r<12>;\n\t.reg .u64 a, b, c;\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r0, r1, r2, r3}, [%2];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r4, r5, r6, r7}, [%3];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {r8, r9, r10, r11}, [%4];\n\t"
+        "tcgen05.wait::ld.sync.aligned;\n\t"
+        "mov.b64 a, {r0, r1};\n\tmov.b64 b, {r4, r5};\n\tmov.b64 c, {r8, r9};\n\tadd.u64 a, a, b;\n\tadd.u64 %0, a, c;\n\t"
+        "mov.b64 a, {r2, r3};\n\tmov.b64 b, {r6, r7};\n\tmov.b64 c, {r10, r11};\n\tadd.u64 a, a, b;\n\tadd.u64 %1, a, c;\n\t"
+        "}"
+        : "=l"(v[0]), "=l"(v[1])
+        : "r"(addr), "r"(addr + 32), "r"(addr + 64)
+        : "memory");
+  else if constexpr (C == 4)
     asm volatile(
         "{\n\t"
         ".reg .b32 r<24>;\n\t.reg .u64 a, b, c;\n\t"
@@ -248,13 +268,13 @@ __device__ __forceinline__ void tmem_sum3(u32 addr, u64 (&v)[C]) {
         : "r"(addr), "r"(addr + 32), "r"(addr + 64)
         : "memory");
   else {
-    u64 w[4];
+    u64 w[4], x[2];
     tmem_sum3<4>(addr, w);
+    tmem_sum3<2>(addr + 8, x);
 #pragma unroll
     for (int m = 0; m < 4; m++) v[m] = w[m];
-    tmem_sum3<4>(addr + 8, w);
-#pragma unroll
-    for (int m = 0; m < 4; m++) v[4 + m] = w[m];
+    v[4] = x[0];
+    v[5] = x[1];
   }
 }
 
@@ -467,15 +487,21 @@ __device__ __forceinline__ void group_sync(const Place &p) {
 __device__ __forceinline__ int at_c(const Place &p, int r) { return (p.c ^ ((r & 1) << 2)) + 128 * r; }
 __device__ __forceinline__ int at_1(const Place &p, int r) { return p.b + 16 * r; }
 
-// Forward transform, layout C -> E, through buffer X.
-template <int GROUPS>
-__device__ __forceinline__ void forward(cplx (&x)[8], cplx *X, const cplx *tw, const Place &p) {
+struct Nothing {
+  __device__ __forceinline__ void operator()() const {}
+};
+// Forward transform, layout C -> E, through buffer X.  meanwhile(): loads from
+// shared memory that are to run under the levels after the exchange.
+template <int GROUPS, class Meanwhile = Nothing>
+__device__ __forceinline__ void forward(cplx (&x)[8], cplx *X, const cplx *tw, const Place &p,
+                                        const Meanwhile &meanwhile = Nothing()) {
   fwd8(x, PZ_FFT_C0);
 #pragma unroll
   for (int r = 0; r < 8; r++) X[at_c(p, r)] = x[r];
   group_sync<GROUPS>(p);
 #pragma unroll
   for (int r = 0; r < 8; r++) x[r] = X[at_1(p, r)];
+  meanwhile();
   const int w = p.t >> 5, l = p.t & 31;
   {
     const cplx *c = tw + TW_R1 + 2 * w + (l & 1);
