@@ -102,44 +102,70 @@ __device__ __forceinline__ void build_schedule(const BrParams &P, const u32 *kso
     }
     __syncthreads();
     // ---- the blind-rotation schedule (pbs.rs:240-414): buckets of -g^k for
-    // k = q/4-1..1, -g^0, +g^k, +g^0, each followed by an automorphism when
-    // the next bucket is non-empty, the window w is reached or k == 1; the
-    // automorphisms before the first external product act on a trivial RLWE.
-    if (j == 0) {
-      u32 no = 0;
-      bool trivial = true;
-      auto bucket = [&](u32 b) {
-        const u32 e = s_start[b + 1];
-        for (u32 t = s_start[b]; t < e; t++) s_ops[no++] = s_list[t];
-        if (e != s_start[b]) trivial = false;
-      };
-      auto autom = [&](u32 v) {
-        if (!trivial) s_ops[no - 1] |= (unsigned short)OP_KEEPB;  // b stays in the evaluation domain
-        s_ops[no++] = (unsigned short)(OP_AUTO | (trivial ? OP_TRIVIAL : 0u) | v);
-      };
-      u32 v = 0;
-      for (u32 i = q4 - 1; i >= 1; i--) {  // -(g^k)
-        bucket(q4 + i);
-        v++;
-        if (s_start[q4 + i] != s_start[q4 + i - 1] || v == P.w || i == 1) {
-          autom(v);
-          v = 0;
-        }
-      }
-      bucket(q4);  // -(g^0)
-      autom(0);
-      v = 0;
-      for (u32 i = q4 - 1; i >= 1; i--) {  // +(g^k)
-        bucket(i);
-        v++;
-        if (s_start[i] != s_start[i - 1] || v == P.w || i == 1) {
-          autom(v);
-          v = 0;
-        }
-      }
-      bucket(0);  // +(g^0)
-      *s_nops = no;
+    // k = q/4-1..1, -g^0, +g^k, +g^0 (R - 1 down to 0), each followed by an
+    // automorphism when the next bucket is non-empty, the window w is reached or
+    // k == 1; the automorphisms before the first external product act on a
+    // trivial RLWE.  Thread j takes buckets R - 1 - p, p0 <= p < p1: where the
+    // window starts and how many automorphisms come before are scans over the
+    // threads (one thread walking over all took 0.25 ms, 4 % of one gate).
+    int *part = (int *)scan;  // per warp: maxima, then (from 32) sums
+    const u32 per = (R + T - 1) / T;
+    const int p0 = (int)min(per * j, R), p1 = (int)min(per * (j + 1), R);
+    // an automorphism follows whatever the window (b == q4: -g^0, with slot 0)
+    auto forced = [&](u32 b) {
+      return b != 0 && (b == q4 || b == 1 || b == q4 + 1 || s_start[b - 1] != s_start[b]);
+    };
+    int last = -1;
+    for (int p = p0; p < p1; p++)
+      if (forced(R - 1 - p)) last = p;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, last, o);
+      if (lane >= o) last = max(last, y);
     }
+    if (lane == 31) part[warp] = last;
+    last = __shfl_up_sync(0xffffffffu, last, 1);
+    if (lane == 0) last = -1;
+    __syncthreads();
+    for (int w2 = 0; w2 < warp; w2++) last = max(last, part[w2]);
+    const u32 v0 = (u32)(p0 - last - 1) % P.w;
+    // every bucket of this thread: put(bucket, an automorphism follows, its slot)
+    auto walk = [&](auto put) {
+      u32 v = v0;
+      for (int p = p0; p < p1; p++) {
+        const u32 b = R - 1 - (u32)p;
+        v++;
+        const bool f = forced(b), follows = f || (b != 0 && v == P.w);
+        put(b, follows, b == q4 ? 0u : v);
+        if (follows) v = 0;
+      }
+    };
+    int mine = 0;
+    walk([&](u32, bool follows, u32) { mine += follows; });
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) part[32 + warp] = incl;
+    __syncthreads();
+    u32 before = (u32)(incl - mine);
+    for (int w2 = 0; w2 < warp; w2++) before += (u32)part[32 + w2];
+    walk([&](u32 b, bool follows, u32 slot) {
+      u32 no = n - s_start[b + 1] + before;
+      for (u32 t = s_start[b]; t < s_start[b + 1]; t++) s_ops[no++] = s_list[t];
+      if (follows) {
+        s_ops[no] = (unsigned short)(OP_AUTO | (s_start[b] == n ? OP_TRIVIAL : 0u) | slot);
+        before++;
+      }
+    });
+    if (p0 < p1 && p1 == (int)R) *s_nops = n + before;
+    __syncthreads();
+    // b stays in the evaluation domain before a non-trivial automorphism
+    const u32 nops = *s_nops;
+    for (u32 o = j; o + 1 < nops; o += T)
+      if ((s_ops[o + 1] & (OP_AUTO | OP_TRIVIAL)) == OP_AUTO) s_ops[o] |= (unsigned short)OP_KEEPB;
   }
 }
 

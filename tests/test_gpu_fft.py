@@ -140,3 +140,28 @@ def test_sample_extract_rows_off_16_bytes(gpu_available, shift):
         k = int(k) % N
         want = np.concatenate([b[k:k + 1], a[k::-1], np.uint64(Q) - a[:k:-1]])
         assert np.array_equal(row, want)
+
+
+@pytest.mark.parametrize("pattern", ["zero", "same", "two", "spread"])
+@pytest.mark.parametrize("param", ["I_2P_LB_SR", "NI_8P"])
+def test_schedules_of_few_buckets(gpu_available, param, pattern):
+    """Key switches whose LWEs put every index in one bucket (-g^0's or another),
+    in two, or a few in many: windows from end to end, and the automorphisms
+    before the first product."""
+    O = oracle()
+    ev = O.Evaluator(param)
+    i, N, Q = ev.info, ev.N, ev.Q
+    g = np.random.default_rng(17)
+    rgsw = g.integers(0, Q, (ev.n, i.rgsw_rows, N), dtype=np.uint64)
+    autos = g.integers(0, Q, (i.w + 1, i.auto_rows, N), dtype=np.uint64)
+    col = np.arange(ev.n + 1)
+    c = {"zero": 0 * col, "same": 1 + 0 * col, "two": np.where(col % 3 == 0, 1, i.lwe_q - 1), "spread": col}[pattern]
+    ksk = np.broadcast_to(c.astype(np.uint64), (i.lwe_d * N, ev.n + 1)).copy()
+    okey = O.OracleKey(ev, O.ServerKeyCoeff(rgsw, autos, ksk))
+    eng = pz().Engine(param)
+    key = eng.upload_key(rgsw, autos, ksk)
+    gates = np.array([1, 4], np.uint8)
+    c0, c1 = (g.integers(0, Q, (2, ev.L), dtype=np.uint64) for _ in range(2))
+    out = to_dev(np.zeros((2, ev.L), np.uint64))
+    eng.gate_batch_device(key, to_dev(gates), to_dev(c0), to_dev(c1), out)
+    assert np.array_equal(to_host(out), okey.gate_batch(gates, c0, c1, threads=2))
