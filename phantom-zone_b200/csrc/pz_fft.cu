@@ -592,14 +592,15 @@ __device__ __forceinline__ void tmem_end(u32 *slot) {
   if (threadIdx.x < 32) tmem_free<Shape<F>::COLS>(*slot);
 }
 
-// The batch (gates of one key; descs and item_desc null), or a ragged one:
-// ciphertext ct uses the parameter set and server key of descriptor
+// Ciphertexts [begin, end) of a batch (gates of one key; descs and item_desc
+// null), or of a ragged one: ciphertext ct uses the parameter set and server key of descriptor
 // item_desc[ct] and its output goes to out_idx[ct].  SPLIT: launched in
 // clusters of two, both on the same items.
 template <Form F>
 __global__ void __launch_bounds__(Shape<F>::THREADS, Shape<F>::CTAS)
     pbs_fft_kernel(const __grid_constant__ BrParams P, const BrParams *descs, const u32 *item_desc, const u32 *out_idx,
-                   const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out, int count, u64 *rlwe_dbg) {
+                   const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out, int begin, int end,
+                   u64 *rlwe_dbg) {
   extern __shared__ __align__(128) u64 smem[];
   __shared__ BrParams sp;
   __shared__ u32 tmem_slot;
@@ -613,8 +614,9 @@ __global__ void __launch_bounds__(Shape<F>::THREADS, Shape<F>::CTAS)
     mbar_init_fence();
   }
   Waits W{bars, bars + 3, &lost, nullptr, 0, 0, false, rank};
-  const int first = F == SPLIT ? blockIdx.x / 2 : blockIdx.x, step = F == SPLIT ? gridDim.x / 2 : gridDim.x;
-  for (int ct = first; ct < count; ct += step) {
+  const int step = F == SPLIT ? gridDim.x / 2 : gridDim.x;
+  const int first = begin + (int)(F == SPLIT ? blockIdx.x / 2 : blockIdx.x);
+  for (int ct = first; ct < end; ct += step) {
     __syncthreads();  // the previous item is done with sp
     if (threadIdx.x == 0) {
       sp = descs ? descs[item_desc[ct]] : P;
@@ -743,16 +745,6 @@ cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const
   return cudaGetLastError();
 }
 
-// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 5.8 up to 74 ciphertexts;
-// TRIO 8.8 for 148, 17.4 for 296; QUAD 15.1, 18.6, 24.4 and 30.6 for 148, 296, 444
-// and 592, and from there by the number of ciphertexts (20.7 k/s).
-static fft::Form fft_form(size_t resident, bool split) {
-  if (split) return fft::SPLIT;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return resident <= (size_t)sms ? fft::TRIO : fft::QUAD;
-}
-
 cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas) {
   typedef fft::Shape<fft::QUAD> H;
   const size_t smem = H::smem_bytes(br_q, n);
@@ -762,12 +754,19 @@ cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas) {
                                                                           H::THREADS, smem);
 }
 
+struct Batch {  // the arguments of pbs_fft_kernel
+  const BrParams &P;
+  const BrParams *descs;
+  const u32 *item_desc, *out_idx, *ks;
+  u32 ks_stride;
+  const unsigned char *gates;
+  u64 *out, *rlwe_dbg;
+  u32 br_q, n;  // the largest of the batch
+};
 template <fft::Form F>
-static cudaError_t launch_form(const BrParams &P, const BrParams *d_descs, const u32 *item_desc, const u32 *out_idx,
-                               u32 br_q, u32 n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
-                               size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s) {
+static cudaError_t launch_form(const Batch &b, size_t begin, size_t end, int grid, cudaStream_t s) {
   typedef fft::Shape<F> H;
-  const size_t smem = H::smem_bytes(br_q, n);
+  const size_t smem = H::smem_bytes(b.br_q, b.n);
   cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel<F>, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -780,31 +779,58 @@ static cudaError_t launch_form(const BrParams &P, const BrParams *d_descs, const
   attr[0].val.clusterDim = {2, 1, 1};
   cfg.attrs = attr;
   cfg.numAttrs = F == fft::SPLIT ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, fft::pbs_fft_kernel<F>, P, d_descs, item_desc, out_idx, ks, ks_stride, gates, out,
-                         (int)count, rlwe_dbg);
+  e = cudaLaunchKernelEx(&cfg, fft::pbs_fft_kernel<F>, b.P, b.descs, b.item_desc, b.out_idx, b.ks, b.ks_stride, b.gates,
+                         b.out, (int)begin, (int)end, b.rlwe_dbg);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
-static cudaError_t launch_fft(const BrParams &P, const BrParams *d_descs, const u32 *item_desc, const u32 *out_idx,
-                              u32 br_q, u32 n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
-                              size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split) {
-  switch (fft_form((size_t)grid, split)) {
-    case fft::SPLIT: return launch_form<fft::SPLIT>(P, d_descs, item_desc, out_idx, br_q, n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
-    case fft::TRIO: return launch_form<fft::TRIO>(P, d_descs, item_desc, out_idx, br_q, n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
-    default: return launch_form<fft::QUAD>(P, d_descs, item_desc, out_idx, br_q, n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s);
+static cudaError_t launch_form(fft::Form form, const Batch &b, size_t begin, size_t end, int grid, cudaStream_t s) {
+  switch (form) {
+    case fft::SPLIT: return launch_form<fft::SPLIT>(b, begin, end, grid, s);
+    case fft::TRIO: return launch_form<fft::TRIO>(b, begin, end, grid, s);
+    default: return launch_form<fft::QUAD>(b, begin, end, grid, s);
   }
+}
+
+// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 5.5 for up to 74
+// ciphertexts; TRIO 8.6 for up to 148 and again for each 148 more; QUAD 15.1,
+// 18.9, 24.2 and 30.3 for up to 148, 296, 444 and 592, and from there 28.3 per
+// 592, but 39.6 for 600 (the last few take as long as on an idle GPU).  So,
+// with as many CTAs as ciphertexts:
+//   up to 148     SPLIT (if asked for) or TRIO
+//   up to 222     148 in TRIO, the rest in SPLIT (180: 18.8 -> 14.1)
+//   up to 296     TRIO (18.9 -> 16.9)
+//   up to 370     296 in TRIO, the rest in SPLIT (300: 23.9 -> 22.5)
+//   more          QUAD; of more than 592, up to 74 or 148 above a multiple of 592
+//                 go by themselves, in SPLIT or TRIO (600: 39.6 -> 36.0)
+// With fewer CTAs (a limited grid) the form by their number.
+static cudaError_t launch_fft(const Batch &b, size_t count, int grid, bool split, cudaStream_t s) {
+  int dev = 0, sm = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+  const size_t sms = (size_t)sm, half = sms / 2;
+  if (split) return launch_form(fft::SPLIT, b, 0, count, grid, s);
+  if ((size_t)grid < count || count <= sms || b.rlwe_dbg)
+    return launch_form((size_t)grid <= sms ? fft::TRIO : fft::QUAD, b, 0, count, grid, s);
+  const fft::Form form = count <= 2 * sms + half ? fft::TRIO : fft::QUAD;
+  const size_t wave = form == fft::TRIO ? sms : 4 * sms, over = count % wave;
+  const bool peel = count > wave && over > 0 && over <= (form == fft::TRIO ? half : sms);
+  const size_t whole = peel ? count - over : count;
+  const cudaError_t e = launch_form(form, b, 0, whole, (int)whole, s);
+  if (e != cudaSuccess || !peel) return e;
+  return launch_form(over <= half ? fft::SPLIT : fft::TRIO, b, whole, count, (int)over, s);
 }
 
 cudaError_t launch_pbs_fft(const BrParams &P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
                            size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split) {
-  return launch_fft(P, nullptr, nullptr, nullptr, P.br_q, P.n, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s,
-                    split);
+  const Batch b{P, nullptr, nullptr, nullptr, ks, ks_stride, gates, out, rlwe_dbg, P.br_q, P.n};
+  return launch_fft(b, count, grid, split, s);
 }
 
 cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc, u32 max_br_q, u32 max_n, const u32 *ks,
                                   u32 ks_stride, const unsigned char *gates, u64 *out, const u32 *out_idx,
                                   size_t count, int grid, cudaStream_t s, bool split) {
-  return launch_fft(BrParams{}, d_descs, item_desc, out_idx, max_br_q, max_n, ks, ks_stride, gates, out, count, nullptr,
-                    grid, s, split);
+  const BrParams none{};
+  const Batch b{none, d_descs, item_desc, out_idx, ks, ks_stride, gates, out, nullptr, max_br_q, max_n};
+  return launch_fft(b, count, grid, split, s);
 }
 
 template <bool AUTO>

@@ -61,7 +61,7 @@ def test_forms_agree(gpu_available, param):
     eng = pz().Engine(param)
     key = eng.upload_key(coeff.rgsw, coeff.autos, coeff.ksk)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    most = 4 * sms + 3
+    most = 4 * sms + sms // 2 + 3
     r = oracle().Rng(b"\x5f" * 32)
     ks = r.uniform_mod(ev.info.lwe_q, most * (ev.n + 1)).reshape(most, -1).astype(np.uint32)
     gates = (np.arange(most) % 6).astype(np.uint8)
@@ -76,6 +76,8 @@ def test_forms_agree(gpu_available, param):
     try:
         full = run(most)
         for count, limit, split in [(1, 0, -1), (sms // 2, 0, -1), (sms // 2 + 1, 0, -1), (sms, 0, 0), (sms + 1, 0, -1),
+                                    (sms + sms // 2 + 1, 0, -1), (2 * sms + 1, 0, -1), (2 * sms + sms // 2 + 1, 0, -1),
+                                    (4 * sms, 0, -1), (4 * sms + 3, 0, -1), (2 * sms + 1, sms + 1, -1),
                                     (13, 5, 74), (13, 5, 0), (2, 0, 0)]:
             assert np.array_equal(run(count, limit, split), full[:count]), (count, limit, split)
         # one gate through the debug entry point: the rotated RLWE is the oracle's
