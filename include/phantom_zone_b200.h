@@ -188,9 +188,8 @@ pz_status pz_not_batch_device(pz_ctx *ctx, const uint64_t *d_in, uint64_t *d_out
                               void *stream);
 
 /* Kernel-level entry points (device memory, asynchronous).  The external
- * product and the automorphism of the one-digit parameter sets run with the
- * register cap of the context's blind-rotation variant (0 / 1 / 2: 2 / 3 / 4
- * CTAs per SM; others: 3). */
+ * product and the automorphism of the one-digit N = 2048 parameter sets run on
+ * the key's FFT form when the device had room for it at upload. */
 pz_status pz_ntt_forward_device(pz_ctx *ctx, uint64_t *d_polys, size_t count, void *stream);
 pz_status pz_ntt_backward_device(pz_ctx *ctx, uint64_t *d_polys, size_t count, void *stream);
 pz_status pz_rlwe_by_rgsw_device(pz_ctx *ctx, const pz_key *key, uint64_t *d_rlwe,
@@ -204,12 +203,14 @@ pz_status pz_lwe_key_switch_device(pz_ctx *ctx, const pz_key *key, const uint64_
 /* Blind-rotation launch shape: 0 = one CTA per ciphertext; > 0 caps the grid
  * (the kernel then strides over the batch). */
 pz_status pz_ctx_set_pbs_grid_limit(pz_ctx *ctx, int grid_limit);
-/* Blind-rotation kernel variant for N = 2048: registers capped for 2, 3 or 4
- * resident CTAs per SM (variant 0, 1, 2; default 0), or 3: each ciphertext on a
- * cluster of two CTAs (a and b on different SMs: lower latency per gate). */
+/* Blind-rotation launch shape for N = 2048: 0 (the default), 1, 2 and 4 are
+ * names of one shape, which places a batch by its size (four ciphertexts per SM,
+ * one, or one on two SMs); 3: every ciphertext on a cluster of two CTAs (a and b
+ * on different SMs: lower latency per gate). */
 pz_status pz_ctx_set_pbs_variant(pz_ctx *ctx, int variant);
 /* Launches of at most max_gates gates use variant 3 whatever the variant set
- * (-1, the default: half the GPU's SMs; 0: only if variant 3 is set). */
+ * (-1, the default: half the GPU's SMs; 0: only if variant 3 is set, or for the
+ * few ciphertexts above whole rounds of a larger batch). */
 pz_status pz_ctx_set_split_threshold(pz_ctx *ctx, int max_gates);
 int pz_ctx_pbs_variant(const pz_ctx *ctx);
 /* Ciphertexts a blind-rotation launch of shape `variant` (-1: the context's
@@ -221,7 +222,7 @@ pz_status pz_ctx_pbs_slots(pz_ctx *ctx, int variant, size_t *slots);
  * their code; a profile applies to the revision it was taken on).  No
  * reference counterpart. */
 const char *pz_kernel_revision(void);
-/* Autotuner: times every blind-rotation variant on synthetic key-switched
+/* Autotuner: times the blind-rotation variants 0 and 3 on synthetic key-switched
  * LWEs with this key -- `batch` of them, or, from one wave up, the largest
  * whole number of that variant's waves not above `batch` -- and keeps the
  * fastest per ciphertext (*ms: its time for `batch`); then times the
@@ -528,8 +529,7 @@ pz_status pz_server_stats_get(pz_server *s, pz_server_stats *out);
  * 1, 2 or 4 -- steps of at most half the SMs' gates take the two-CTA shape 3
  * by themselves; grid limit 0 = one CTA per gate) */
 pz_status pz_server_set_launch(pz_server *s, int pbs_variant, int grid_limit);
-/* Autotuner: times the variants 0, 1, 2, 4 x {one CTA per gate, persistent
- * 2 x SMs} on `batch` synthetic gates spread over the sessions with a
+/* Autotuner: times variant 0 x {one CTA per gate, persistent 4 x SMs} on `batch` synthetic gates spread over the sessions with a
  * resident key and keeps the fastest.  Needs an idle server (no admitted
  * job). */
 pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid_limit, double *ms);

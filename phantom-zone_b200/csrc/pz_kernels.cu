@@ -6,12 +6,15 @@
 //                 (ntt.rs:409-441), the kernel microbench
 //   ext_product   batched RLWE x RGSW (runtime.rs:754-855)
 //   rlwe_auto     batched RLWE automorphism (runtime.rs:530-643)
+//                 (both by integer transforms: N = 512, several digits, RGSW x
+//                 RGSW, and keys without their FFT form; else pz_fft.cu)
 //   ks            gate prelude (evaluator.rs:2118-2133) + mod-down Q -> q_ks
 //                 (pbs.rs:128-132) + LWE key switch (lwe.rs:14-44), batched
 //   pbs           one CTA per ciphertext: odd mod-switch, dlog buckets, the
 //                 blind-rotation schedule, test vector rotation, the whole
 //                 blind rotation with the RLWE accumulator in registers,
-//                 sample extraction (pbs.rs:146-449)
+//                 sample extraction (pbs.rs:146-449), by integer transforms:
+//                 N = 512 and keys without their FFT form (else pz_fft.cu)
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -472,8 +475,7 @@ __device__ __forceinline__ void bootstrap_op(u64 (&acc)[2][8], u32 op, const BrP
   }
 }
 
-// One-digit (D1) forms come register-capped for MINB = 2, 3 or 4 CTAs per SM,
-// picked like the blind rotation's launch shapes (the context's variant).
+// MINB: CTAs per SM that the register allocation allows.
 template <int LOGN, bool D1, int MINB>
 __global__ void __launch_bounds__(NttShape<LOGN>::T, MINB)
     ext_product_kernel(BrParams P, u64 *rlwe, const u32 *idx, size_t count, int trivial) {
@@ -860,8 +862,6 @@ size_t pbs_smem_bytes(int logn, u32 br_q, u32 n) {
   return OP_REGIONS * N * 8 + extra;
 }
 
-// MINB: CTAs per SM the register allocation must allow (launch-shape
-// variants chosen at run time, see pz_ctx_set_pbs_variant).
 // One gate bootstrap of ciphertext ct (key-switched LWE kso, gate code
 // gcode) with the parameters and key of P; the whole CTA takes part.
 template <int LOGN, bool D1>
@@ -1230,7 +1230,7 @@ cudaError_t launch_pbs(int logn, bool d1, const BrParams &P, const u32 *ks, u32 
   int grid = (int)count;
   if (grid_limit > 0 && grid > grid_limit) grid = grid_limit;
   cudaError_t e;
-  if (logn == 11 && d1 && P.fft_rgsw) 
+  if (logn == 11 && d1 && P.fft_rgsw)
     return launch_pbs_fft(P, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s,
                           variant == PBS_SPLIT && rlwe_dbg == nullptr);
 #define PZ_LAUNCH(LN, DD, MB, TH)                                                                    \

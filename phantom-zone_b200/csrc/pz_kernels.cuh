@@ -7,7 +7,7 @@ namespace pz {
 constexpr int MAX_KS_D = 16;   // key-switch decomposition count bound
 // Revision of the blind-rotation kernels: bumped with every change to their
 // code, so that a profile taken on one revision is not reported for another.
-constexpr const char *BR_KERNEL_REVISION = "br-v16";
+constexpr const char *BR_KERNEL_REVISION = "br-v17";
 constexpr int MAX_AUTO_SLOTS = 16;
 
 // Everything the blind rotation needs for one parameter set + server key.
@@ -98,9 +98,9 @@ cudaError_t launch_pbs(int logn, bool d1, const BrParams &P, const u32 *ks, u32 
                        const unsigned char *gates, u64 *out, size_t count, u64 *rlwe_dbg,
                        int grid_limit, cudaStream_t s, int variant);
 // Launch shapes of the N = 2048 one-digit sets.  0, 1, 2 and 4: one CTA per
-// ciphertext (these were register caps and key staging of an integer kernel;
-// they stay as names of the one shape that is left).  3: one ciphertext per
-// cluster of two CTAs (lower latency, for small batches).
+// ciphertext, or by batch size on part of an SM, on one or on two (names of one
+// shape, kept for callers that set them).  3: every ciphertext on a cluster of two
+// CTAs (lower latency, for small batches).
 constexpr int PBS_SPLIT = 3, PBS_MAX_VARIANT = 4;
 // Ragged batches (several sessions / parameter sets in one launch): per-item
 // descriptors in device memory; max_* bound the sizes over the descriptors.
