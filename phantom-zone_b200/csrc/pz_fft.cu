@@ -46,8 +46,8 @@ __global__ void __launch_bounds__(256)
 //          transform both digit polynomials, and the new digits go to both.
 //          For batches that leave SMs idle.
 // Shared memory: exchange buffers (M complex words; two per group, one in SPLIT) | what passes from an operation to the next: b or its digits
-// (N words), a's digits (N ints) | TRIO and SPLIT: the groups' next blocks of
-// the key | twiddles | the schedule.  In TRIO and SPLIT the second part is
+// (N words), a's digits (N ints) | SPLIT: the groups' next blocks of the
+// key | twiddles | the schedule.  In TRIO and SPLIT the second part is
 // there twice: an operation reads one and writes the other, while other threads
 // may still be reading.  QUAD has no room for it: b (or its digits) sits in the
 // exchange buffer that the last transform did not use, and is read before the

@@ -238,9 +238,9 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   if (e == cudaSuccess && ps == PZ_OK) e = cudaStreamSynchronize(st);  // the host arrays are read until here
   // ---- RGSWs, in groups whose products (two leader RLWEs per index, one CTA
   // per SM) fill the chip once: 620 indices of three users take 18 launches of
-  // 91 us; 22 of 24 indices each took 54 launches of 91 us.  The digits of a group
-  // are made in equal chunks of at most 1 GiB with their sums, so that the
-  // scratch stays within what the pool keeps.
+  // 91 us (in groups of 24 indices 54 launches of 91 us).  The digits of a group
+  // are made in equal chunks of at most 1 GiB with their sums, so that the scratch
+  // stays within what the pool keeps.
   const size_t sum_bytes = users * pz::ni_fft_sum_bytes();
   const size_t per_index = R * ((size_t)d * N * 8 + sum_bytes) + ((size_t)R + max_d) * N * 8;
   const size_t per_product = (users - 1) * rows1 * N * 8;
