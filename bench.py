@@ -440,7 +440,7 @@ def microbench(P, torch, device, count=4096, reps=5):
     idx = torch.arange(count, dtype=torch.int32, device="cuda") % p.lwe_n
     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     ep_by_shape = {}
-    for v in (0, 1, 2):  # register caps of 2 / 3 / 4 CTAs per SM
+    for v in (0, 1, 2):  # names of one launch shape: three runs of it
         eng.pbs_variant = v
         eng.rlwe_by_rgsw_device(key, rl, idx)
         torch.cuda.synchronize()
@@ -1157,15 +1157,15 @@ def main():
                     "h2d_bytes_per_step": int(info["inputs"] * L * 8),
                     "d2h_bytes_per_step": int(info["outputs"] * L * 8)},
             "gpu_launches": launches_per_step * args.steps,
-            "roofline": {"bound": "int", "kernel": "pbs_kernel (blind rotation)", "achieved": achieved,
+            "roofline": {"bound": "int", "kernel": "pbs_fft_kernel (blind rotation)", "achieved": achieved,
                          "peak": peak, "unit": "TIMAD/s", "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": traffic_source,
                          "peak_source": "pz_probe_imad_rate on this GPU (MEASURED_PEAKS.json has no integer peak)",
                          "launch_ms": br_ms, "bootstraps_per_launch": B,
                          "modmuls_per_bootstrap": modmuls / B,
                          "pipe_rates_tips": pipes,
-                         "convention": "10 IMAD per 64-bit modmul; the butterflies' quotient runs on the FP64 "
-                                       "pipe and the conversion unit, so part of the work is off the IMAD pipe"},
+                         "convention": "10 IMAD per 64-bit modmul of integer transforms; the products run as FP64 "
+                                       "FFTs, so none of this work is on the IMAD pipe"},
             "plain": plain,
             "parity": parity,
             **extras,
