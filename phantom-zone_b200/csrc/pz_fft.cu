@@ -398,10 +398,11 @@ __device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, Next &now, con
       ky[r] = ld_key(kp + (2 * r + 1) * T);
     }
   };
-  // SPLIT: half of the block into registers while the digits are transformed
-  // (the products would wait for all of it otherwise, 96 KB in 770 cycles: one
-  // gate 5.96 -> 5.78 ms together with the sums dealt out 6, 6 and 4)
-  constexpr int EARLY = 4;
+  // SPLIT: some of the block's points into registers while the digits are
+  // transformed (the products would wait for all of it otherwise, 96 KB in 770
+  // cycles: one gate 5.96 -> 5.78 ms together with the sums dealt out 6, 6 and 4;
+  // of 2 to 5 points 3 are the fastest, 5.62 ms against 5.65 to 5.67)
+  constexpr int EARLY = 3;
   const cplx *const sk = F == SPLIT ? S.key(g) + t : nullptr;
   auto take = [&]() {
     if constexpr (F == SPLIT) {
