@@ -121,6 +121,11 @@ const char *pz_last_error(const pz_ctx *ctx);
  * returns the bits in *bits and clears them.  No reference counterpart (the
  * reference panics on the CPU). */
 pz_status pz_ctx_device_error(pz_ctx *ctx, uint32_t *bits);
+/* Longest wait of a two-CTA blind rotation of this context for a key's copy or
+ * the other CTA, in SM clock cycles (-1, the default: 2^31, about a second; 0:
+ * every wait gives up at once, which is how the error path is tested).  A server
+ * takes the value that the context has when a session is added. */
+pz_status pz_ctx_set_wait_limit(pz_ctx *ctx, int64_t cycles);
 pz_status pz_ctx_params(const pz_ctx *ctx, pz_params *out);
 uint64_t pz_ctx_ntt_root(const pz_ctx *ctx);
 

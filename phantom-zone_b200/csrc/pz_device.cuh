@@ -884,12 +884,12 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, u32 bytes,
                : "memory");
 }
 // Wait for the phase of *bar with the given parity to complete, for at most
-// about `limit` SM clock cycles; false when the limit ran out.
+// about `limit` SM clock cycles; false when the limit ran out (0: at once).
 constexpr long long MBAR_WAIT_LIMIT = 1ll << 31;  // ~1.1 s at 1965 MHz
 __device__ __forceinline__ bool mbar_wait(u64 *bar, u32 parity, long long limit = MBAR_WAIT_LIMIT) {
   const u32 a = smem_addr(bar);
   const long long t0 = clock64();
-  for (;;) {
+  while (limit > 0) {
     u32 done;
     asm volatile(
         "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
@@ -897,8 +897,9 @@ __device__ __forceinline__ bool mbar_wait(u64 *bar, u32 parity, long long limit 
         : "r"(a), "r"(parity)
         : "memory");
     if (done) return true;
-    if (clock64() - t0 > limit) return false;
+    if (clock64() - t0 > limit) break;
   }
+  return false;
 }
 // One thread: ask L2 to fetch `bytes` (a multiple of 16, 16-byte aligned)
 // from global memory ahead of their use; no completion to wait for.  Used for

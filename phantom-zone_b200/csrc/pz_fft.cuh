@@ -161,7 +161,7 @@ __device__ __forceinline__ u32 cluster_addr(const void *p, u32 rank) {
 __device__ __forceinline__ bool mbar_wait_cluster(u64 *bar, u32 parity, long long limit = MBAR_WAIT_LIMIT) {
   const u32 a = smem_addr(bar);
   const long long t0 = clock64();
-  for (;;) {
+  while (limit > 0) {
     u32 done;
     asm volatile(
         "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
@@ -169,8 +169,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(u64 *bar, u32 parity, long lon
         : "r"(a), "r"(parity)
         : "memory");
     if (done) return true;
-    if (clock64() - t0 > limit) return false;
+    if (clock64() - t0 > limit) break;
   }
+  return false;
 }
 __device__ __forceinline__ void mbar_expect(u64 *bar, u32 bytes) {  // one arrival
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");

@@ -7,7 +7,7 @@ namespace pz {
 constexpr int MAX_KS_D = 16;   // key-switch decomposition count bound
 // Revision of the blind-rotation kernels: bumped with every change to their
 // code, so that a profile taken on one revision is not reported for another.
-constexpr const char *BR_KERNEL_REVISION = "br-v17";
+constexpr const char *BR_KERNEL_REVISION = "br-v18";
 constexpr int MAX_AUTO_SLOTS = 16;
 
 // Everything the blind rotation needs for one parameter set + server key.
@@ -26,6 +26,7 @@ struct BrParams {
   const u64 *autos;                // [w+1][auto_rows][N]
   const u32 *out_idx;              // optional scatter: output of gate ct -> LWE out_idx[ct]
   u32 *err;                        // the context's device error word (DEVERR_* bits)
+  long long wait_limit;            // of a wait for a copy or another CTA, in clock cycles; 0: gives up at once
   // FFT form of the same keys (N = 2048 one-digit sets; null: not built) and its twiddle tables
   const void *fft_rgsw, *fft_autos, *fft_tw;
 };

@@ -482,6 +482,7 @@ pz_status pz_ctx_create_ex(int id, int device, uint64_t root, pz_ctx **out) {
   pz::BrParams &br = c->br;
   br.rc = rc;
   br.err = c->d_err;
+  br.wait_limit = pz::MBAR_WAIT_LIMIT;
   br.da = make_decomp(Q, P.rlrg_logb, P.rlrg_d_a);
   br.db = make_decomp(Q, P.rlrg_logb, P.rlrg_d_b);
   br.dauto = make_decomp(Q, P.auto_logb, P.auto_d);
@@ -537,6 +538,12 @@ pz_status pz_ctx_device_error(pz_ctx *c, uint32_t *bits) {
   PZ_CK(c, cudaMemcpy(&v, c->d_err, sizeof v, cudaMemcpyDeviceToHost));
   if (v) PZ_CK(c, cudaMemset(c->d_err, 0, sizeof v));
   *bits = v;
+  return PZ_OK;
+}
+
+pz_status pz_ctx_set_wait_limit(pz_ctx *c, int64_t cycles) {
+  if (!c || cycles < -1) return PZ_ERR_INVALID_ARGUMENT;
+  c->br.wait_limit = cycles < 0 ? pz::MBAR_WAIT_LIMIT : cycles;
   return PZ_OK;
 }
 

@@ -207,6 +207,11 @@ class Engine:
         check(lib().pz_ctx_device_error(self.h, ctypes.byref(v)), self.h, "pz_ctx_device_error")
         return v.value
 
+    def set_wait_limit(self, cycles=-1):
+        """Longest wait of a two-CTA blind rotation, in SM clock cycles (-1: the
+        default, about a second; 0: every wait gives up at once)."""
+        check(lib().pz_ctx_set_wait_limit(self.h, int(cycles)), self.h, "pz_ctx_set_wait_limit")
+
     def pbs_slots(self, variant=-1):
         """Ciphertexts a blind-rotation launch of shape `variant` (-1: the
         current one) holds resident at once; multiples run in whole waves."""

@@ -167,3 +167,36 @@ def test_schedules_of_few_buckets(gpu_available, param, pattern):
     out = to_dev(np.zeros((2, ev.L), np.uint64))
     eng.gate_batch_device(key, to_dev(gates), to_dev(c0), to_dev(c1), out)
     assert np.array_equal(to_host(out), okey.gate_batch(gates, c0, c1, threads=2))
+
+
+@pytest.mark.parametrize("count, limit", [(1, 0), (3, 0), (7, 2)])
+def test_waits_that_run_out_end_the_kernel(gpu_available, count, limit):
+    """Two-CTA blind rotations whose waits all give up (one ciphertext per
+    cluster, and several in turn): the kernel ends and says so in the error word,
+    no copy or message of it disturbs what runs next, and with the usual limit
+    the same call gives the one-CTA words."""
+    eng = pz().Engine("I_2P_LB_SR")
+    p = eng.p
+    g = np.random.default_rng(23)
+    key = eng.upload_key(g.integers(0, eng.Q, (p.lwe_n, p.rgsw_rows, eng.N), dtype=np.uint64),
+                         g.integers(0, eng.Q, (p.n_auto_keys, p.auto_rows, eng.N), dtype=np.uint64),
+                         g.integers(0, p.lwe_q, (p.lwe_d * eng.N, p.lwe_n + 1), dtype=np.uint64))
+    c0, c1 = (to_dev(g.integers(0, eng.Q, (count, eng.L), dtype=np.uint64)) for _ in range(2))
+    gates = to_dev((np.arange(count) % 6).astype(np.uint8))
+
+    def run():
+        out = to_dev(np.zeros((count, eng.L), np.uint64))
+        eng.gate_batch_device(key, gates, c0, c1, out)
+        return to_host(out)
+
+    eng.set_split_threshold(0)
+    want = run()
+    eng.set_split_threshold(-1)
+    eng.set_pbs_grid_limit(limit)
+    for _ in range(2):
+        eng.set_wait_limit(0)
+        run()
+        assert eng.device_error() == 1
+        eng.set_wait_limit(-1)
+        assert np.array_equal(run(), want)
+        assert eng.device_error() == 0
