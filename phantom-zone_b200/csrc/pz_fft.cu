@@ -593,7 +593,7 @@ __device__ __forceinline__ void fft_item(const BrParams &P, int ct, const u32 *k
   u32 op = ops[i];
   Next now(op, P);
 #pragma unroll 1
-  for (; op != OP_END; i++) {
+  for (; F == SPLIT ? op != OP_END : i < nops; i++) {  // (TRIO by the first: 8.55 -> 8.60 ms)
     const u32 nx_op = i + 1 < nops ? ops[i + 1] : OP_END;
     const cplx *key = op_key(P, op), *next_key = nx_op != OP_END ? op_key(P, nx_op) : nullptr;
     if constexpr (F == SPLIT) W.message(i, op, S);
