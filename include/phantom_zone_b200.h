@@ -116,10 +116,13 @@ pz_status pz_ctx_create_ex(int param_id, int device, uint64_t ntt_root, pz_ctx *
 void pz_ctx_destroy(pz_ctx *ctx);
 const char *pz_last_error(const pz_ctx *ctx);
 /* Error bits kernels of this context set on the device instead of trapping
- * (bit 0: a bounded wait for a bulk copy into shared memory ran out; the
- * kernel returned and its outputs are not valid).  Synchronizes the device,
- * returns the bits in *bits and clears them.  No reference counterpart (the
- * reference panics on the CPU). */
+ * (bit 0: a bounded wait for a bulk copy into shared memory or for the other CTA
+ * ran out; the kernel returned and its outputs are not valid).  Synchronizes the
+ * device, returns the bits in *bits and clears them.  Entry points that wait for
+ * their own work (pz_gate_batch, pz_circuit_run, pz_ni_ingest,
+ * pz_ni_aggregate_*) return PZ_ERR_CUDA while bits are set, whichever call set
+ * them; asynchronous ones (*_device, graph replays) leave it to the caller to
+ * ask.  No reference counterpart (the reference panics on the CPU). */
 pz_status pz_ctx_device_error(pz_ctx *ctx, uint32_t *bits);
 /* Longest wait of a two-CTA blind rotation of this context for a key's copy or
  * the other CTA, in SM clock cycles (-1, the default: 2^31, about a second; 0:
@@ -523,7 +526,9 @@ pz_status pz_server_session_resident(pz_server *s, uint32_t session, int *reside
 pz_status pz_server_submit(pz_server *s, uint32_t session, pz_circuit *c, const uint64_t *inputs,
                            uint64_t *outputs, int device_io, uint64_t *job);
 /* One scheduling step (admit, one level of every admitted job, retire);
- * returns when its device work is complete.  *gates: bootstraps run. */
+ * returns when its device work is complete.  *gates: bootstraps run.  If a
+ * kernel of the step gave up a wait (see pz_ctx_device_error), the jobs that the
+ * step advanced fail (state 3) and it returns PZ_ERR_CUDA; later steps run. */
 pz_status pz_server_step(pz_server *s, size_t *gates);
 /* state: 0 pending, 1 running, 2 done, 3 failed (needs more than the whole
  * arena); latency = done - submit, queue = admit - submit (ms, -1 if n/a) */

@@ -617,8 +617,8 @@ pz_status pz_circuit_run(pz_ctx *ctx, const pz_key *k, pz_circuit *c, const uint
             ? PZ_OK
             : pz::fail(ctx, PZ_ERR_CUDA, "output copy failed");
   cudaFreeAsync(d_o, ctx->stream);
-  PZ_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return s;
+  const pz_status done = pz::finish(ctx, ctx->stream);
+  return s == PZ_OK ? done : s;
 }
 
 // Capture the whole circuit (input copy, every level, output gather) as one

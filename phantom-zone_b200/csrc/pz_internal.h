@@ -112,6 +112,12 @@ pz_status fail(pz_ctx *ctx, pz_status s, const std::string &msg);
 // forget the no-alloc scratch address cached for a device (pz_noalloc.cu)
 void noalloc_forget_device(int device);
 pz_status cuda_fail(pz_ctx *ctx, const char *what, cudaError_t e);
+// For entry points that wait for their own work on s: waits for it, and reports
+// the context's device error word.
+pz_status finish(pz_ctx *c, cudaStream_t s);
+// a device error word, once what is on s is done (one 4-byte copy to pageable
+// memory, which waits; a pinned word took 1.5 ms to allocate)
+cudaError_t read_error_word(const u32 *d_err, u32 *bits, cudaStream_t s);
 u32 ks_stride(const pz_params &P);
 // DefaultDecomposer parameters for (q, logb, d) (decomposer.rs:158-178)
 Decomp decomposer(u64 q, u32 logb, u32 d);

@@ -449,10 +449,10 @@ pz_status pz_ni_ingest(pz_ctx *c, const pz_ni_ksk *k, const uint8_t seed[32], co
   cudaFreeAsync(d_k, st);
   cudaFreeAsync(d_l, st);
   cudaFreeAsync(d_i, st);
-  cudaStreamSynchronize(st);
+  const pz_status done = pz::finish(c, st);
   if (s != PZ_OK) return s;
   if (e != cudaSuccess) return pz::cuda_fail(c, "pz_ni_ingest", e);
-  return PZ_OK;
+  return done;
 }
 
 }  // extern "C"

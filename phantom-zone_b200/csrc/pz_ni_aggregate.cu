@@ -293,10 +293,10 @@ pz_status pz_ni_aggregate_device(pz_ctx *c, const uint8_t crs[32], const pz_ni_s
   cudaFreeAsync((void *)d_src, st);
   cudaFreeAsync(d_users, st);
   cudaFreeAsync(d_rows, st);
-  cudaStreamSynchronize(st);
+  const pz_status done = pz::finish(c, st);
   if (ps != PZ_OK) return ps;
   if (e != cudaSuccess) return pz::cuda_fail(c, "pz_ni_aggregate_device", e);
-  return PZ_OK;
+  return done;
 }
 
 pz_status pz_ni_aggregate_server_key(pz_ctx *c, const uint8_t crs[32], const pz_ni_server_key_share_view *shares,

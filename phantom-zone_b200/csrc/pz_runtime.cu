@@ -173,6 +173,19 @@ pz_status fail(pz_ctx *ctx, pz_status s, const std::string &msg) {
   if (ctx) ctx->err = msg;
   return s;
 }
+cudaError_t read_error_word(const u32 *d_err, u32 *bits, cudaStream_t s) {
+  const cudaError_t e = cudaMemcpyAsync(bits, d_err, sizeof(u32), cudaMemcpyDeviceToHost, s);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+}
+pz_status finish(pz_ctx *c, cudaStream_t s) {
+  u32 bits = 0;
+  const cudaError_t e = read_error_word(c->d_err, &bits, s);
+  if (e != cudaSuccess) return cuda_fail(c, "waiting for the device", e);
+  if (!bits) return PZ_OK;
+  return fail(c, PZ_ERR_CUDA, "a kernel gave up a wait (device error bits " + std::to_string(bits) +
+                                  "): outputs are not valid; pz_ctx_device_error clears the bits");
+}
+
 pz_status cuda_fail(pz_ctx *ctx, const char *what, cudaError_t e) {
   pz_status s = (e == cudaErrorMemoryAllocation) ? PZ_ERR_OUT_OF_MEMORY : PZ_ERR_CUDA;
   return fail(ctx, s, std::string(what) + ": " + cudaGetErrorString(e));
@@ -731,8 +744,7 @@ pz_status pz_gate_batch(pz_ctx *c, const pz_key *k, const uint8_t *gates, const 
                      false)) != PZ_OK)
     return s;
   PZ_CK(c, cudaMemcpyAsync(out, c->d_out, bytes, cudaMemcpyDeviceToHost, c->stream));
-  PZ_CK(c, cudaStreamSynchronize(c->stream));
-  return PZ_OK;
+  return pz::finish(c, c->stream);
 }
 
 static pz_status gate_device_common(pz_ctx *c, const pz_key *k, const uint8_t *d_gates, const uint64_t *d_c0,

@@ -78,6 +78,7 @@ struct pz_server {
   size_t L = 0;
   u64 q = 0;
   u32 max_n = 0, max_br_q = 0, max_d = 0, ks_stride = 0;
+  u32 *d_err = nullptr;  // device error word of the server's launches
   pz::BrParams *d_br = nullptr;
   pz::KsParams *d_ksp = nullptr;
 
@@ -206,6 +207,7 @@ struct pz_server {
       cudaFree(d_outref);
       cudaFree(d_br);
       cudaFree(d_ksp);
+      cudaFree(d_err);
       if (stream) cudaStreamDestroy(stream);
     }
   }
@@ -231,6 +233,7 @@ pz_status upload_descs(pz_server *s) {
     br[i] = se.ctx->br;  // a session without a resident key gets no items: null key pointers
     pz::br_bind_key(se.ctx, se.key, br[i]);
     br[i].out_idx = nullptr;
+    br[i].err = s->d_err;
     ks[i] = se.ctx->ks;
     ks[i].ksk = nullptr;
     if (se.key) pz::ks_bind_key(se.ctx, se.key, ks[i]);
@@ -593,6 +596,10 @@ pz_status pz_server_create(int device, size_t arena_bytes, size_t max_items, pz_
       delete s;
       return PZ_ERR_CUDA;
     }
+    if (pz::dev_malloc(&s->d_err, sizeof(u32)) != cudaSuccess || cudaMemset(s->d_err, 0, sizeof(u32)) != cudaSuccess) {
+      delete s;
+      return PZ_ERR_OUT_OF_MEMORY;
+    }
     const pz_server::Layout lay = s->layout(max_items);
     for (int b = 0; b < 2; b++) {
       if (cudaMallocHost(&s->h_buf[b], lay.total) != cudaSuccess || pz::dev_malloc(&s->d_buf[b], lay.total) != cudaSuccess ||
@@ -724,22 +731,42 @@ pz_status pz_server_step(pz_server *s, size_t *gates_run) {
   for (auto *j : s->active) (j->level >= j->v.levels ? fin : still).push_back(j);
   st = finish_outputs(s, fin);
   if (st != PZ_OK) return st;
+  u32 lost = 0;  // a kernel of this step gave up a wait: what the step computed is not valid
   if (!s->dry) {
-    cudaError_t e = cudaStreamSynchronize(s->stream);
+    cudaError_t e = pz::read_error_word(s->d_err, &lost, s->stream);
     if (e != cudaSuccess) return s->cuda("step", e);
+  }
+  if (lost) {
+    fin.insert(fin.end(), still.begin(), still.end());
+    still.clear();
+    std::sort(run.begin(), run.end());
+    for (auto *j : fin)
+      if (!std::binary_search(run.begin(), run.end(), j) && j->level < j->v.levels) still.push_back(j);
   }
   const double t = now_ms();
   for (auto *j : fin) {
-    j->state = 2;
+    const bool failed = lost && std::binary_search(run.begin(), run.end(), j);
+    if (!failed && j->level < j->v.levels) continue;  // not run this step: still active
+    j->state = failed ? 3 : 2;
     j->t_done = t;
     s->release(j->base, j->slots);
     s->sessions[j->session].jobs_in_flight--;
-    s->n_done++;
+    failed ? s->n_failed++ : s->n_done++;
   }
   s->active.swap(still);
   s->steps++;
   s->gates += total;
   if (gates_run) *gates_run = total;
+  if (lost) {
+    cudaError_t e = cudaMemsetAsync(s->d_err, 0, sizeof(u32), s->stream);
+    for (auto *j : run)  // their contexts' pz_ctx_device_error reports it too
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(s->sessions[j->session].ctx->d_err, &lost, sizeof(u32), cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return s->cuda("step", e);
+    return s->fail(PZ_ERR_CUDA, "a kernel gave up a wait (device error bits " + std::to_string(lost) +
+                                    "): the jobs of this step failed");
+  }
   return PZ_OK;
 }
 

@@ -200,3 +200,50 @@ def test_waits_that_run_out_end_the_kernel(gpu_available, count, limit):
         eng.set_wait_limit(-1)
         assert np.array_equal(run(), want)
         assert eng.device_error() == 0
+
+
+def test_waits_that_run_out_are_errors_of_the_call(gpu_available):
+    """What a synchronous call computed after a wait gave up is never returned as
+    good: host-buffer gates, circuits and non-interactive inputs fail until the
+    error word has been asked for, a server's step fails the jobs that it
+    advanced and no others, and all of them work again afterwards."""
+    P = pz()
+    eng = P.Engine("NI_2P")
+    p = eng.p
+    g = np.random.default_rng(29)
+    key = eng.upload_key(g.integers(0, eng.Q, (p.lwe_n, p.rgsw_rows, eng.N), dtype=np.uint64),
+                         g.integers(0, eng.Q, (p.n_auto_keys, p.auto_rows, eng.N), dtype=np.uint64),
+                         g.integers(0, p.lwe_q, (p.lwe_d * eng.N, p.lwe_n + 1), dtype=np.uint64))
+    ksk = eng.upload_ni_ksk(g.integers(0, eng.Q, (2 * p.ni_ks_d, eng.N), dtype=np.uint64))
+    C = P.Circuit()
+    C.output(C.gate("nand", C.input(), C.input()))
+    x = g.integers(0, eng.Q, (2, eng.L), dtype=np.uint64)
+    b = g.integers(0, eng.Q, (1, eng.N), dtype=np.uint64)
+    calls = [lambda: eng.gate_batch(key, np.array([1], np.uint8), x[:1], x[1:]), lambda: C.run(eng, key, x),
+             lambda: eng.ni_ingest(ksk, b"\x05" * 32, b, 3)]
+    want = [call() for call in calls]
+    eng.set_wait_limit(0)
+    S = P.Server(device=0, arena_bytes=1 << 22, max_items=64)
+    sid = S.add_session(eng, key)
+    for _ in range(2):
+        for call in calls:  # the last has no such waits: it reports what the others set
+            with pytest.raises(RuntimeError, match="gave up a wait"):
+                call()
+        assert eng.device_error() == 1
+    wires = P.Circuit()
+    wires.output(wires.input())  # no gate: nothing of it is computed
+    job, other = S.submit(sid, C, x), S.submit(sid, wires, x[:1])
+    with pytest.raises(RuntimeError, match="gave up a wait"):
+        S.step()
+    assert S.status(job)["state"] == P.server.FAILED and S.status(other)["state"] == P.server.DONE
+    st = S.stats()
+    assert (st["active"], st["failed"], st["done"], st["arena_slots_used"]) == (0, 1, 1, 0)
+    assert np.array_equal(S.result(other), x[:1])
+    assert eng.device_error() == 1
+    eng.set_wait_limit(-1)
+    for call, w in zip(calls, want):
+        assert np.array_equal(call(), w)
+    sid = S.add_session(eng, key)
+    job = S.submit(sid, C, x)
+    S.run_until_idle()
+    assert np.array_equal(S.result(job), want[1])
