@@ -231,8 +231,8 @@ pz_status pz_ctx_pbs_slots(pz_ctx *ctx, int variant, size_t *slots);
  * reference counterpart. */
 const char *pz_kernel_revision(void);
 /* Autotuner: times the blind-rotation variants 0 and 3 on synthetic key-switched
- * LWEs with this key -- `batch` of them, or, from one wave up, the largest
- * whole number of that variant's waves not above `batch` -- and keeps the
+ * LWEs with this key -- `batch` of them, or, from one wave of variant 0 up, the
+ * largest whole number of its waves not above `batch` -- and keeps the
  * fastest per ciphertext (*ms: its time for `batch`); then times the
  * key-switch kernel with 8, 16 and 32 ciphertexts per CTA and its
  * tensor-core form (64) on `batch` inputs and keeps the fastest.  Both become the context's defaults and the choice

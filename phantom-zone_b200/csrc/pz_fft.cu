@@ -774,13 +774,24 @@ cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const
   return cudaGetLastError();
 }
 
+// From the resources: the occupancy calculator answers one CTA per SM for every
+// kernel that allocates tensor memory, and four run (592 ciphertexts take 30.3 ms,
+// 148 take 15.1).
 cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas) {
   typedef fft::Shape<fft::QUAD> H;
   const size_t smem = H::smem_bytes(br_q, n);
-  const cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel<fft::QUAD>, smem);
-  return e != cudaSuccess ? e
-                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, fft::pbs_fft_kernel<fft::QUAD>,
-                                                                          H::THREADS, smem);
+  cudaFuncAttributes a;
+  int dev = 0, shared = 0, reserved = 0, regs = 0;
+  cudaError_t e = cudaFuncGetAttributes(&a, fft::pbs_fft_kernel<fft::QUAD>);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
+  if (e != cudaSuccess) return e;
+  const size_t by_shared = (size_t)shared / (smem + a.sharedSizeBytes + reserved);
+  const size_t by_regs = (size_t)regs / ((size_t)std::max(a.numRegs, 1) * H::THREADS);
+  *ctas = (int)std::min({by_shared, by_regs, (size_t)(512 / H::COLS)});
+  return cudaSuccess;
 }
 
 struct Batch {  // the arguments of pbs_fft_kernel
@@ -792,25 +803,41 @@ struct Batch {  // the arguments of pbs_fft_kernel
   u64 *out, *rlwe_dbg;
   u32 br_q, n;  // the largest of the batch
 };
+// The launch of `grid` CTAs (SPLIT: clusters) of form F, its attribute in attr.
+template <fft::Form F>
+static cudaError_t form_config(u32 br_q, u32 n, int grid, cudaStream_t s, cudaLaunchConfig_t *cfg,
+                               cudaLaunchAttribute *attr) {
+  typedef fft::Shape<F> H;
+  const size_t smem = H::smem_bytes(br_q, n);
+  *cfg = {};
+  cfg->gridDim = dim3((unsigned)(F == fft::SPLIT ? 2 * grid : grid));
+  cfg->blockDim = dim3(H::THREADS);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = s;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim = {2, 1, 1};
+  cfg->attrs = attr;
+  cfg->numAttrs = F == fft::SPLIT ? 1 : 0;
+  return opt_in_smem((const void *)fft::pbs_fft_kernel<F>, smem);
+}
 template <fft::Form F>
 static cudaError_t launch_form(const Batch &b, size_t begin, size_t end, int grid, cudaStream_t s) {
-  typedef fft::Shape<F> H;
-  const size_t smem = H::smem_bytes(b.br_q, b.n);
-  cudaError_t e = opt_in_smem((const void *)fft::pbs_fft_kernel<F>, smem);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(F == fft::SPLIT ? 2 * grid : grid));
-  cfg.blockDim = dim3(H::THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
+  cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim = {2, 1, 1};
-  cfg.attrs = attr;
-  cfg.numAttrs = F == fft::SPLIT ? 1 : 0;
+  cudaError_t e = form_config<F>(b.br_q, b.n, grid, s, &cfg, attr);
+  if (e != cudaSuccess) return e;
   e = cudaLaunchKernelEx(&cfg, fft::pbs_fft_kernel<F>, b.P, b.descs, b.item_desc, b.out_idx, b.ks, b.ks_stride, b.gates,
                          b.out, (int)begin, (int)end, b.rlwe_dbg);
   return e != cudaSuccess ? e : cudaGetLastError();
+}
+cudaError_t pbs_fft_clusters(u32 br_q, u32 n, size_t *clusters) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  int m = 0;
+  cudaError_t e = form_config<fft::SPLIT>(br_q, n, 1, nullptr, &cfg, attr);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&m, fft::pbs_fft_kernel<fft::SPLIT>, &cfg);
+  *clusters = (size_t)std::max(m, 1);
+  return e;
 }
 static cudaError_t launch_form(fft::Form form, const Batch &b, size_t begin, size_t end, int grid, cudaStream_t s) {
   switch (form) {

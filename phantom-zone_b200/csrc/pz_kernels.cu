@@ -1255,20 +1255,19 @@ cudaError_t pbs_slots(int logn, bool d1, u32 br_q, u32 n, int variant, size_t *s
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const size_t smem = pbs_smem_bytes(logn, br_q, n);
-  size_t div = 1;
 #define PZ_OCC(K, TH, SM)                                                                 \
   if ((e = set_smem(K, SM)) != cudaSuccess) return e;                                      \
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, TH, SM);
   if (logn == 11 && d1) {
+    if (variant == PBS_SPLIT) return pbs_fft_clusters(br_q, n, slots);
     e = pbs_fft_per_sm(br_q, n, &per_sm);
-    div = variant == PBS_SPLIT ? 2 : 1;
   } else if (logn == 11) { PZ_OCC((pbs_kernel<11, false, 1>), 256, smem) }
   else if (logn == 9 && d1) { PZ_OCC((pbs_kernel<9, true, 1>), 64, smem) }
   else if (logn == 9) { PZ_OCC((pbs_kernel<9, false, 1>), 64, smem) }
   else return cudaErrorInvalidValue;
 #undef PZ_OCC
   if (e != cudaSuccess) return e;
-  *slots = std::max<size_t>((size_t)per_sm * sms / div, 1);
+  *slots = std::max<size_t>((size_t)per_sm * sms, 1);
   return cudaSuccess;
 }
 

@@ -833,11 +833,12 @@ pz_status pz_ctx_autotune(pz_ctx *c, const pz_key *k, size_t batch, int *variant
   int bv = c->pbs_variant;
   for (int v : shapes) {
     if (e != cudaSuccess) break;
-    // a batch of at least one wave is timed in whole waves of this shape (a
-    // partial last wave would charge the shape for the batch's remainder):
-    // the largest multiple of the shape's resident items not above the batch
+    // a batch of at least one wave of shape 0 (592 ciphertexts, eight waves of
+    // shape 3) is timed in whole waves of it for every shape, as a partial last
+    // wave would charge the shape for the batch's remainder; smaller ones as they
+    // are, since 100 ciphertexts cost shape 3 two waves
     size_t slots = 1, items = batch;
-    if ((e = pz::pbs_slots((int)c->logn, d1, c->P.br_q, c->P.lwe_n, v, &slots)) != cudaSuccess) break;
+    if ((e = pz::pbs_slots((int)c->logn, d1, c->P.br_q, c->P.lwe_n, 0, &slots)) != cudaSuccess) break;
     if (batch >= slots) items = batch / slots * slots;
     auto launch = [&]() {
       return pz::launch_pbs((int)c->logn, d1, br, d_ks, cols, d_g, d_out, items, nullptr, c->grid_limit, c->stream, v);

@@ -247,3 +247,13 @@ def test_waits_that_run_out_are_errors_of_the_call(gpu_available):
     job = S.submit(sid, C, x)
     S.run_until_idle()
     assert np.array_equal(S.result(job), want[1])
+
+
+@pytest.mark.parametrize("param", ["I_2P_LB_SR", "NI_8P"])
+def test_resident_ciphertexts_of_each_shape(gpu_available, param):
+    """The two-SM form holds a ciphertext per pair of SMs, the names of the other
+    shape four per SM."""
+    import torch
+    eng = pz().Engine(param)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert [eng.pbs_slots(v) for v in range(5)] == [4 * sms, 4 * sms, 4 * sms, sms // 2, 4 * sms]
