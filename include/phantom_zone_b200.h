@@ -136,6 +136,14 @@ uint64_t pz_ctx_ntt_root(const pz_ctx *ctx);
 pz_status pz_key_upload(pz_ctx *ctx, const pz_server_key_view *key, pz_key **out);
 void pz_key_release(pz_key *key);
 size_t pz_key_device_bytes(const pz_key *key);
+/* Keys of the N = 2048 one-digit parameter sets also get their FFT form, which
+ * the products run on (NI_8P: 132 of 310 MB).  on = 0: keys made from now on
+ * (upload, import, aggregation) do without, like keys that the device had no room
+ * for: the same words by integer transforms, 1.2 to 1.8 times slower.
+ * pz_key_has_fft tells which (1: the FFT form is there).  No reference
+ * counterpart. */
+pz_status pz_ctx_set_key_fft(pz_ctx *ctx, int on);
+int pz_key_has_fft(const pz_key *key);
 
 /* out[i] = gate[i](c0[i], c1[i]); c0, c1, out: [count][N + 1].
  * Host memory, synchronous (copies in and out inside the call). */

@@ -11,6 +11,7 @@
 struct pz_ctx {
   int param_id = 0, device = 0;
   bool pooled = false;  // holds a reference to the device's memory pool
+  bool key_fft = true;  // keys get their FFT form
   pz_params P{};
   pz::u32 logn = 0;
   pz::u64 root = 0;
@@ -87,10 +88,13 @@ cudaError_t dev_malloc(T **p, size_t bytes) {
 // Build k->d_ksk8 from k->d_ksk (when the parameter set's digits fit s8 and
 // the rows come in whole 32-row blocks; otherwise, or when the device is out
 // of memory, the key keeps the IMAD key-switch kernels only).
-void build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s);
+cudaError_t build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s);
 // Build the FFT form of k's RGSW and automorphism keys (N = 2048 one-digit
-// sets; without the memory for it the key keeps the integer kernels only).
-void build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s);
+// sets; without the memory for it, or with c->key_fft off, the key keeps the
+// integer kernels only).
+cudaError_t build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s);
+// both; any failure but lack of memory is one of the caller's
+cudaError_t build_key_forms(pz_ctx *c, pz_key *k, cudaStream_t s);
 void free_key_arrays(pz_key *k);
 // BrParams of context c bound to key k (both key forms; k null: no key)
 void br_bind_key(const pz_ctx *c, const pz_key *k, BrParams &br);

@@ -276,42 +276,55 @@ pz_status check_gates_host(pz_ctx *c, const uint8_t *gates, size_t count, bool r
 }  // namespace
 
 namespace pz {
-void build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s) {
-  const pz_params &P = c->P;
-  const u32 rows = P.lwe_d * P.rlwe_n;
-  if (!k->d_ksk || rows % 32 || P.rlwe_n % 32 || P.lwe_d > 16 || P.lwe_logb > 7) return;
-  const u32 planes = ksk8_planes(c->ks.mask), cols = ksk8_cols(P.lwe_n);
-  const size_t bytes = (size_t)planes * rows * cols;
-  if (pz::dev_malloc(&k->d_ksk8, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    k->d_ksk8 = nullptr;
-    return;
-  }
-  if (launch_ksk_planes(k->d_ksk, rows, ks_stride(P), P.lwe_n, planes, k->d_ksk8, s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(k->d_ksk8);
-    k->d_ksk8 = nullptr;
-    return;
-  }
-  k->bytes += bytes;
+// A derived form of a key in *p: bytes allocated, then made by launch().  Lack of
+// memory leaves *p null and is no error.
+template <class Launch>
+static cudaError_t derive(void **p, size_t bytes, cudaStream_t s, const Launch &launch) {
+  cudaError_t e = dev_malloc(p, bytes);
+  if (e == cudaSuccess && (e = launch()) == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) return e;
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  cudaFree(*p);
+  *p = nullptr;
+  return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
 }
 
-void build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s) {
+cudaError_t build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s) {
   const pz_params &P = c->P;
-  if (!c->d_fft) return;
+  const u32 rows = P.lwe_d * P.rlwe_n;
+  if (k->d_ksk8 || !k->d_ksk || rows % 32 || P.rlwe_n % 32 || P.lwe_d > 16 || P.lwe_logb > 7) return cudaSuccess;
+  const u32 planes = ksk8_planes(c->ks.mask), cols = ksk8_cols(P.lwe_n);
+  const size_t bytes = (size_t)planes * rows * cols;
+  const cudaError_t e = derive((void **)&k->d_ksk8, bytes, s, [&] {
+    return launch_ksk_planes(k->d_ksk, rows, ks_stride(P), P.lwe_n, planes, k->d_ksk8, s);
+  });
+  if (k->d_ksk8) k->bytes += bytes;
+  return e;
+}
+
+cudaError_t build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s) {
+  const pz_params &P = c->P;
+  if (k->d_fft_rgsw || !c->d_fft || !c->key_fft) return cudaSuccess;
   const size_t rg = fft_key_bytes(P.lwe_n), au = fft_key_bytes(P.n_auto_keys);
-  if (pz::dev_malloc(&k->d_fft_rgsw, rg) == cudaSuccess && pz::dev_malloc(&k->d_fft_autos, au) == cudaSuccess &&
-      launch_fft_key(k->d_rgsw, P.rgsw_rows, P.lwe_n, c->rc, c->d_fft, k->d_fft_rgsw, s) == cudaSuccess &&
-      launch_fft_key(k->d_autos, P.auto_rows, P.n_auto_keys, c->rc, c->d_fft, k->d_fft_autos, s) == cudaSuccess &&
-      cudaStreamSynchronize(s) == cudaSuccess) {
+  cudaError_t e = derive(&k->d_fft_rgsw, rg, s, [&] {
+    return launch_fft_key(k->d_rgsw, P.rgsw_rows, P.lwe_n, c->rc, c->d_fft, k->d_fft_rgsw, s);
+  });
+  if (e == cudaSuccess && k->d_fft_rgsw)
+    e = derive(&k->d_fft_autos, au, s, [&] {
+      return launch_fft_key(k->d_autos, P.auto_rows, P.n_auto_keys, c->rc, c->d_fft, k->d_fft_autos, s);
+    });
+  if (k->d_fft_autos) {
     k->bytes += rg + au;
-    return;
+  } else {
+    cudaFree(k->d_fft_rgsw);
+    k->d_fft_rgsw = nullptr;
   }
-  cudaGetLastError();
-  cudaFree(k->d_fft_rgsw);
-  cudaFree(k->d_fft_autos);
-  k->d_fft_rgsw = k->d_fft_autos = nullptr;
+  return e;
+}
+
+cudaError_t build_key_forms(pz_ctx *c, pz_key *k, cudaStream_t s) {
+  const cudaError_t e = build_ksk8(c, k, s);
+  return e == cudaSuccess ? build_fft_key(c, k, s) : e;
 }
 
 void br_bind_key(const pz_ctx *c, const pz_key *k, BrParams &br) {
@@ -640,8 +653,8 @@ pz_status pz_key_upload(pz_ctx *c, const pz_server_key_view *v, pz_key **out) {
     for (size_t col = 0; col < cols; col++) ksk32[r * stride + col] = (u32)(v->lwe_ksk[r * cols + col] & (P.lwe_q - 1));
   if ((e = cudaMemcpy(k->d_ksk, ksk32.data(), ksk32.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
     return cleanup(PZ_ERR_CUDA, std::string("ksk copy: ") + cudaGetErrorString(e));
-  pz::build_ksk8(c, k, c->stream);
-  pz::build_fft_key(c, k, c->stream);
+  if ((e = pz::build_key_forms(c, k, c->stream)) != cudaSuccess)
+    return cleanup(PZ_ERR_CUDA, std::string("key forms: ") + cudaGetErrorString(e));
   *out = k;
   return PZ_OK;
 }
@@ -711,8 +724,8 @@ pz_status pz_key_upload_seeded(pz_ctx *c, const pz_seeded_server_key_view *v, pz
     return cleanup(PZ_ERR_CUDA, std::string("ksk b column: ") + cudaGetErrorString(e));
   cudaFree(d_stage);
   d_stage = nullptr;
-  pz::build_ksk8(c, k, c->stream);
-  pz::build_fft_key(c, k, c->stream);
+  if ((e = pz::build_key_forms(c, k, c->stream)) != cudaSuccess)
+    return cleanup(PZ_ERR_CUDA, std::string("key forms: ") + cudaGetErrorString(e));
   *out = k;
   return PZ_OK;
 }
@@ -724,6 +737,12 @@ void pz_key_release(pz_key *k) {
   delete k;
 }
 size_t pz_key_device_bytes(const pz_key *k) { return k ? k->bytes : 0; }
+int pz_key_has_fft(const pz_key *k) { return k && k->d_fft_rgsw ? 1 : 0; }
+pz_status pz_ctx_set_key_fft(pz_ctx *c, int on) {
+  if (!c || (on != 0 && on != 1)) return PZ_ERR_INVALID_ARGUMENT;
+  c->key_fft = on != 0;
+  return PZ_OK;
+}
 
 pz_status pz_gate_batch(pz_ctx *c, const pz_key *k, const uint8_t *gates, const uint64_t *c0,
                         const uint64_t *c1, uint64_t *out, size_t count) {

@@ -9,8 +9,8 @@
 // of ks_stride words).  The evaluation domain depends on the NTT root and
 // the scale on the build's multiply-accumulate reduction, so the header
 // (version 2) records both and an import into a context with another root,
-// key form or parameter set is refused.  Import is a plain copy: no forward
-// NTT, no conversion.
+// key form or parameter set is refused.  Import is a plain copy, and the
+// key's derived forms (KSK byte planes, FFT form) made from it on the device.
 //
 // (The circuit blob lives with the circuit in pz_circuit.cu.)
 #include <cstring>
@@ -104,13 +104,13 @@ pz_status pz_key_import(pz_ctx *c, const void *buf, size_t size, pz_key **out) {
   if (e == cudaSuccess) e = cudaMemcpy(k->d_rgsw, p, rg, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(k->d_autos, p + rg, au, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(k->d_ksk, p + rg + au, ks, cudaMemcpyHostToDevice);
+  // derived on the device; the blob carries only the u32 rows and the integer form
+  if (e == cudaSuccess) e = pz::build_key_forms(c, k, c->stream);
   if (e != cudaSuccess) {
     pz::free_key_arrays(k);
     delete k;
     return pz::cuda_fail(c, "pz_key_import", e);
   }
-  pz::build_ksk8(c, k, c->stream);  // derived on the device; the blob carries only the u32 rows
-  pz::build_fft_key(c, k, c->stream);
   *out = k;
   return PZ_OK;
 }

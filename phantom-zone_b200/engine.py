@@ -88,6 +88,11 @@ class DeviceKey:
     def device_bytes(self):
         return lib().pz_key_device_bytes(self.h)
 
+    @property
+    def has_fft(self):
+        """Whether the key's FFT form is on the device (see Engine.set_key_fft)."""
+        return bool(lib().pz_key_has_fft(self.h))
+
     def export(self):
         """Device-form key as bytes (checkpoint / hand-over between processes)."""
         size = ctypes.c_size_t()
@@ -240,6 +245,11 @@ class Engine:
         return {"variant": v.value, "ks_tile": t.value}
 
     # -- keys --------------------------------------------------------------
+    def set_key_fft(self, on=True):
+        """Whether keys made from now on get their FFT form (default) or keep to
+        the integer kernels, in less memory and with the same words."""
+        check(lib().pz_ctx_set_key_fft(self.h, int(on)), self.h, "pz_ctx_set_key_fft")
+
     def upload_key(self, rgsw, autos, lwe_ksk):
         """Upload a coefficient-domain server key (layouts of pz_server_key_view)."""
         p = self.p
