@@ -17,7 +17,8 @@
 //      session and runs them as ONE ragged key-switch launch (tiles of one
 //      session each) plus ONE ragged blind-rotation launch (each CTA loads
 //      its gate's parameter set and key from a descriptor table), chunked at
-//      max_items gates,
+//      max_items gates (and one such pair per kind of key, where some lack
+//      forms that others have),
 //   3. retires jobs whose last level ran: outputs are gathered (not() applied)
 //      and copied out, their arena ranges are freed.
 // Jobs admitted while others are mid-circuit join at their own level 1, so
@@ -71,8 +72,6 @@ struct pz_server {
   size_t key_budget = SIZE_MAX, managed_bytes = 0;
   u64 use_clock = 0, key_imports = 0, key_evictions = 0;
   bool descs_dirty = false;
-  bool fft = false;     // every session with a resident key has its FFT form
-  bool ks_mma = false;  // every session with a resident key has its KSK byte planes: tensor-core key switch
   int logn = -1;
   bool d1 = true;
   size_t L = 0;
@@ -188,6 +187,15 @@ struct pz_server {
   }
 
   bool resident(const Session &se) const { return !se.managed || se.owned || se.virt_resident; }
+  // the kernels that a session's resident key has the forms for (dry run: one kind)
+  struct Kind {
+    bool fft, mma;  // blind rotation over FFTs; key switch on the tensor cores
+    bool operator==(const Kind &o) const { return fft == o.fft && mma == o.mma; }
+    int rank() const { return (fft ? 0 : 2) + (mma ? 0 : 1); }
+  };
+  Kind kind(const Session &se) const {
+    return {se.key && se.key->d_fft_rgsw, se.key && se.key->d_ksk8 && se.ctx->P.lwe_d <= 16};
+  }
 
   ~pz_server() {
     for (auto &kv : jobs) delete kv.second;
@@ -238,13 +246,6 @@ pz_status upload_descs(pz_server *s) {
     ks[i].ksk = nullptr;
     if (se.key) pz::ks_bind_key(se.ctx, se.key, ks[i]);
   }
-  bool mma = s->max_d <= 16, fft = true;
-  for (size_t i = 0; i < s->sessions.size(); i++) {
-    if (s->sessions[i].key && !s->sessions[i].key->d_ksk8) mma = false;
-    if (s->sessions[i].key && !s->sessions[i].key->d_fft_rgsw) fft = false;
-  }
-  s->ks_mma = mma;
-  s->fft = fft;
   s->descs_dirty = false;
   cudaFree(s->d_br);
   cudaFree(s->d_ksp);
@@ -429,12 +430,16 @@ struct Item {
   u32 in0, in1, out;
 };
 
-// Run the sorted items of one step, in chunks of max_items.
+// Run the sorted items of one step, in chunks of max_items and one kind of key.
 pz_status run_items(pz_server *s, const std::vector<Item> &items) {
   if (s->dry || items.empty()) return PZ_OK;
   const pz_server::Layout lay = s->layout(s->max_items);
-  for (size_t c0 = 0; c0 < items.size(); c0 += s->max_items) {
-    const size_t n = std::min(s->max_items, items.size() - c0);
+  for (size_t c0 = 0, n = 0; c0 < items.size(); c0 += n) {
+    const pz_server::Kind kind = s->kind(s->sessions[items[c0].session]);
+    for (n = 1; n < s->max_items && c0 + n < items.size(); n++)
+      if (items[c0 + n].session != items[c0 + n - 1].session &&
+          !(s->kind(s->sessions[items[c0 + n].session]) == kind))
+        break;
     const int b = s->flip;
     s->flip ^= 1;
     cudaError_t e = cudaEventSynchronize(s->buf_free[b]);  // its previous chunk has been read
@@ -445,7 +450,7 @@ pz_status run_items(pz_server *s, const std::vector<Item> &items) {
     u32 *hd = (u32 *)(h + lay.desc);
     pz::KsTile *ht = (pz::KsTile *)(h + lay.tiles);
     size_t ntiles = 0;
-    const u32 tile_cap = s->ks_mma ? (u32)pz::KSM_ROWS : (u32)pz::KS_TILE_CT;
+    const u32 tile_cap = kind.mma ? (u32)pz::KSM_ROWS : (u32)pz::KS_TILE_CT;
     for (size_t i = 0; i < n; i++) {
       const Item &it = items[c0 + i];
       hg[i] = it.gate;
@@ -461,15 +466,16 @@ pz_status run_items(pz_server *s, const std::vector<Item> &items) {
     if ((e = cudaMemcpyAsync(d, h, lay.total, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess)
       return s->cuda("item upload", e);
     if ((e = cudaEventRecord(s->buf_free[b], s->stream)) != cudaSuccess) return s->cuda("cudaEventRecord", e);
-    e = (s->ks_mma ? pz::launch_ks_mma_ragged : pz::launch_ks_ragged)(
-        s->d_ksp, (const pz::KsTile *)(d + lay.tiles), ntiles, n, s->max_n, (u32)(s->L - 1), s->max_d, d + lay.gate,
+    e = (kind.mma ? pz::launch_ks_mma_ragged : pz::launch_ks_ragged)(
+        s->d_ksp, (const pz::KsTile *)(d + lay.tiles), ntiles, n, s->max_n, (u32)(s->L - 1),
+        kind.mma ? std::min(s->max_d, 16u) : s->max_d, d + lay.gate,
         s->d_arena, (const u32 *)(d + lay.in0), (const u32 *)(d + lay.in1), s->d_ksout, s->ks_stride, s->stream);
     if (e != cudaSuccess) return s->cuda("launch_ks_ragged", e);
     // a step of at most half the SMs' gates: one cluster of two CTAs per gate (the latency form)
     const int variant = (s->logn == 11 && s->d1 && n <= (size_t)s->sm_count / 2) ? pz::PBS_SPLIT : s->pbs_variant;
     e = pz::launch_pbs_ragged(s->logn, s->d1, s->d_br, (const u32 *)(d + lay.desc), s->max_br_q, s->max_n,
                               s->d_ksout, s->ks_stride, d + lay.gate, s->d_arena, (const u32 *)(d + lay.out), n,
-                              s->grid_limit, s->stream, variant, s->fft);
+                              s->grid_limit, s->stream, variant, kind.fft);
     if (e != cudaSuccess) return s->cuda("launch_pbs_ragged", e);
     s->launches += 2;
   }
@@ -705,11 +711,19 @@ pz_status pz_server_step(pz_server *s, size_t *gates_run) {
   if (st != PZ_OK) return st;
   std::vector<pz_server::Job *> run;
   select_jobs(s, run);
-  // next level of every selected job, sorted by session (counting sort)
-  std::vector<size_t> per(s->sessions.size() + 1, 0);
-  for (auto *j : run) per[j->session + 1] += j->v.level_off[j->level + 1] - j->v.level_off[j->level];
-  for (size_t i = 1; i < per.size(); i++) per[i] += per[i - 1];
-  const size_t total = per.back();
+  // next level of every selected job, sorted by session (counting sort), sessions
+  // whose keys take the same kernels together: each kind is launched by itself, so
+  // a key without its derived forms holds up nobody else's
+  std::vector<size_t> per(s->sessions.size(), 0);
+  for (auto *j : run) per[j->session] += j->v.level_off[j->level + 1] - j->v.level_off[j->level];
+  size_t total = 0;
+  for (int rank = 0; rank < 4; rank++)
+    for (size_t i = 0; i < per.size(); i++)
+      if (s->kind(s->sessions[i]).rank() == rank) {
+        const size_t width = per[i];
+        per[i] = total;
+        total += width;
+      }
   std::vector<Item> items(total);
   for (auto *j : run) {
     s->sessions[j->session].last_use = ++s->use_clock;
@@ -847,6 +861,11 @@ pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid
   for (u32 i = 0; i < (u32)s->sessions.size(); i++)
     if (s->sessions[i].key) live.push_back(i);
   if (live.empty()) return s->fail(PZ_ERR_INVALID_ARGUMENT, "autotune needs a session with a resident key");
+  // of one kind, the fastest there is
+  auto rank = [&](u32 i) { return s->kind(s->sessions[i]).rank(); };
+  const u32 top = *std::min_element(live.begin(), live.end(), [&](u32 x, u32 y) { return rank(x) < rank(y); });
+  live.erase(std::remove_if(live.begin(), live.end(), [&](u32 i) { return rank(i) != rank(top); }), live.end());
+  const bool fft = s->kind(s->sessions[top]).fft;
   for (size_t i = 0; i < batch; i++) {
     desc[i] = live[i % live.size()];
     const pz_params &P = s->sessions[desc[i]].ctx->P;
@@ -879,7 +898,7 @@ pz_status pz_server_autotune(pz_server *s, size_t batch, int *variant, int *grid
       for (int gi = 0; gi < 2 && st == PZ_OK; gi++) {
         auto launch = [&]() {
           return pz::launch_pbs_ragged(s->logn, s->d1, s->d_br, d_desc, s->max_br_q, s->max_n, d_ks, s->ks_stride,
-                                       d_g, s->d_arena, d_out, batch, grids[gi], s->stream, 0, s->fft);
+                                       d_g, s->d_arena, d_out, batch, grids[gi], s->stream, 0, fft);
         };
         if (!CK(launch(), "launch_pbs_ragged")) break;  // warm-up
         if (!CK(cudaEventRecord(a, s->stream), "cudaEventRecord")) break;

@@ -103,3 +103,39 @@ def test_products_and_automorphisms(gpu_available):
             call(key, t, to_dev(idx), trivial=True)
             trivial.append(to_host(t))
         assert np.array_equal(trivial[0], trivial[1])
+
+
+@pytest.mark.parametrize("width", [5, 75, 149, 223, 297, 371, 596])
+def test_server_with_keys_of_both_forms(gpu_available, width):
+    """A step whose width lies on either side of each placing boundary (the ragged
+    launches scatter their outputs): sessions whose keys have the FFT form run over
+    it in a launch of their own beside one whose key does not, every job with the
+    words it has alone."""
+    P = pz()
+    g = np.random.default_rng(41)
+    sessions = []
+    S = P.Server(device=0, arena_bytes=1 << 27, max_items=4096)
+    for param, fft in (("I_2P_LB_SR", True), ("NI_8P", True), ("I_8P", False)):
+        eng = P.Engine(param)
+        p = eng.p
+        eng.set_key_fft(fft)
+        key = eng.upload_key(g.integers(0, eng.Q, (p.lwe_n, p.rgsw_rows, eng.N), dtype=np.uint64),
+                             g.integers(0, eng.Q, (p.n_auto_keys, p.auto_rows, eng.N), dtype=np.uint64),
+                             g.integers(0, p.lwe_q, (p.lwe_d * eng.N, p.lwe_n + 1), dtype=np.uint64))
+        assert key.has_fft == fft
+        sessions.append((eng, key, S.add_session(eng, key)))
+    counts = (width // 2, width - width // 2, 3)
+    jobs = []
+    for (eng, key, sid), count in zip(sessions, counts):
+        gates = (np.arange(count) % 6).astype(np.uint8)
+        C = P.Circuit()
+        inputs = [C.input() for _ in range(count + 1)]
+        C.outputs([C.gate(["and", "nand", "or", "nor", "xor", "xnor"][t], inputs[i], inputs[i + 1])
+                   for i, t in enumerate(gates)])
+        x = g.integers(0, eng.Q, (count + 1, eng.L), dtype=np.uint64)
+        jobs.append((S.submit(sid, C, x), eng.gate_batch(key, gates, x[:-1], x[1:])))
+    assert S.step() == width + 3
+    st = S.stats()
+    assert st["done"] == 3 and st["launches"] == 4  # a key switch and a blind rotation for either form
+    for job, want in jobs:
+        assert np.array_equal(S.result(job), want)
