@@ -20,6 +20,8 @@
 #include <mutex>
 #include <utility>
 
+#include <cooperative_groups.h>
+
 #include "pz_blind.cuh"
 #include "pz_kernels.cuh"
 
@@ -943,6 +945,206 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, MINB)
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same on a cluster of two CTAs (two SMs), for small batches: rank 0 holds a,
+// rank 1 b, in the one-CTA kernel's layouts and domains.  Each CTA transforms its
+// own polynomial; the transformed digits cross through distributed shared memory
+// (two slots, alternating by operation), with one cluster barrier per operation on
+// both (both build the same schedule from the same input) and one per ciphertext.
+// External product: each CTA forms one output from both digit polynomials.
+// Automorphism: rank 0 permutes, decomposes and transforms a(X^k) while rank 1
+// permutes b in the evaluation domain; after the barrier each multiplies by its row
+// of the key.  N = 2048, one-digit sets.  Bound by barriers and latency: one
+// ciphertext takes 8.3 ms (I_2P) and 10.3 (NI_8P), in one CTA 11.2 and 13.3.
+// ---------------------------------------------------------------------------
+constexpr int SPLIT_REGIONS = 4;  // two of exchange buffer, two slots of digits
+namespace cg = cooperative_groups;
+
+// out = mac_reduce(x ka + y kb), x, y in the evaluation layout, key rows in the device layout
+template <int LOGN>
+__device__ __forceinline__ void mac_two_rows(u64 (&x)[8], const u64 (&y)[8], const u64 *ka, const u64 *kb,
+                                             const RingConsts &rc) {
+  const int j = threadIdx.x;
+  const u64 q = rc.q, qi = rc.qinv_neg;
+#pragma unroll
+  for (int rr = 0; rr < 4; rr++) {
+    const int di = dev_index<LOGN>(j, 2 * rr);
+    u64 a[2], b[2];
+    ld_key2(ka + di, a[0], a[1]);
+    ld_key2(kb + di, b[0], b[1]);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int r = 2 * rr + e;
+      u64 hi, lo;
+      sum2_128(x[r], a[e], y[r], b[e], hi, lo);
+      x[r] = mac_reduce<LOGN>(hi, lo, q, qi);
+    }
+  }
+}
+
+template <int LOGN>
+__device__ __forceinline__ void split_op(u64 (&x)[8], u32 op, u32 t, const BrParams &P, u64 *sm, u64 *slots,
+                                         const u64 *peer_slots, unsigned rank, cg::cluster_group &cl) {
+  constexpr int N = 1 << LOGN, T = NttShape<LOGN>::T;
+  const u64 q = P.rc.q, q2 = P.rc.q << 1;
+  const int j = threadIdx.x;
+  u64 *own = slots + (t & 1) * N;
+  const u64 *peer = peer_slots + (t & 1) * N;
+  const bool keep_b = (op & OP_KEEPB) != 0;
+  if (op & OP_AUTO) {
+    const u32 k = P.auto_k[op & OP_SLOT];
+    if (op & OP_TRIVIAL) {  // runtime.rs:625-642: only b, permuted in the coefficient domain
+      if (rank == 1) {
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          u32 tt = ((u32)pos_coef<LOGN>(j, r) * k) & (2 * N - 1);
+          const bool neg = tt >= (u32)N;
+          if (neg) tt -= N;
+          sm[swz(tt)] = neg ? q - x[r] : x[r];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 8; r++) x[r] = sm[swz(pos_coef<LOGN>(j, r))];
+      }
+      cl.sync();
+      return;
+    }
+    const u64 *K = P.autos + (size_t)(op & OP_SLOT) * P.auto_rows * N;
+    if (rank == 0) {  // a(X^k) with sign, one digit, forward transform
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        u32 tt = ((u32)pos_coef<LOGN>(j, r) * k) & (2 * N - 1);
+        const bool neg = tt >= (u32)N;
+        if (neg) tt -= N;
+        sm[swz(tt)] = neg ? q - x[r] : x[r];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = decompose1<AUTO_LOGB, AUTO_IGN>(sm[swz(pos_coef<LOGN>(j, r))], q);
+      ntt_fwd<LOGN, false>(x, x, sm, P.rc);
+#pragma unroll
+      for (int r = 0; r < 8; r++) own[r * T + j] = x[r];
+    } else {  // b in the evaluation domain, permuted there
+      u64 *sb = sm + N;
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 8; r++) sb[swz(pos_eval<LOGN>(j, r))] = x[r];
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = sb[swz(auto_eval_src<LOGN>(pos_eval<LOGN>(j, r), k))];
+    }
+    cl.sync();
+    if (rank == 0) {
+      u64 z[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) z[r] = 0;
+      mac_two_rows<LOGN>(x, z, K, K, P.rc);  // a' = d A (second product is 0)
+      ntt_inv<LOGN, false>(x, x, sm, P.rc);
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = reduce2(x[r], q);
+    } else {
+      u64 d[8], z[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        d[r] = peer[r * T + j];
+        z[r] = 0;
+      }
+      mac_two_rows<LOGN>(d, z, K + N, K + N, P.rc);  // d B
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = mac_add_b<LOGN>(d[r] + x[r], q2);
+      if (!keep_b) {
+        ntt_inv<LOGN, false>(x, x, sm, P.rc);
+#pragma unroll
+        for (int r = 0; r < 8; r++) x[r] = reduce2(x[r], q);
+      }
+    }
+    return;
+  }
+  // external product: rows A(-sm), B(-sm), A(m), B(m) (d_a = d_b = 1)
+  const u64 *K = P.rgsw + (size_t)(op & OP_INDEX) * P.rgsw_rows * N;
+#pragma unroll
+  for (int r = 0; r < 8; r++) x[r] = decompose1<RLRG_LOGB, RLRG_IGN>(x[r], q);
+  ntt_fwd<LOGN, false>(x, x, sm, P.rc);
+#pragma unroll
+  for (int r = 0; r < 8; r++) own[r * T + j] = x[r];
+  cl.sync();
+  u64 y[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) y[r] = peer[r * T + j];
+  // rank 0: a' = da A(-sm) + db A(m); rank 1: b' = da B(-sm) + db B(m)
+  if (rank == 0) mac_two_rows<LOGN>(x, y, K, K + 2 * N, P.rc);
+  else {
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      const u64 tmp = x[r];
+      x[r] = y[r];
+      y[r] = tmp;
+    }
+    mac_two_rows<LOGN>(x, y, K + N, K + 3 * N, P.rc);
+  }
+  if (rank == 0 || !keep_b) {
+    ntt_inv<LOGN, false>(x, x, sm, P.rc);
+#pragma unroll
+    for (int r = 0; r < 8; r++) x[r] = reduce2(x[r], q);
+  }
+}
+
+// A plain batch (descs null), or a ragged one as pbs_ragged_kernel's.
+template <int LOGN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NttShape<LOGN>::T, 2)
+    pbs_split_kernel(const __grid_constant__ BrParams P, const BrParams *descs, const u32 *item_desc,
+                     const u32 *out_idx, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
+                     int count) {
+  constexpr int N = 1 << LOGN;
+  extern __shared__ u64 smem[];
+  __shared__ BrParams sp;
+  cg::cluster_group cl = cg::this_cluster();
+  const unsigned rank = cl.block_rank();
+  u64 *slots = smem + 2 * N;
+  const u64 *peer_slots = cl.map_shared_rank(slots, rank ^ 1u);
+  const int j = threadIdx.x;
+  for (int ct = blockIdx.x / 2; ct < count; ct += gridDim.x / 2) {  // both CTAs of a cluster take the same items
+    if (j == 0) {
+      sp = descs ? descs[item_desc[ct]] : P;
+      if (descs) sp.out_idx = out_idx;
+    }
+    __syncthreads();
+    const SchedSmem S = sched_smem<LOGN>(smem, SPLIT_REGIONS, sp.br_q >> 1, sp.n);
+    const u64 q = sp.rc.q;
+    const u32 *kso = ks + (size_t)ct * ks_stride;
+    build_schedule<LOGN>(sp, kso, smem, S);
+    u64 x[8];
+    if (rank == 0) {
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = 0;
+    } else {
+      test_rlwe_b<LOGN>(sp, kso, gates[ct], x);
+    }
+    __syncthreads();
+    const u32 nops = *S.nops;
+#pragma unroll 1
+    for (u32 t = 0; t < nops; t++) {
+      if (j == 0 && t + 1 < nops) prefetch_next_key<LOGN>(sp, S.ops[t + 1]);
+      split_op<LOGN>(x, S.ops[t], t, sp, smem, slots, peer_slots, rank, cl);
+    }
+    // sample extract at index 0 (pbs.rs:423-449): rank 0 the a-part, rank 1 b[0]
+    u64 *o = out + (size_t)(sp.out_idx ? sp.out_idx[ct] : (u32)ct) * (N + 1);
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      const u32 p = (u32)pos_coef<LOGN>(j, r);
+      if (rank == 0) {
+        if (p == 0) o[1] = x[r];
+        else o[1 + N - p] = q - x[r];
+      } else if (p == 0) {
+        o[0] = x[r];
+      }
+    }
+    cl.sync();  // the digit slots and sp are reused by the next ciphertext
+  }
+}
+
 // Throughput probe for the roofline denominator: 8 independent chains of
 // 32-bit multiply-adds per thread (mad.lo.u32, the IMAD the 64-bit modular
 // multiplications are built from).  `sink` keeps the chains live.
@@ -1222,6 +1424,23 @@ cudaError_t launch_ksk_planes(const u32 *ksk, u32 rows, u32 stride, u32 n, u32 p
   return cudaGetLastError();
 }
 
+static bool two_per_sm(size_t count) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return count <= 2 * (size_t)sms;
+}
+
+// Keys without their FFT form, variant PBS_SPLIT: clusters of two CTAs.
+static cudaError_t launch_split(const BrParams &P, const BrParams *descs, const u32 *item_desc, const u32 *out_idx,
+                                u32 br_q, u32 n, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
+                                size_t count, int grid, cudaStream_t s) {
+  const size_t smem = pbs_smem_bytes(11, br_q, n) + (SPLIT_REGIONS - OP_REGIONS) * 2048 * 8;
+  const cudaError_t e = set_smem(pbs_split_kernel<11>, smem);
+  if (e != cudaSuccess) return e;
+  pbs_split_kernel<11><<<2 * grid, 256, smem, s>>>(P, descs, item_desc, out_idx, ks, ks_stride, gates, out, (int)count);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_pbs(int logn, bool d1, const BrParams &P, const u32 *ks, u32 ks_stride,
                        const unsigned char *gates, u64 *out, size_t count, u64 *rlwe_dbg, int grid_limit,
                        cudaStream_t s, int variant) {
@@ -1233,10 +1452,16 @@ cudaError_t launch_pbs(int logn, bool d1, const BrParams &P, const u32 *ks, u32 
   if (logn == 11 && d1 && P.fft_rgsw)
     return launch_pbs_fft(P, ks, ks_stride, gates, out, count, rlwe_dbg, grid, s,
                           variant == PBS_SPLIT && rlwe_dbg == nullptr);
+  if (logn == 11 && d1 && variant == PBS_SPLIT && rlwe_dbg == nullptr)
+    return launch_split(P, nullptr, nullptr, nullptr, P.br_q, P.n, ks, ks_stride, gates, out, count, grid, s);
 #define PZ_LAUNCH(LN, DD, MB, TH)                                                                    \
   if ((e = set_smem(pbs_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;                        \
   pbs_kernel<LN, DD, MB><<<grid, TH, smem, s>>>(P, ks, ks_stride, gates, out, (int)count, rlwe_dbg);
-  if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }  // a key without its FFT form
+  // a key without its FFT form: two CTAs per SM (128 registers) up to 296
+  // ciphertexts, three (80, spilling) above: NI_8P 148 take 13.2 and 14.1 ms, 296
+  // 20.8 and 21.5, 444 31.2 and 30.5
+  if (logn == 11 && d1 && two_per_sm(count)) { PZ_LAUNCH(11, true, 2, 256) }
+  else if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }
   else if (logn == 11) { PZ_LAUNCH(11, false, 1, 256) }
   else if (logn == 9 && d1) { PZ_LAUNCH(9, true, 1, 64) }
   else if (logn == 9) { PZ_LAUNCH(9, false, 1, 64) }
@@ -1311,11 +1536,15 @@ cudaError_t launch_pbs_ragged(int logn, bool d1, const BrParams *d_descs, const 
   if (logn == 11 && d1 && fft)
     return launch_pbs_fft_ragged(d_descs, item_desc, max_br_q, max_n, ks, ks_stride, gates, out, out_idx, count, grid,
                                  s, variant == PBS_SPLIT);
+  if (logn == 11 && d1 && variant == PBS_SPLIT)
+    return launch_split(BrParams{}, d_descs, item_desc, out_idx, max_br_q, max_n, ks, ks_stride, gates, out, count, grid,
+                        s);
 #define PZ_LAUNCH(LN, DD, MB, TH)                                                                    \
   if ((e = set_smem(pbs_ragged_kernel<LN, DD, MB>, smem)) != cudaSuccess) return e;                 \
   pbs_ragged_kernel<LN, DD, MB><<<grid, TH, smem, s>>>(d_descs, item_desc, ks, ks_stride, gates, out, out_idx, \
                                                        (int)count);
-  if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }  // a session's key without its FFT form
+  if (logn == 11 && d1 && two_per_sm(count)) { PZ_LAUNCH(11, true, 2, 256) }  // keys without their FFT form
+  else if (logn == 11 && d1) { PZ_LAUNCH(11, true, 3, 256) }
   else if (logn == 11) { PZ_LAUNCH(11, false, 1, 256) }
   else if (logn == 9 && d1) { PZ_LAUNCH(9, true, 1, 64) }
   else if (logn == 9) { PZ_LAUNCH(9, false, 1, 64) }

@@ -42,7 +42,7 @@ def test_gates_and_rotations(gpu_available, param):
         return to_host(out)
 
     want = rotate(fast, 451)
-    for count, limit in [(1, 0), (75, 0), (451, 0), (13, 3)]:
+    for count, limit in [(1, 0), (74, 0), (75, 0), (296, 0), (297, 0), (451, 0), (13, 3), (90, 5)]:  # to 74 on two SMs each
         assert np.array_equal(rotate(slow, count, limit), want[:count]), (count, limit)
     blob = slow.export()
     assert blob == fast.export()
