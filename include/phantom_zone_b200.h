@@ -516,17 +516,24 @@ pz_status pz_server_add_virtual_session(pz_server *s, int param_id, uint32_t *se
 /* Managed session: the server holds the session's device key only while it
  * is needed, importing it from the caller's device-form blob (pz_key_export;
  * the blob must stay valid and unchanged while the server exists).  A job of
- * a managed session is admitted when its key is resident or fits the key
- * budget after evicting the least recently used resident managed keys of
- * sessions with no job in flight (import: a plain host-to-device copy of the
- * blob); otherwise it waits, in arrival order.  A job whose key alone exceeds
- * the budget fails (state 3).  No reference counterpart (the reference holds
- * one server key per process, bool/mp_api.rs:128-146). */
+ * a managed session is admitted when its key is resident or can be within the
+ * key budget; otherwise it waits, in arrival order.  A managed key holds what
+ * the server's launches read: of the LWE KSK its byte planes, and of the RGSW and
+ * automorphism keys the FFT form (NI_8P: 190 MB in all) or the integer form
+ * (102 MB; the exported blob has 121).  Room is made by taking the FFT form of
+ * the least recently used keys back to the integer one first, then by evicting
+ * the keys of sessions with no job in flight; a key comes in, or gets its FFT
+ * form later, over FFTs where the budget has room (import: a host-to-device copy
+ * of the blob, its forms made on the device).  A job whose key's integer form
+ * exceeds the budget fails (state 3).  A dry run counts exported bytes.  No
+ * reference counterpart (the reference holds one server key per process,
+ * bool/mp_api.rs:128-146). */
 pz_status pz_server_add_managed_session(pz_server *s, pz_ctx *ctx, const void *key_blob, size_t blob_bytes,
                                         uint32_t *session);
 /* dry-run servers only: a managed session of param_id (residency bookkeeping only) */
 pz_status pz_server_add_virtual_managed_session(pz_server *s, int param_id, uint32_t *session);
-/* Device bytes resident managed keys may hold (0: no limit, the default). */
+/* Device bytes resident managed keys may hold (0: no limit, the default);
+ * resident_key_bytes of the statistics is what they and the other sessions' hold. */
 pz_status pz_server_set_key_budget(pz_server *s, size_t bytes);
 /* *resident = 1 when the session's key is on the device now. */
 pz_status pz_server_session_resident(pz_server *s, uint32_t session, int *resident);

@@ -96,6 +96,18 @@ cudaError_t build_fft_key(pz_ctx *c, pz_key *k, cudaStream_t s);
 // both; any failure but lack of memory is one of the caller's
 cudaError_t build_key_forms(pz_ctx *c, pz_key *k, cudaStream_t s);
 void free_key_arrays(pz_key *k);
+size_t ksk8_bytes(const pz_ctx *c);  // of the byte planes (0: the set has none)
+// The keys that a server imports and releases by itself hold only what its
+// launches read: of the KSK its byte planes (the u32 rows where there are none),
+// and of the RGSW and automorphism keys the FFT form or, in less memory, the
+// integer one (`fft` and `least` device bytes; equal without an FFT form).
+struct ManagedBytes {
+  size_t least, fft;
+};
+ManagedBytes managed_key_bytes(const pz_ctx *c);
+pz_status managed_import(pz_ctx *c, const void *blob, size_t size, bool fft, pz_key **out);
+pz_status managed_to_integer(pz_key *k, const void *blob);  // ... and give the FFT form back
+pz_status managed_to_fft(pz_key *k);                        // (unchanged without the memory)
 // BrParams of context c bound to key k (both key forms; k null: no key)
 void br_bind_key(const pz_ctx *c, const pz_key *k, BrParams &br);
 // KsParams of context c bound to key k (both KSK forms)

@@ -289,12 +289,18 @@ static cudaError_t derive(void **p, size_t bytes, cudaStream_t s, const Launch &
   return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
 }
 
-cudaError_t build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s) {
+size_t ksk8_bytes(const pz_ctx *c) {
   const pz_params &P = c->P;
   const u32 rows = P.lwe_d * P.rlwe_n;
-  if (k->d_ksk8 || !k->d_ksk || rows % 32 || P.rlwe_n % 32 || P.lwe_d > 16 || P.lwe_logb > 7) return cudaSuccess;
-  const u32 planes = ksk8_planes(c->ks.mask), cols = ksk8_cols(P.lwe_n);
-  const size_t bytes = (size_t)planes * rows * cols;
+  if (rows % 32 || P.rlwe_n % 32 || P.lwe_d > 16 || P.lwe_logb > 7) return 0;
+  return (size_t)ksk8_planes(c->ks.mask) * rows * ksk8_cols(P.lwe_n);
+}
+
+cudaError_t build_ksk8(pz_ctx *c, pz_key *k, cudaStream_t s) {
+  const pz_params &P = c->P;
+  const size_t bytes = ksk8_bytes(c);
+  if (k->d_ksk8 || !k->d_ksk || !bytes) return cudaSuccess;
+  const u32 rows = P.lwe_d * P.rlwe_n, planes = ksk8_planes(c->ks.mask);
   const cudaError_t e = derive((void **)&k->d_ksk8, bytes, s, [&] {
     return launch_ksk_planes(k->d_ksk, rows, ks_stride(P), P.lwe_n, planes, k->d_ksk8, s);
   });

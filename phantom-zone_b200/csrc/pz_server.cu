@@ -56,10 +56,11 @@ struct pz_server {
     pz_ctx *ctx = nullptr;
     const pz_key *key = nullptr;  // the device key while resident (null: not resident)
     int param_id = 0;
-    size_t key_bytes = 0;
+    size_t key_bytes = 0;  // device bytes of the key: held, or (managed, not resident) the least it can do with
     // managed: the server owns the device key, imported from the caller's
     // blob (the pz_key_export form) when a job needs it, released on eviction
     bool managed = false;
+    pz::ManagedBytes need{};  // device bytes with the integer form and with the FFT form
     const void *blob = nullptr;
     size_t blob_bytes = 0;
     pz_key *owned = nullptr;
@@ -223,6 +224,7 @@ struct pz_server {
 
 namespace {
 
+// bytes of a key as exported; what a dry run charges for it
 size_t key_bytes_of(const pz_params &P) {
   // RGSW + auto keys (u64, device form) + KSK (u32 rows of ks_stride words)
   return (size_t)P.lwe_n * P.rgsw_rows * P.rlwe_n * 8 + (size_t)P.n_auto_keys * P.auto_rows * P.rlwe_n * 8 +
@@ -278,7 +280,8 @@ pz_status add_session_common(pz_server *s, int param_id, pz_ctx *ctx, const pz_k
   se.ctx = ctx;
   se.key = key;
   se.param_id = param_id;
-  se.key_bytes = key ? key->bytes : key_bytes_of(P);
+  se.need = managed && !s->dry ? pz::managed_key_bytes(ctx) : pz::ManagedBytes{key_bytes_of(P), key_bytes_of(P)};
+  se.key_bytes = key ? key->bytes : se.need.least;
   se.managed = managed;
   se.blob = blob;
   se.blob_bytes = blob_bytes;
@@ -317,38 +320,102 @@ void evict(pz_server *s, pz_server::Session &se) {
   se.key = nullptr;
   se.virt_resident = false;
   s->managed_bytes -= se.key_bytes;
+  se.key_bytes = se.need.least;
   s->key_evictions++;
   s->descs_dirty = true;
 }
 
-// Make the key of session `sid` resident: evict the least recently used
-// resident managed keys of sessions without jobs in flight until it fits the
-// budget, then import it.  *fits = false: not now (the keys in the way are
-// pinned by running jobs); a CUDA or blob error is returned as such.
+// a managed key's forms changed: its bytes, and the total, with them
+void recharge(pz_server *s, pz_server::Session &se) {
+  s->managed_bytes -= se.key_bytes;
+  se.key_bytes = se.owned->bytes;
+  s->managed_bytes += se.key_bytes;
+  s->descs_dirty = true;
+}
+
+// The running jobs of a session whose key is lost.
+void fail_active(pz_server *s, u32 session) {
+  std::vector<pz_server::Job *> still;
+  for (auto *j : s->active) {
+    if (j->session != session) {
+      still.push_back(j);
+      continue;
+    }
+    j->state = 3;
+    j->t_done = now_ms();
+    s->release(j->base, j->slots);
+    s->n_failed++;
+  }
+  s->sessions[session].jobs_in_flight = 0;
+  s->active.swap(still);
+}
+
+// Make room among the resident managed keys (other than that of `but`), least
+// recently used and idle ones first: an FFT form back to the integer one, which
+// runs the same jobs 1.4 to 1.8 times slower, and only then, where `evictions`, a
+// whole key of a session without jobs in flight.  *made = false: nothing left.
+pz_status make_room(pz_server *s, const pz_server::Session *but, bool evictions, bool *made) {
+  auto least_recent = [&](auto eligible) {
+    pz_server::Session *v = nullptr;
+    for (auto &o : s->sessions)
+      if (&o != but && o.managed && s->resident(o) && eligible(o) &&
+          (!v || std::make_pair(o.jobs_in_flight > 0, o.last_use) < std::make_pair(v->jobs_in_flight > 0, v->last_use)))
+        v = &o;
+    return v;
+  };
+  *made = true;
+  if (pz_server::Session *o = least_recent([](auto &x) { return x.owned && x.owned->d_fft_rgsw; })) {
+    const pz_status st = pz::managed_to_integer(o->owned, o->blob);
+    recharge(s, *o);
+    if (st != PZ_OK) {  // it has neither form now
+      fail_active(s, (u32)(o - s->sessions.data()));
+      evict(s, *o);
+      return s->fail(st, std::string("managed session key: ") + pz_last_error(o->ctx));
+    }
+    return PZ_OK;
+  }
+  if (pz_server::Session *o = evictions ? least_recent([](auto &x) { return x.jobs_in_flight == 0; }) : nullptr) {
+    evict(s, *o);
+    return PZ_OK;
+  }
+  *made = false;
+  return PZ_OK;
+}
+
+// Make the key of session `sid` resident: make room for its integer form within
+// the budget, then import it, over FFTs where that fits too (a key that came in
+// without gets its FFT form once it fits).  *fits = false: not now (the keys in the
+// way are pinned by running jobs); a CUDA or blob error is returned as such.
 pz_status make_resident(pz_server *s, u32 sid, bool *fits) {
   pz_server::Session &se = s->sessions[sid];
   *fits = true;
-  if (s->resident(se)) return PZ_OK;
-  while (s->managed_bytes + se.key_bytes > s->key_budget) {
-    pz_server::Session *victim = nullptr;
-    for (auto &o : s->sessions)
-      if (&o != &se && o.managed && s->resident(o) && o.jobs_in_flight == 0 &&
-          (!victim || o.last_use < victim->last_use))
-        victim = &o;
-    if (!victim) {
-      *fits = false;
+  if (s->resident(se)) {
+    if (!se.owned || se.owned->d_fft_rgsw || se.need.fft == se.need.least ||
+        s->managed_bytes - se.key_bytes + se.need.fft > s->key_budget)
       return PZ_OK;
-    }
-    evict(s, *victim);
+    const pz_status st = pz::managed_to_fft(se.owned);
+    recharge(s, se);
+    return st == PZ_OK ? st : s->fail(st, std::string("managed session key: ") + pz_last_error(se.ctx));
+  }
+  while (s->managed_bytes + se.need.least > s->key_budget) {
+    const pz_status st = make_room(s, &se, true, fits);
+    if (st != PZ_OK || !*fits) return st;
   }
   if (s->dry) {
     se.virt_resident = true;
   } else {
     pz_key *k = nullptr;
-    pz_status st = pz_key_import(se.ctx, se.blob, se.blob_bytes, &k);
+    const bool fft = s->managed_bytes + se.need.fft <= s->key_budget;
+    pz_status st = pz::managed_import(se.ctx, se.blob, se.blob_bytes, fft, &k);
+    for (bool made = true; st == PZ_ERR_OUT_OF_MEMORY && made;) {  // of the device: others' FFT forms make room
+      const pz_status r = make_room(s, &se, false, &made);
+      if (r != PZ_OK) return r;
+      if (made) st = pz::managed_import(se.ctx, se.blob, se.blob_bytes, false, &k);
+    }
     if (st != PZ_OK) return s->fail(st, std::string("managed session key import: ") + pz_last_error(se.ctx));
     se.owned = k;
     se.key = k;
+    se.key_bytes = k->bytes;
   }
   s->managed_bytes += se.key_bytes;
   s->key_imports++;
@@ -380,23 +447,19 @@ pz_status ensure_device_buffers(pz_server *s) {
 }
 
 // Admit pending jobs in arrival order while their wires fit the arena and
-// their session's key is (or can be made) resident.  Resident managed keys
-// over the budget (it may have been lowered) are evicted first, least
-// recently used idle ones, as far as idle ones go.
+// their session's key is (or can be made) resident.  While the resident managed
+// keys are over the budget (it may have been lowered), room is made first, as far
+// as that goes.
 pz_status admit(pz_server *s) {
-  while (s->managed_bytes > s->key_budget) {
-    pz_server::Session *victim = nullptr;
-    for (auto &o : s->sessions)
-      if (o.managed && s->resident(o) && o.jobs_in_flight == 0 && (!victim || o.last_use < victim->last_use))
-        victim = &o;
-    if (!victim) break;
-    evict(s, *victim);
+  for (bool made = true; made && s->managed_bytes > s->key_budget;) {
+    const pz_status st = make_room(s, nullptr, true, &made);
+    if (st != PZ_OK) return st;
   }
   while (!s->pending.empty()) {
     pz_server::Job *j = s->pending.front();
     const size_t need = j->v.n_inputs + j->v.n_gates;
     pz_server::Session &se = s->sessions[j->session];
-    if (need > s->arena_slots || (se.managed && se.key_bytes > s->key_budget)) {  // can never fit
+    if (need > s->arena_slots || (se.managed && se.need.least > s->key_budget)) {  // can never fit
       fail_job(s, j);
       continue;
     }

@@ -260,3 +260,70 @@ def test_staged_key_ragged_shape(gpu_available, grid_limit):
         assert np.array_equal(got, C.run(eng, key, inp)), f"{p} {op}: words differ from the job alone"
         expect(op, ev, s, got, x, y)
     assert session("NI_8P")[0].device_error() == 0
+
+
+def test_managed_keys_stay_within_the_budget(gpu_available):
+    """What the resident managed keys hold is what the statistics say, what the
+    device lost, and never more than the budget: without one they run over FFTs;
+    a lower one takes them back to the integer form before any is evicted, also
+    while their jobs run; a higher one brings the FFT form back.  Every job gives
+    the words that it has alone."""
+    import torch
+    P = pz()
+    eng, key, ev, s, _ = session("I_2P_LB_SR")
+    blob = key.export()
+    p = eng.p
+    exported = len(blob) - 64
+    rows = (p.lwe_n * p.rgsw_rows + p.n_auto_keys * p.auto_rows) * p.rlwe_n * 8
+    planes = key.device_bytes - exported - (p.lwe_n + p.n_auto_keys) * 196608
+    integer, fft = rows + planes, (p.lwe_n + p.n_auto_keys) * 196608 + planes
+    assert integer <= exported < fft
+    S = P.Server(device=0, arena_bytes=1 << 27, max_items=1024)
+    sids = [S.add_managed_session(eng, blob) for _ in range(3)]
+    C = circuit("lt")
+    count = [0]
+
+    def submit(sid):
+        count[0] += 1
+        inp = enc_pair(ev, s, 11 * count[0], 200 - 7 * count[0], 90 + count[0])
+        return S.submit(sid, C, inp), C.run(eng, key, inp)
+
+    def finish(jobs):
+        while S.stats()["pending"] or S.stats()["active"]:
+            S.step()
+            st = S.stats()
+            assert not st["key_budget"] or st["resident_key_bytes"] <= st["key_budget"]
+        for j, want in jobs:
+            assert np.array_equal(S.result(j), want)
+
+    def held():
+        st = S.stats()
+        return st["resident_key_bytes"], [S.resident(x) for x in sids], st["key_evictions"]
+
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    finish([submit(x) for x in sids])
+    assert held() == (3 * fft, [True] * 3, 0)
+    assert abs((free - torch.cuda.mem_get_info()[0]) - 3 * fft) < (16 << 20)  # allocations come in 2 MB pages
+    jobs = [submit(x) for x in sids]
+    S.step()
+    S.set_key_budget(2 * fft + integer)  # all in flight: one goes back to integers
+    finish(jobs)
+    assert held() == (2 * fft + integer, [True] * 3, 0)
+    S.set_key_budget(3 * exported)
+    finish([submit(sids[1])])
+    resident, where, evictions = held()
+    assert where == [True] * 3 and evictions == 0
+    S.set_key_budget(2 * exported)  # as many keys as their exported forms would be
+    finish([submit(sids[1])])
+    assert held() == (2 * integer, [False, True, True], 1)
+    finish([submit(sids[0])])
+    assert held() == (2 * integer, [True, True, False], 2)
+    S.set_key_budget(0)
+    finish([submit(sids[1])])
+    assert held() == (integer + fft, [True, True, False], 2)
+    S.set_key_budget(integer - 1)
+    j, _ = submit(sids[0])
+    S.step()
+    assert S.status(j)["state"] == P.server.FAILED
+    assert eng.device_error() == 0
