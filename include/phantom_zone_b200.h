@@ -106,6 +106,13 @@ typedef struct pz_server_key_view {
 
 const char *pz_status_string(pz_status s);
 pz_status pz_param_get(int param_id, pz_params *out);
+/* Calls that take device scratch (non-interactive inputs, aggregation, key
+ * switches) keep up to 2 GiB of it per device for the next call, for as long as
+ * the device has a context.  This gives back what is not in use, down to `keep`
+ * bytes (0: all); synchronize first for scratch of work still running.  The
+ * library's own allocations do it by themselves when memory is short.  No
+ * reference counterpart. */
+pz_status pz_scratch_trim(int device, size_t keep);
 
 /* Context: parameter set + device tables + a private stream.  ntt_root = 0
  * selects the library's own 2N-th root of unity; a nonzero value must be a

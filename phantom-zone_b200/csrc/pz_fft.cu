@@ -754,7 +754,7 @@ cudaError_t fft_tables(void **out) {
     }
   }
   void *d = nullptr;
-  cudaError_t e = cudaMalloc(&d, h.size() * 8);
+  cudaError_t e = dev_malloc(&d, h.size() * 8);
   if (e == cudaSuccess) e = cudaMemcpy(d, h.data(), h.size() * 8, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(d);

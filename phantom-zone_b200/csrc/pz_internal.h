@@ -74,6 +74,7 @@ namespace pz {
 constexpr size_t POOL_KEEP = (size_t)2 << 30;
 cudaError_t pool_acquire(int device);
 void pool_release(int device);
+cudaError_t pool_trim(int device, size_t keep);  // what is not in use, down to `keep` bytes
 cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t st);  // on the current device
 template <typename T>
 cudaError_t pool_malloc(T **p, size_t bytes, cudaStream_t st) {

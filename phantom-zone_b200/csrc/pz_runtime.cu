@@ -146,6 +146,11 @@ void pool_release(int device) {
     d.pool = nullptr;
   }
 }
+cudaError_t pool_trim(int device, size_t keep) {
+  if (device < 0 || device >= MAX_POOLS) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(pool_mu);
+  return pools[device].pool ? cudaMemPoolTrimTo(pools[device].pool, keep) : cudaSuccess;
+}
 static cudaMemPool_t current_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_POOLS) return nullptr;
@@ -421,6 +426,11 @@ pz_status pz_param_get(int id, pz_params *out) {
   if (id < 0 || id >= PZ_NUM_PARAMS || !out) return PZ_ERR_INVALID_ARGUMENT;
   *out = full_params(id);
   return PZ_OK;
+}
+
+pz_status pz_scratch_trim(int device, size_t keep) {
+  if (device < 0 || cudaSetDevice(device) != cudaSuccess) return PZ_ERR_INVALID_ARGUMENT;
+  return pz::pool_trim(device, keep) == cudaSuccess ? PZ_OK : PZ_ERR_CUDA;
 }
 
 pz_status pz_ctx_create(int id, int device, pz_ctx **out) { return pz_ctx_create_ex(id, device, 0, out); }

@@ -64,6 +64,12 @@ def kernel_revision():
     return lib().pz_kernel_revision().decode()
 
 
+def trim_scratch(device=0, keep=0):
+    """Give back the device scratch kept between calls (up to 2 GiB), down to
+    `keep` bytes; synchronize first for scratch of work still running."""
+    check(lib().pz_scratch_trim(int(device), int(keep)), None, "pz_scratch_trim")
+
+
 def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
 

@@ -82,3 +82,13 @@ def test_interactive_crs_seeds_host_matches_oracle():
     crs = bytes(range(5, 37))
     for what in range(3):
         assert pz().engine.interactive_crs_seed(crs, what) == O.interactive_crs_seed(crs, what)
+
+
+def test_every_device_allocation_can_have_the_scratch_back():
+    """Device memory is asked for through dev_malloc, which gives back the scratch
+    kept between calls when there is none left, and stream-ordered scratch through
+    the library's own pool."""
+    text = "".join(open(f).read() for f in glob.glob(os.path.join(ROOT, "phantom-zone_b200", "csrc", "*.cu*")))
+    body = re.search(r"cudaError_t dev_malloc\(void \*\*p, size_t bytes\) \{.*?\n\}", text, re.S).group(0)
+    assert len(re.findall(r"\bcudaMalloc\(", text)) == len(re.findall(r"\bcudaMalloc\(", body)) == 2
+    assert len(re.findall(r"\bcudaMallocAsync\(", text)) == 1  # pool_malloc's, without a pool
