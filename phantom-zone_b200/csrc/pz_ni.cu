@@ -116,41 +116,73 @@ __global__ void seeded_place_kernel(const u64 *samples, const unsigned char *acc
   }
 }
 
+// Row c of a batch, LWE i of the RLWE at x: 16-byte stores from the row's first
+// 16-byte boundary (rows are N + 1 words, so every other one starts off it).
+template <class Load>
+__device__ __forceinline__ void extract_row(const u64 *x, u32 i, u64 *o, u64 q, const Load &load) {
+  constexpr int N = 1 << NI_LOGN;
+  const int k = (int)(i % N);
+  const int first = ((size_t)o & 8) ? 1 : 0;
+  auto word = [&](int t) -> u64 {
+    if (t == 0) return load(x + N + k);
+    return t - 1 <= k ? load(x + k + 1 - t) : q - load(x + N + k + 1 - t);  // neg = q - x (modulus_u64.rs:147-149)
+  };
+  if (threadIdx.x == 0) o[first ? 0 : N] = word(first ? 0 : N);
+#pragma unroll
+  for (int p = 0; p < N / 512; p++) {
+    const int t = first + 2 * (threadIdx.x + 256 * p);
+    *(ulonglong2 *)(o + t) = make_ulonglong2(word(t), word(t + 1));
+  }
+}
+
 // out[c] = sample_extract(rlwe[idx[c] / N], idx[c] % N); an index past the
-// batch leaves out[c] unchanged.  Bound by the writes (16 KB per bool): a CTA
-// takes EXTRACT_RUN entries in a row, keeps their RLWE in shared memory while it
-// stays the same, and stores 16 bytes per thread from the row's first 16-byte
-// boundary (rows are N + 1 words, so every other one starts off it).  49,152
-// bools of 24 RLWEs: 160 -> 129 us (6.2 TB/s).
-constexpr int EXTRACT_RUN = 8;
+// batch leaves out[c] unchanged.  Bound by the writes (16 KB per bool).  One entry to
+// a CTA; CTAs that run together take entries a 148th of the batch apart, since many
+// SMs reading the same 32 KB of L2 at once (a batch in order) are slower than each
+// its own: 9,472 entries in order 28 us (32 with neighbours together, 36 with
+// 8-byte stores besides), shuffled 30 (37).
+constexpr u32 EXTRACT_APART = 148;
 __global__ void __launch_bounds__(256)
     extract_kernel(const u64 *rlwe, size_t rlwe_count, const u32 *idx, u64 *out, size_t count, u64 q) {
   constexpr int N = 1 << NI_LOGN;
-  __shared__ u64 ab[2 * N];  // a, b
-  size_t have = rlwe_count;  // the RLWE in ab
+  const size_t per = (count + EXTRACT_APART - 1) / EXTRACT_APART;
+  for (size_t b = blockIdx.x; b < per * EXTRACT_APART; b += gridDim.x) {
+    const size_t c = b % EXTRACT_APART * per + b / EXTRACT_APART;
+    const u32 i = c < count ? idx[c] : 0;
+    if (c >= count || i / N >= rlwe_count) continue;  // uniform over the CTA
+    extract_row(rlwe + (size_t)(i / N) * 2 * N, i, out + c * (size_t)(N + 1), q, [](const u64 *p) { return __ldg(p); });
+  }
+}
+
+// The same for large batches: EXTRACT_RUN entries in a row to a CTA, which reads
+// their RLWE once, into shared memory, when they are all of one.  From 256 entries
+// per SM on, where the writes have to reach HBM in step with the kernels and are
+// the faster for being in order: 24 RLWEs unseeded, switched and extracted in a row
+// of calls 210 us against 213 (48: 346 and 357; 18: 177 and 176), by themselves 129
+// us either way, shuffled 149 against 131 (160 with 8-byte stores).
+constexpr int EXTRACT_RUN = 8;
+__global__ void __launch_bounds__(256)
+    extract_runs_kernel(const u64 *rlwe, size_t rlwe_count, const u32 *idx, u64 *out, size_t count, u64 q) {
+  constexpr int N = 1 << NI_LOGN;
+  __shared__ u64 ab[2 * N];  // a, b of the run's RLWE
   for (size_t c0 = (size_t)blockIdx.x * EXTRACT_RUN; c0 < count; c0 += (size_t)gridDim.x * EXTRACT_RUN) {
-    for (size_t c = c0; c < c0 + EXTRACT_RUN && c < count; c++) {
-      const u32 i = idx[c];
-      const size_t ct = i / N;
-      const int k = (int)(i % N);
-      if (ct >= rlwe_count) continue;  // uniform over the CTA
-      if (ct != have) {
-        __syncthreads();  // the last RLWE has been read
-        for (int t = threadIdx.x; t < 2 * N; t += 256) ab[t] = rlwe[ct * 2 * N + t];
-        __syncthreads();
-        have = ct;
-      }
-      auto word = [&](int t) -> u64 {
-        if (t == 0) return ab[N + k];
-        return t - 1 <= k ? ab[k + 1 - t] : q - ab[N + k + 1 - t];  // neg = q - x (modulus_u64.rs:147-149)
-      };
-      u64 *o = out + c * (size_t)(N + 1);
-      const int first = ((size_t)o & 8) ? 1 : 0;  // the row's words up to a 16-byte boundary
-      if (threadIdx.x == 0) o[first ? 0 : N] = word(first ? 0 : N);
+    bool one = idx[c0] / N < rlwe_count;  // uniform over the CTA
 #pragma unroll
-      for (int p = 0; p < N / 512; p++) {
-        const int t = first + 2 * (threadIdx.x + 256 * p);
-        *(ulonglong2 *)(o + t) = make_ulonglong2(word(t), word(t + 1));
+    for (int r = 1; r < EXTRACT_RUN; r++) one = one && (c0 + r >= count || idx[c0 + r] / N == idx[c0] / N);
+    if (one) {
+      __syncthreads();  // the last RLWE has been read
+      const u64 *src = rlwe + (size_t)(idx[c0] / N) * 2 * N;
+      for (int t = threadIdx.x; t < 2 * N; t += 256) ab[t] = src[t];
+      __syncthreads();
+      for (size_t c = c0; c < c0 + EXTRACT_RUN && c < count; c++)
+        extract_row(ab, idx[c], out + c * (size_t)(N + 1), q, [](const u64 *p) { return *p; });
+    } else {
+#pragma unroll 2
+      for (int r = 0; r < EXTRACT_RUN; r++) {
+        const u32 i = c0 + r < count ? __ldg(idx + c0 + r) : 0;
+        if (c0 + r < count && i / N < rlwe_count)
+          extract_row(rlwe + (size_t)(i / N) * 2 * N, i, out + (c0 + r) * (size_t)(N + 1), q,
+                      [](const u64 *p) { return __ldg(p); });
       }
     }
   }
@@ -401,13 +433,18 @@ pz_status pz_sample_extract_device(pz_ctx *c, const uint64_t *d_rlwe, size_t rlw
   if (count && (!d_rlwe || !d_index || !d_lwe)) return pz::fail(c, PZ_ERR_INVALID_ARGUMENT, "NULL argument");
   if (count == 0) return PZ_OK;
   PZ_CK(c, cudaSetDevice(c->device));
-  if (c->logn != NI_LOGN) {
-    extract_any_kernel<<<grid_of(count, 65535), 256, 0, (cudaStream_t)stream>>>(d_rlwe, rlwe_count, d_index, d_lwe,
-                                                                                count, c->P.rlwe_n, c->P.rlwe_q);
-  } else {
-    extract_kernel<<<grid_of((count + EXTRACT_RUN - 1) / EXTRACT_RUN, 65535), 256, 0, (cudaStream_t)stream>>>(
+  cudaStream_t st = (cudaStream_t)stream;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  if (c->logn != NI_LOGN)
+    extract_any_kernel<<<grid_of(count, 65535), 256, 0, st>>>(d_rlwe, rlwe_count, d_index, d_lwe, count, c->P.rlwe_n,
+                                                              c->P.rlwe_q);
+  else if (count >= (size_t)256 * sms)
+    extract_runs_kernel<<<grid_of((count + EXTRACT_RUN - 1) / EXTRACT_RUN, 65535), 256, 0, st>>>(
         d_rlwe, rlwe_count, d_index, d_lwe, count, c->P.rlwe_q);
-  }
+  else
+    extract_kernel<<<grid_of((count + EXTRACT_APART - 1) / EXTRACT_APART * EXTRACT_APART, 65535), 256, 0, st>>>(
+        d_rlwe, rlwe_count, d_index, d_lwe, count, c->P.rlwe_q);
   PZ_CK(c, cudaGetLastError());
   return PZ_OK;
 }

@@ -257,3 +257,32 @@ def test_resident_ciphertexts_of_each_shape(gpu_available, param):
     eng = pz().Engine(param)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert [eng.pbs_slots(v) for v in range(5)] == [4 * sms, 4 * sms, 4 * sms, sms // 2, 4 * sms]
+
+
+@pytest.mark.parametrize("count", [1, 147, 148, 149, 2961, 37887, 37888, 37893])
+@pytest.mark.parametrize("order", ["in order", "shuffled", "runs"])
+def test_sample_extract_of_many(gpu_available, order, count):
+    """Batches around the distance at which CTAs take entries, and around the size
+    from which they take several in a row (in order; shuffled; in runs of one RLWE
+    with indices past the batch between them), against the definition."""
+    import torch
+    eng = pz().Engine("NI_2P")
+    N, Q = eng.N, eng.Q
+    g = np.random.default_rng(47)
+    rl = to_dev(g.integers(0, Q, (6, 2, N), dtype=np.uint64))
+    idx = np.arange(count) % (6 * N)
+    if order == "shuffled":
+        idx = g.permutation(6 * N)[idx]
+    if order == "runs":
+        idx = np.arange(count) // 5 % 6 * N + g.integers(0, N, count)
+        idx[7::29], idx[8::40], idx[count - 1] = 6 * N, 6 * N + 3, 0xffffffff
+    out = torch.full((count, N + 1), 5, dtype=torch.int64, device="cuda")
+    eng.sample_extract_device(rl, to_dev(idx.astype(np.uint32)), out)
+    col = torch.arange(N, device="cuda")
+    for at in range(0, count, 1000):
+        i = torch.from_numpy(idx[at:at + 1000].astype(np.int64)).cuda()
+        there = i < 6 * N
+        x, k = rl[torch.where(there, i // N, 0)], (i % N)[:, None]
+        low = torch.gather(x[:, 0], 1, (k - col) % N)  # a_k .. a_0, then a_{N-1} .. a_{k+1}
+        want = torch.cat([torch.gather(x[:, 1], 1, k), torch.where(col <= k, low, Q - low)], 1)
+        assert torch.equal(out[at:at + 1000], torch.where(there[:, None], want, 5))
