@@ -875,6 +875,19 @@ static cudaError_t launch_fft(const Batch &b, size_t count, int grid, bool split
   return launch_form(over <= half ? fft::SPLIT : fft::TRIO, b, whole, count, (int)over, s);
 }
 
+// By the table above, full rounds of QUAD take 0.048 ms per ciphertext.  What fills
+// up places for less is worth adding: to 148 (from 74 on two SMs 0.041), from
+// there to 296 (0.056, but 148 to 222 0.074), from 296 to 592 (0.045), and above
+// whole rounds to 148 (0.058; 74 on two SMs 0.076).  The integer kernels: rounds of
+// three per SM, and whole SMs below.
+size_t pbs_fill(size_t count, size_t sms, bool fft) {
+  auto up = [](size_t x, size_t step) { return std::max<size_t>(1, (x + step - 1) / step) * step; };
+  const size_t round = (fft ? 4 : 3) * sms;
+  if (count <= (fft ? 2 * sms : round)) return up(count, sms);
+  const size_t over = count % round;
+  return fft && count > round && over > 0 && over <= sms ? count - over + sms : up(count, round);
+}
+
 cudaError_t launch_pbs_fft(const BrParams &P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
                            size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split) {
   const Batch b{P, nullptr, nullptr, nullptr, ks, ks_stride, gates, out, rlwe_dbg, P.br_q, P.n};

@@ -128,6 +128,9 @@ cudaError_t launch_fft_key(const u64 *rows, u32 rows_per_key, size_t keys, const
                            void *out, cudaStream_t s);
 cudaError_t launch_pbs_fft(const BrParams &P, const u32 *ks, u32 ks_stride, const unsigned char *gates, u64 *out,
                            size_t count, u64 *rlwe_dbg, int grid, cudaStream_t s, bool split);
+// How many ciphertexts a blind rotation of `count` is best filled up to where more
+// are waiting, with the FFT form or without.
+size_t pbs_fill(size_t count, size_t sms, bool fft);
 cudaError_t pbs_fft_per_sm(u32 br_q, u32 n, int *ctas);  // resident CTAs per SM (as four ciphertexts)
 cudaError_t pbs_fft_clusters(u32 br_q, u32 n, size_t *clusters);  // resident clusters of the two-SM form
 cudaError_t launch_pbs_fft_ragged(const BrParams *d_descs, const u32 *item_desc, u32 max_br_q, u32 max_n, const u32 *ks,

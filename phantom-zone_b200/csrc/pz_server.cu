@@ -548,12 +548,11 @@ pz_status run_items(pz_server *s, const std::vector<Item> &items) {
 // The jobs that advance one level this step.  PZ_SCHEDULE_ALL_READY: every
 // admitted job with a level left.  PZ_SCHEDULE_CRITICAL_PATH: the jobs with
 // the most levels left always advance (they set the number of steps the
-// batch needs); the others, most levels left first, fill the step only up to
-// the launch-time tier the mandatory gates already pay for -- one CTA per SM,
-// two, ... up to the variant's CTAs per SM, then whole waves -- so work with
-// slack moves into steps that would otherwise leave SMs idle.  A job waits
-// at most until its remaining depth is the largest, so the batch still ends
-// after (deepest circuit) steps.
+// batch needs); the others, most levels left first, fill the step up to where
+// another gate would cost more than in full rounds (pbs_fill, from the blind
+// rotation's own placing rule), so work with slack moves into steps that would
+// otherwise leave SMs idle.  A job waits at most until its remaining depth is the
+// largest, so the batch still ends after (deepest circuit) steps.
 size_t level_width(const pz_server::Job *j) { return j->v.level_off[j->level + 1] - j->v.level_off[j->level]; }
 
 void select_jobs(pz_server *s, std::vector<pz_server::Job *> &run) {
@@ -578,9 +577,9 @@ void select_jobs(pz_server *s, std::vector<pz_server::Job *> &run) {
     }
   }
   const size_t sms = (size_t)std::max(1, s->sm_count);
-  const size_t cps = (s->pbs_variant == 0 || s->pbs_variant == 4) ? 2 : s->pbs_variant == 2 ? 4 : 3;
-  const size_t wave = sms * cps;
-  const size_t cap = g <= wave ? std::max<size_t>(1, (g + sms - 1) / sms) * sms : (g + wave - 1) / wave * wave;
+  bool fft = false;  // (a dry run has no keys: the integer kernels' rule)
+  for (auto *j : run) fft = fft || s->kind(s->sessions[j->session]).fft;
+  const size_t cap = pz::pbs_fill(g, sms, fft);
   std::stable_sort(opt.begin(), opt.end(), [](const pz_server::Job *a, const pz_server::Job *b) {
     return a->v.levels - a->level > b->v.levels - b->level;
   });

@@ -327,3 +327,40 @@ def test_managed_keys_stay_within_the_budget(gpu_available):
     S.step()
     assert S.status(j)["state"] == P.server.FAILED
     assert eng.device_error() == 0
+
+
+def test_critical_path_fills_steps_by_the_placing_rule(gpu_available):
+    """Steps of a wide, deep circuit beside 700 single gates: filled to a whole
+    number of ciphertexts per SM up to two, then to four, whatever name the launch
+    shape is set by, and the outputs are those of the jobs alone."""
+    import torch
+    P = pz()
+    eng, key, ev, s, _ = session("I_2P_LB_SR")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    deep = P.Circuit()
+    for _ in range(9):
+        deep.outputs(deep.u8_mul(deep.input_u8(), deep.input_u8()))
+    C = P.Circuit()
+    C.output(C.gate("nand", C.input(), C.input()))
+    inp = np.concatenate([enc_pair(ev, s, 3 + k, 5, 21 + k) for k in range(9)])
+    want, one = deep.run(eng, key, inp), C.run(eng, key, inp[:2])
+    seen = []
+    for variant in (0, 1, 2, 4):
+        S = P.Server(device=0, arena_bytes=1 << 27, max_items=4096)
+        S.set_schedule(P.server.SCHEDULE_CRITICAL_PATH)
+        S.set_launch(variant)
+        sid = S.add_session(eng, key)
+        job = S.submit(sid, deep, inp)
+        rest = [S.submit(sid, C, inp[:2]) for _ in range(700)]
+        steps = []
+        while S.stats()["pending"] or S.stats()["active"]:
+            steps.append(S.step())
+        assert np.array_equal(S.result(job), want)
+        assert all(np.array_equal(S.result(j), one) for j in rest[::97])
+        left = 700
+        for got, need in zip(steps, deep.level_sizes()):
+            fill = min(left, (-(-need // sms) * sms if need <= 2 * sms else 4 * sms) - need)
+            assert need <= 4 * sms and got == need + fill
+            left -= fill
+        seen.append(steps)
+    assert seen[1:] == seen[:1] * 3
