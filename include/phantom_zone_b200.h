@@ -131,6 +131,9 @@ const char *pz_last_error(const pz_ctx *ctx);
  * them; asynchronous ones (*_device, graph replays) leave it to the caller to
  * ask.  No reference counterpart (the reference panics on the CPU). */
 pz_status pz_ctx_device_error(pz_ctx *ctx, uint32_t *bits);
+/* PZ_ERR_CUDA while error bits are set, without clearing them: for callers that
+ * have waited for asynchronous work and are about to use its results. */
+pz_status pz_ctx_check(pz_ctx *ctx);
 /* Longest wait of a two-CTA blind rotation of this context for a key's copy or
  * the other CTA, in SM clock cycles (-1, the default: 2^31, about a second; 0:
  * every wait gives up at once, which is how the error path is tested).  A server

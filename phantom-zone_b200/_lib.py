@@ -94,6 +94,7 @@ SIGNATURES = {
     "pz_ctx_set_ks_tile": (st, [vp, ctypes.c_int]),
     "pz_ctx_launch_shape": (st, [vp, ctypes.c_size_t, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     "pz_ctx_device_error": (st, [vp, ctypes.POINTER(ctypes.c_uint32)]),
+    "pz_ctx_check": (st, [vp]),
     "pz_ctx_set_wait_limit": (st, [vp, ctypes.c_int64]),
     "pz_scratch_trim": (st, [ctypes.c_int, ctypes.c_size_t]),
     "pz_ctx_set_key_fft": (st, [vp, ctypes.c_int]),

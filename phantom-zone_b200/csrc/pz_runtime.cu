@@ -583,6 +583,12 @@ pz_status pz_ctx_device_error(pz_ctx *c, uint32_t *bits) {
   return PZ_OK;
 }
 
+pz_status pz_ctx_check(pz_ctx *c) {
+  if (!c) return PZ_ERR_INVALID_ARGUMENT;
+  PZ_CK(c, cudaSetDevice(c->device));
+  return pz::finish(c, c->stream);
+}
+
 pz_status pz_ctx_set_wait_limit(pz_ctx *c, int64_t cycles) {
   if (!c || cycles < -1) return PZ_ERR_INVALID_ARGUMENT;
   c->br.wait_limit = cycles < 0 ? pz::MBAR_WAIT_LIMIT : cycles;

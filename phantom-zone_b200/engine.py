@@ -218,6 +218,11 @@ class Engine:
         check(lib().pz_ctx_device_error(self.h, ctypes.byref(v)), self.h, "pz_ctx_device_error")
         return v.value
 
+    def check_device(self):
+        """Raises while device_error() bits are set (and leaves them): after waiting
+        for asynchronous work, before its results are used."""
+        check(lib().pz_ctx_check(self.h), self.h, "pz_ctx_check")
+
     def set_wait_limit(self, cycles=-1):
         """Longest wait of a two-CTA blind rotation, in SM clock cycles (-1: the
         default, about a second; 0: every wait gives up at once)."""

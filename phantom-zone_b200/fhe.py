@@ -146,6 +146,16 @@ def _device(ct, rows):
     return t
 
 
+def _host(t):
+    """The words of a device tensor, once what made them is done; raises if a
+    kernel of the engine gave up a wait (Engine.device_error)."""
+    words = t.cpu().numpy().view(np.uint64)
+    engine = _KEY.get("engine")
+    if engine is not None:
+        engine.check_device()
+    return words
+
+
 def _fold_div_zero(flag_now):
     """The thread's flag becomes flag_now (first division) -- the circuits
     with an ``_or`` suffix already OR'd the previous flag in."""
@@ -168,7 +178,7 @@ class FheBool:
 
     def lwe(self):
         """The ciphertext on the host: u64[N + 1]."""
-        return self.data.cpu().numpy().view(np.uint64)
+        return _host(self.data)
 
     def _gate(self, name, other):
         return FheBool._wrap(_run(name, self.data, other.data)[0])
@@ -239,7 +249,7 @@ class FheUint8:
 
     def lwe(self):
         """The ciphertexts on the host: u64[8][N + 1], LSB first."""
-        return self.data.cpu().numpy().view(np.uint64)
+        return _host(self.data)
 
     # -- arithmetic (shortint/mod.rs:63-205) ---------------------------------------------
     def __add__(self, other):

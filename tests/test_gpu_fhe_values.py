@@ -135,3 +135,23 @@ def test_operators_bit_exact_with_oracle(ctx):
     assert np.array_equal(q.lwe(), want_q) and np.array_equal(r.lwe(), want_r)
     assert np.array_equal(P.div_zero_error_flag().lwe(), want_f)
     P.reset_error_flags()
+
+
+def test_values_of_a_lost_wait_are_not_handed_out(ctx):
+    """Operators are asynchronous: lwe() raises while a kernel of the engine is
+    known to have given up a wait, and works again once that has been asked for."""
+    P, _, _, enc, encb, dec = ctx
+    from importlib import import_module
+    eng = import_module("phantom-zone_b200.fhe")._server()[0]
+    a, b = encb(1), encb(1)
+    assert dec(a & b) == 1
+    eng.set_wait_limit(0)
+    try:
+        lost = a & b
+    finally:
+        eng.set_wait_limit(-1)
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="gave up a wait"):
+            lost.lwe()
+    assert eng.device_error() == 1
+    assert dec(a & b) == 1
