@@ -286,3 +286,23 @@ def test_sample_extract_of_many(gpu_available, order, count):
         low = torch.gather(x[:, 0], 1, (k - col) % N)  # a_k .. a_0, then a_{N-1} .. a_{k+1}
         want = torch.cat([torch.gather(x[:, 1], 1, k), torch.where(col <= k, low, Q - low)], 1)
         assert torch.equal(out[at:at + 1000], torch.where(there[:, None], want, 5))
+
+
+@pytest.mark.parametrize("width", [74, 149, 223, 297, 371, 595])
+def test_circuit_levels_at_the_placing_boundaries(gpu_available, width):
+    """A circuit's level gathers its inputs and scatters its outputs by wire; split
+    over two launches, each half writes where the whole would have."""
+    P = pz()
+    eng = P.Engine("I_2P_LB_SR")
+    p = eng.p
+    g = np.random.default_rng(53)
+    key = eng.upload_key(g.integers(0, eng.Q, (p.lwe_n, p.rgsw_rows, eng.N), dtype=np.uint64),
+                         g.integers(0, eng.Q, (p.n_auto_keys, p.auto_rows, eng.N), dtype=np.uint64),
+                         g.integers(0, p.lwe_q, (p.lwe_d * eng.N, p.lwe_n + 1), dtype=np.uint64))
+    x = g.integers(0, eng.Q, (width + 1, eng.L), dtype=np.uint64)
+    C = P.Circuit()
+    wires = [C.input() for _ in x]
+    gates = [C.gate(["and", "nand", "or", "nor", "xor", "xnor"][i % 6], wires[i], wires[i + 1]) for i in range(width)]
+    C.outputs(gates[::-1])
+    want = eng.gate_batch(key, (np.arange(width) % 6).astype(np.uint8), x[:-1], x[1:])
+    assert np.array_equal(C.run(eng, key, x), want[::-1])
