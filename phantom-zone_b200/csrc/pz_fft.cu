@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256)
 // scheduler, the register file being full; TRIO and SPLIT the barriers and fixed
 // latencies between FP64 phases and integer ones.  With integer transforms 3552
 // ciphertexts took 228 ms (QUAD 170), 148 took 13.3 (TRIO 8.6), one 10.1 (SPLIT
-// 5.5).
+// 5.6).
 // The key: QUAD loads it into registers, four CTAs covering for each other;
 // TRIO early into more of them (each block while the digits or the output before
 // are transformed); SPLIT has each block copied (cp.async.bulk) into shared
@@ -417,7 +417,7 @@ __device__ __forceinline__ void op_trio(u32 i, u32 op, u32 nx_op, Next &now, con
   // SPLIT: some of the block's points into registers while the digits are
   // transformed (the products would wait for all of it otherwise, 96 KB in 770
   // cycles: one gate 5.96 -> 5.78 ms together with the sums dealt out 6, 6 and 4;
-  // of 2 to 5 points 3 are the fastest, 5.62 ms against 5.65 to 5.67)
+  // of 2 to 5 points 3 are the fastest, 5.60 ms against 5.66 to 5.79)
   constexpr int EARLY = 3;
   const cplx *const sk = F == SPLIT ? S.key(g) + t : nullptr;
   auto take = [&]() {
@@ -847,7 +847,7 @@ static cudaError_t launch_form(fft::Form form, const Batch &b, size_t begin, siz
   }
 }
 
-// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 5.5 for up to 74
+// The forms by batch size.  NI_8P on 148 SMs, ms: SPLIT 5.6 for up to 74
 // ciphertexts; TRIO 8.6 for up to 148 and again for each 148 more; QUAD 15.1,
 // 18.9, 24.2 and 30.3 for up to 148, 296, 444 and 592, and from there 28.3 per
 // 592, but 39.6 for 600 (the last few take as long as on an idle GPU).  So,

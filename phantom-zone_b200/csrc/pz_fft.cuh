@@ -9,15 +9,24 @@
 // real part and j + 1024 as the imaginary part of c_j, in
 // C[t]/(t^1024 - i)), rounded to the nearest integer and recombined mod Q.
 //
-// The rounding is exact for every input.  With u = 2^-53, one operation sums
-// two products with |d| <= 2^16, so sum ||d||_2 ||k_l||_2 <= 2 * 2^(16 + 5.5)
-// * 2^(17 + 5.5) = 2^45.  Every level of a transform adds at most 3u of
-// relative error (two roundings in a + w b, one more in 2a - (a + w b) or in
-// the product of the inverse, and the rounding of w), ten levels forward and
-// ten inverse; the pointwise products add 4u and the key transforms, which
-// are computed in double-double and rounded once, u.  By Cauchy-Schwarz over
-// the spectra every output coefficient is off by at most
-// (30 + 30 + 5) u 2^45 < 0.26 < 1/2.  (Measured: below 2^-8.)
+// The rounding is exact for every input.  With u = 2^-53 and to first order, write
+// S = sum ||d|| ||k_l|| over an operation's two products, |d| <= 2^16: S <=
+// 2 * 2^(16 + 5.5) * 2^(17 + 5.5) = 2^45.  Each of these is at most c u S in every
+// output coefficient, and the c add up to 87: 87 u 2^45 < 0.35 < 1/2.  (Measured:
+// below 2^-8.)
+//   forward, 40: a butterfly's t = a + w b has two roundings per component, of
+//   a + Re(w) b and of t, and w one; 2a - t repeats them and adds its own.  In the
+//   2-norm of the pair, with |a|^2 + |b|^2 = 1, that is u (sqrt2 |a + Re(w) b| +
+//   sqrt2 |t| + |2a - t| + sqrt2 |b|) <= u (sqrt2 sqrt5 + sqrt3 sqrt2) < 5.7 u
+//   against the pair's norm of sqrt2: 4 u per level, ten levels; the spectra's
+//   errors reach a coefficient as a sum over the points, at most (Cauchy-Schwarz)
+//   the product of the 2-norms of the error and of the key's spectrum.
+//   products, 6: four roundings in a chain per component, 4 sqrt2 u.
+//   keys, 1: transformed in double-double and rounded once.
+//   inverse, 40: of a + b one rounding, of conj(w) (a - b) three and w's own: 4 u
+//   (|a| + |b|) per butterfly.  Summed over the values that a coefficient is made
+//   of, whose 1-norm no level increases and which is at most S (Cauchy-Schwarz), 4
+//   u S per level, ten levels.
 //
 // Why FFTs: on B200 an FP64 multiply-add costs what a 32-bit integer one
 // does, and a complex radix-2 butterfly over 2048 real coefficients takes 6
@@ -585,8 +594,9 @@ __device__ __forceinline__ void add_limb2(u64 &acc, double z) {
   const u64 w = (u64)__double_as_longlong(z + ROUND);
   acc += ((u64)(((u32)w & 0x3ffffu) << 4) << 32) + (u64)((long long)(int)(u32)(w >> 18) * 77823ll);
 }
-// The sum of the limbs (in (-2^47, 2^56) once ROUND_SUM is taken off) -> a
-// representative mod Q in [-2^53 - 2^20, 2^53 + 2^20].
+// The sum of the limbs (once ROUND_SUM is taken off in (-2^47, 2^55 + 2^47), with
+// an automorphism's b, of at most 2 Q, in (-2^56, 2^57)) -> a representative mod Q
+// in [-2^53 - 2^20, 2^53 + 2^20].
 __device__ __forceinline__ long long settle_sum(u64 acc) {
   const int h = ((int)(acc >> 32) + (1 << 21)) >> 22;
   return (long long)(acc - ((u64)((u32)h << 22) << 32)) + (long long)h * 77823ll;
@@ -627,6 +637,8 @@ static_assert(RLRG_LOGB + RLRG_IGN == 54 && AUTO_LOGB + AUTO_IGN == 54, "one dig
 // into limbs, and each limb transformed in double-double arithmetic, scaled by
 // 1 / M (exact) and rounded once.  CTAs of 256 threads.
 // ---------------------------------------------------------------------------
+// Double-double arithmetic (Dekker 1971; the two-sum Knuth's, the product's low
+// part by a fused multiply-add).
 struct dd {
   double h, l;
 };

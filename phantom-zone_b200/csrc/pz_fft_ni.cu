@@ -6,8 +6,9 @@
 //
 // The digits are the d = 50 one-bit signed digits of a value, in {-1, 0, 1}, so
 // two limbs of 27 bits do: sum_j ||digit_j|| ||k_j|| <= 50 * 2^5.5 * 2^(26 + 5.5)
-// < 2^42.7, the transforms' error is 61 u of that (pz_fft.cuh) and the sum of
-// 50 products' another 100 u: less than 2^-2.9 < 1/2 in every coefficient.
+// < 2^42.7, the transforms' and keys' error is 81 u of that (pz_fft.cuh) and that of
+// the sum of 50 products, 100 roundings in a chain, 100 sqrt2 u: 223 u, less than
+// 2^-2.4 < 1/2 in every coefficient.
 //
 // A batch of 24 values takes 65 us (the integer transforms took 95 with their
 // digits split over CTAs); three users' 620-index key 13 ms (37).
