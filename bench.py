@@ -11,9 +11,9 @@ launch; the whole circuit is one CUDA graph replayed per step.
   e2e     the same through pz_circuit_run: host buffers in pinned memory,
           host->device inputs and device->host outputs inside the timed region
   plain   InteractiveLTE2Party, 128 NAND gates, one gate per launch
-  roofline  blind-rotation kernel: algorithmic 32-bit multiply instructions
-          (10 per 64-bit modmul, the roofline convention) per second / the IMAD
-          rate measured on this GPU by pz_probe_imad_rate
+  roofline  blind-rotation kernel: FP64 instructions of its transforms and
+          products per second / the DFMA rate measured on this GPU by
+          pz_probe_pipe_rates
   cpu_baseline  the CPU oracle (a C++ restatement of the reference's pbs path)
           on all host threads, bounded sample of the same gates
 
@@ -40,7 +40,10 @@ sys.path.insert(0, ROOT)
 PARAM = "NI_8P"
 N_MUL = 1024
 N_LT = 1024
-C_MM = 10  # 32-bit multiply instructions per 64-bit Shoup modmul (roofline convention)
+C_MM = 10  # 32-bit multiply instructions per 64-bit Shoup modmul (roofline convention of the batched NTT)
+# FP64 instructions of one operation of the blind rotation over FFTs (N = 2048): two forward and six inverse
+# transforms of 5120 butterflies (6 and 8 each), 6 x 1024 sums of two complex products
+FP64_PER_OP = 2 * 5120 * 6 + 6 * 5120 * 8 + 6 * 1024 * 8
 GATE_NAMES = ["and", "nand", "or", "nor", "xor", "xnor"]
 REF_STEP_SECONDS = 10.0  # wall time of one timed step of the CPU reference arm
 ROOFLINE_WAVES = 8  # whole waves of the blind-rotation launch timed for the roofline
@@ -77,9 +80,10 @@ def wavefront_circuit(P):
 
 
 def schedule_work(p, ks):
-    """Exact counts of the blind rotation's work per ciphertext (pbs.rs:240-414)
-    from key-switched LWEs ks [count][n+1]: returns modmuls by the roofline
-    convention M = F (N/2) logN + I ((N/2) logN + N) + MAC."""
+    """Exact counts of the blind rotation's work (pbs.rs:240-414) from
+    key-switched LWEs ks [count][n+1]: the modmuls of integer transforms,
+    M = F (N/2) logN + I ((N/2) logN + N) + MAC, and the operations (external
+    products and non-trivial automorphisms)."""
     br_q, n, N, g, w = p.br_q, p.lwe_n, p.rlwe_n, p.g, p.w
     dlog = np.zeros(br_q, np.int64)
     for i in range(br_q // 4):
@@ -89,7 +93,7 @@ def schedule_work(p, ks):
     shift = int(np.log2(p.lwe_q)) - int(np.log2(br_q))
     q4 = br_q // 4
     logn = int(np.log2(N))
-    total = 0
+    total = ops = 0
     for row in ks:
         odd = (row[1:].astype(np.int64) >> shift)
         odd = odd + ((odd & 1) ^ 1)
@@ -121,7 +125,8 @@ def schedule_work(p, ks):
         F, I = 2 * n - 1 + A, 2 * n + 2 * A
         MAC = (4 * n - 2) * N + 2 * A * N
         total += F * (N // 2) * logn + I * ((N // 2) * logn + N) + MAC
-    return total
+        ops += n + A
+    return total, ops
 
 
 def measured_hbm_gbs():
@@ -439,26 +444,21 @@ def microbench(P, torch, device, count=4096, reps=5):
     rl = torch.from_numpy(rng.integers(0, p.rlwe_q, (count, 2, N), dtype=np.uint64).view(np.int64)).cuda()
     idx = torch.arange(count, dtype=torch.int32, device="cuda") % p.lwe_n
     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    ep_by_shape = {}
-    for v in (0, 1, 2):  # names of one launch shape: three runs of it
-        eng.pbs_variant = v
+    eng.rlwe_by_rgsw_device(key, rl, idx)
+    torch.cuda.synchronize()
+    a.record()
+    for _ in range(reps):
         eng.rlwe_by_rgsw_device(key, rl, idx)
-        torch.cuda.synchronize()
-        a.record()
-        for _ in range(reps):
-            eng.rlwe_by_rgsw_device(key, rl, idx)
-        b.record()
-        torch.cuda.synchronize()
-        ep_by_shape[v] = a.elapsed_time(b) / reps
-    ep_variant = min(ep_by_shape, key=ep_by_shape.get)
-    ep_ms = ep_by_shape[ep_variant]
+    b.record()
+    torch.cuda.synchronize()
+    ep_ms = a.elapsed_time(b) / reps
     key.release()
     eng.close()
     peak_imad = P.probe_imad_rate(device)
     hbm = measured_hbm_gbs()
     ntt_mm_s = mm / ((fwd_ms + inv_ms) / 1e3)
     ntt_gbs = 4 * count * N * 8 / ((fwd_ms + inv_ms) / 1e3) / 1e9
-    ep_mm_s = count * 57344 / (ep_ms / 1e3)
+    peak_fp64 = P.probe_pipe_rates(device)["dfma"]
     return {"config": f"{count} polys N={N} mod Q fwd+inv NTT; {count} RLWE x RGSW at I_2P_LB_SR (index i mod n)",
             "ntt_fwd_ms": fwd_ms, "ntt_inv_ms": inv_ms, "ntt_roundtrip_exact": roundtrip_ok,
             "ntt_polys_per_s": count / ((fwd_ms + inv_ms) / 1e3),
@@ -466,12 +466,13 @@ def microbench(P, torch, device, count=4096, reps=5):
             "ntt_int_frac": ntt_mm_s * C_MM / peak_imad,
             "ntt_hbm_frac": ntt_gbs / hbm["gbs"] if hbm["gbs"] else None,
             "ext_product_ms": ep_ms, "ext_products_per_s": count / (ep_ms / 1e3),
-            "ext_product_modmul_per_s": ep_mm_s, "ext_product_int_frac": ep_mm_s * C_MM / peak_imad,
-            "ext_product_ms_by_variant": ep_by_shape, "ext_product_variant": ep_variant,
+            "ext_product_fp64_frac": count * FP64_PER_OP / (ep_ms / 1e3) / peak_fp64,
             "roof": {"int_peak_imad_per_s": peak_imad, "int_peak_source": "pz_probe_imad_rate on this GPU",
+                     "fp64_peak_dfma_per_s": peak_fp64,
                      "hbm_gbs": hbm["gbs"], "hbm_source": hbm["source"],
-                     "what": "fractions: algorithmic modmuls x 10 IMAD / the IMAD peak; bytes in + out of both "
-                             "passes / the HBM copy bandwidth"}}
+                     "what": "fractions: the NTT's algorithmic modmuls x 10 IMAD / the IMAD peak, its bytes in + out "
+                             "of both passes / the HBM copy bandwidth; FP64 instructions of the products' transforms "
+                             "/ the DFMA peak"}}
 
 
 def ni_ingest_bench(P, torch, device, count=64, reps=3):
@@ -510,9 +511,8 @@ def ni_ingest_bench(P, torch, device, count=64, reps=3):
     torch.cuda.synchronize()
     all_ms = a.elapsed_time(b) / reps
     ks_ms = b.elapsed_time(c) / reps
-    logn = int(np.log2(N))
-    per_rlwe = p.ni_ks_d * (N // 2) * logn + 2 * ((N // 2) * logn + N) + 2 * p.ni_ks_d * N
-    mm = count * per_rlwe
+    # FP64 instructions: d digits transformed, d x 4 products per point, 4 transforms back
+    per_rlwe = p.ni_ks_d * (5120 * 6 + 4 * 1024 * 4) + 4 * 5120 * 8
     del d_l
     # the key switch alone at a serving-sized batch (the extraction of that
     # many bools would not fit: N + 1 words per bool)
@@ -527,16 +527,16 @@ def ni_ingest_bench(P, torch, device, count=64, reps=3):
     b.record()
     torch.cuda.synchronize()
     big_ms = a.elapsed_time(b) / reps
-    peak = P.probe_imad_rate(device)
+    peak = P.probe_pipe_rates(device)["dfma"]
     ksk.release()
     eng.close()
     return {"config": f"NI_8P, {count} seeded RLWEs = {count * N} bools: unseed + rlwe_key_switch (d=50) + extract; "
                       f"key switch alone also at {big} RLWEs",
             "ingest_ms": all_ms, "bools_per_s": count * N / (all_ms / 1e3), "key_switch_ms": ks_ms,
-            "rlwe_key_switches_per_s": count / (ks_ms / 1e3), "key_switch_modmul_per_s": mm / (ks_ms / 1e3),
-            "key_switch_int_frac": mm / (ks_ms / 1e3) * C_MM / peak,
+            "rlwe_key_switches_per_s": count / (ks_ms / 1e3),
+            "key_switch_fp64_frac": count * per_rlwe / (ks_ms / 1e3) / peak,
             f"key_switch_{big}_ms": big_ms, f"rlwe_key_switches_per_s_{big}": big / (big_ms / 1e3),
-            f"key_switch_int_frac_{big}": big * per_rlwe / (big_ms / 1e3) * C_MM / peak}
+            f"key_switch_fp64_frac_{big}": big * per_rlwe / (big_ms / 1e3) / peak}
 
 
 def key_upload_bench(P, device):
@@ -977,7 +977,7 @@ def kernel_only(args):
     if args.mode == "ks-kernel":
         out["ks_tile"] = args.ks_tile
     if args.mode == "br-kernel":
-        out["modmuls_per_item"] = schedule_work(p, ks) / B
+        out["operations_per_item"] = schedule_work(p, ks)[1] / B
     print(json.dumps(out), flush=True)
 
 
@@ -1104,11 +1104,10 @@ def main():
     eb.record()
     torch.cuda.synchronize()
     br_ms = ea.elapsed_time(eb) / reps
-    modmuls = schedule_work(p, ks)
-    achieved = modmuls * C_MM / (br_ms / 1e3) / 1e12  # T IMAD/s
-    peak = P.probe_imad_rate(local) / 1e12
-    # the other pipes the butterflies use (the quotient runs on the FP64 pipe and the conversion unit)
+    modmuls, operations = schedule_work(p, ks)
+    achieved = operations * FP64_PER_OP / (br_ms / 1e3) / 1e12  # T FP64 instructions/s
     pipes = {k: v / 1e12 for k, v in P.probe_pipe_rates(local).items()}
+    peak = pipes["dfma"]
     traffic, traffic_source = traffic_record(P, tune["variant"], B)
 
     plain = None
@@ -1157,15 +1156,15 @@ def main():
                     "h2d_bytes_per_step": int(info["inputs"] * L * 8),
                     "d2h_bytes_per_step": int(info["outputs"] * L * 8)},
             "gpu_launches": launches_per_step * args.steps,
-            "roofline": {"bound": "int", "kernel": "pbs_fft_kernel (blind rotation)", "achieved": achieved,
-                         "peak": peak, "unit": "TIMAD/s", "frac": achieved / peak, "traffic": traffic,
+            "roofline": {"bound": "fp64", "kernel": "pbs_fft_kernel (blind rotation)", "achieved": achieved,
+                         "peak": peak, "unit": "T FP64 instructions/s", "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": traffic_source,
-                         "peak_source": "pz_probe_imad_rate on this GPU (MEASURED_PEAKS.json has no integer peak)",
+                         "peak_source": "pz_probe_pipe_rates on this GPU (MEASURED_PEAKS.json has no FP64 peak)",
                          "launch_ms": br_ms, "bootstraps_per_launch": B,
-                         "modmuls_per_bootstrap": modmuls / B,
+                         "operations_per_bootstrap": operations / B, "modmuls_per_bootstrap": modmuls / B,
                          "pipe_rates_tips": pipes,
-                         "convention": "10 IMAD per 64-bit modmul of integer transforms; the products run as FP64 "
-                                       "FFTs, so none of this work is on the IMAD pipe"},
+                         "convention": f"{FP64_PER_OP} FP64 instructions per operation (butterflies and products); "
+                                       "modmuls are those of 64-bit integer transforms, for comparison"},
             "plain": plain,
             "parity": parity,
             **extras,
