@@ -543,7 +543,9 @@ pz_status pz_server_add_managed_session(pz_server *s, pz_ctx *ctx, const void *k
 /* dry-run servers only: a managed session of param_id (residency bookkeeping only) */
 pz_status pz_server_add_virtual_managed_session(pz_server *s, int param_id, uint32_t *session);
 /* Device bytes resident managed keys may hold (0: no limit, the default);
- * resident_key_bytes of the statistics is what they and the other sessions' hold. */
+ * resident_key_bytes of the statistics is what they and the other sessions' hold.
+ * While a key comes in or changes its form, what the new form is made from is held
+ * besides (NI_8P: at most 77 MB). */
 pz_status pz_server_set_key_budget(pz_server *s, size_t bytes);
 /* *resident = 1 when the session's key is on the device now. */
 pz_status pz_server_session_resident(pz_server *s, uint32_t session, int *resident);

@@ -116,7 +116,8 @@ pz_status managed_import(pz_ctx *c, const void *blob, size_t size, bool fft, pz_
   key_sizes(c, &rg, &au, &ks);
   pz_key *k = new pz_key();
   k->ctx = c;
-  // one form at a time, each in the place of what it was made from
+  // each form in the place of what it was made from, so that little more than the
+  // key's bytes is held at a time
   cudaError_t e = dev_malloc(&k->d_ksk, ks);
   if (e == cudaSuccess)
     e = cudaMemcpy(k->d_ksk, (const unsigned char *)blob + sizeof(KeyHeader) + rg + au, ks, cudaMemcpyHostToDevice);
