@@ -545,7 +545,7 @@ pz_status pz_server_add_virtual_managed_session(pz_server *s, int param_id, uint
 /* Device bytes resident managed keys may hold (0: no limit, the default);
  * resident_key_bytes of the statistics is what they and the other sessions' hold.
  * While a key comes in or changes its form, what the new form is made from is held
- * besides (NI_8P: at most 77 MB). */
+ * besides (NI_8P: at most 44 MB more). */
 pz_status pz_server_set_key_budget(pz_server *s, size_t bytes);
 /* *resident = 1 when the session's key is on the device now. */
 pz_status pz_server_session_resident(pz_server *s, uint32_t session, int *resident);
